@@ -30,8 +30,8 @@ namespace gps {
 namespace {
 
 constexpr int kMidThreads = 256;
-// Resident CTAs per SM the aligned-buffer kernel is compiled for.
-constexpr int kMidVecCtasPerSm = 8;
+// Resident CTAs per SM the kernel is compiled for.
+constexpr int kMidCtasPerSm = 8;
 
 // ------------------------------------------------------------ descriptors
 // One 16-byte word per tile: {lo: the value (u32 or u64), hi: status:2 |
@@ -54,12 +54,6 @@ struct MidDesc {
         return (w.hi & kGidMask) == (gid & kGidMask) ? static_cast<uint32_t>(w.hi >> 62) : kNotReady;
     }
 };
-
-__device__ __forceinline__ uint64_t grid_id() {
-    uint64_t g;
-    asm volatile("mov.u64 %0, %%gridid;" : "=l"(g));
-    return g;
-}
 
 // ------------------------------------------------------- two-level lookback
 // Tiles form groups of 32. Besides its tile descriptor, the last tile of each
@@ -204,49 +198,7 @@ __device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint
     return pre;
 }
 
-// Buffers not aligned to 16 bytes: each thread loads and stores its 64
-// bytes element by element.
-template <typename T, bool INCL>
-__global__ void __launch_bounds__(kMidThreads, 2) mid_scan_kernel(const ScanArgs a) {
-    constexpr int TILE = 16384 / static_cast<int>(sizeof(T));
-    constexpr int ITEMS = TILE / kMidThreads;  // 16 u32 or 8 u64: 64 bytes
-    __shared__ gps_device::BlockScanStorage<kMidThreads, T> st;
-    __shared__ LookbackSmem lsm;
-    __shared__ T s_pre[1];
-
-    const uint32_t tid = threadIdx.x;
-    const uint32_t t = blockIdx.x;
-    const uint64_t gid = grid_id();
-    const T* in = static_cast<const T*>(a.in);
-    T* out = static_cast<T*>(a.out);
-    const uint64_t i0 = static_cast<uint64_t>(t) * TILE + static_cast<uint64_t>(tid) * ITEMS;
-
-    T v[ITEMS];
-#pragma unroll
-    for (int e = 0; e < ITEMS; ++e) v[e] = i0 + e < a.n ? in[i0 + e] : T(0);
-    T sum = 0;
-#pragma unroll
-    for (int e = 0; e < ITEMS; ++e) sum += v[e];
-    T total;
-    const T before = gps_device::block_exclusive_scan<kMidThreads>(sum, st, gps_device::Plus(), &total);
-    T run = mid_tile_prefix<T>(a, t, gid, total, lsm, s_pre) + before;
-#pragma unroll
-    for (int e = 0; e < ITEMS; ++e) {
-        const T x = v[e];
-        if (INCL) {
-            run += x;
-            v[e] = run;
-        } else {
-            v[e] = run;
-            run += x;
-        }
-    }
-#pragma unroll
-    for (int e = 0; e < ITEMS; ++e)
-        if (i0 + e < a.n) out[i0 + e] = v[e];
-}
-
-// The same scan for 16-byte-aligned buffers. The tile is four rows of 256
+// The scan itself. The tile is four rows of 256
 // 16-byte chunks, and thread tid holds chunk tid of every row, so each warp
 // load or store instruction covers 512 contiguous bytes. The exclusive prefix
 // of chunk (r, tid) within the tile is the sum of the rows before r plus the
@@ -260,8 +212,54 @@ __global__ void __launch_bounds__(kMidThreads, 2) mid_scan_kernel(const ScanArgs
 // eight CTAs per SM: on 152 SMs up to 1216 tiles (2^22 u32 elements fit) run
 // in one wave. There is no shared-memory staging and no mbarrier to set up,
 // so every CTA issues its loads as soon as it starts.
-template <typename T, bool INCL>
-__global__ void __launch_bounds__(kMidThreads, kMidVecCtasPerSm) mid_vec_kernel(const ScanArgs a) {
+//
+// ALIGNED = false takes buffers at any element offset from a 16-byte
+// boundary. Tiles are then counted from the boundary at or below the input
+// ("virtual" index j = i + lead, lead elements of tile 0 lying before the
+// input), so every load but those of the first and last chunk stays a 16-byte
+// one. The output's boundary may lie elsewhere: if virtual element 0 sits
+// `phase` elements past one, an output chunk is the last `phase` elements of
+// the chunk on the left (one shuffle each) and the first of this one, stored
+// as 16 bytes; a warp's two edges, tile 0 and a partial tile store elements.
+// Bound by the same latency chain as the aligned form. Measured on GB300,
+// 10,000,019 u32 from a view one element past a boundary, into an aligned
+// output: 22.9 us a call, where per-thread element loads and stores (64
+// bytes apart across a warp) took 70.9.
+template <typename T>
+__device__ __forceinline__ void store_elems(T* p, uint32_t off, uint32_t first, uint32_t cnt, const Chunk<T>& q) {
+    constexpr int EPC = 16 / static_cast<int>(sizeof(T));
+#pragma unroll
+    for (int e = 0; e < EPC; ++e)
+        if (off + e >= first && off + e < cnt) p[e] = q.v[e];
+}
+
+// Stores a warp's row of chunks of an interior tile, whose output lies P
+// elements past a 16-byte boundary; p is this lane's first output element.
+template <typename T, int P>
+__device__ __forceinline__ void store_shifted(T* p, uint32_t lane, const Chunk<T>& q) {
+    constexpr int EPC = 16 / static_cast<int>(sizeof(T));
+    Chunk<T> w;
+#pragma unroll
+    for (int e = 0; e < EPC; ++e) {
+        if (e < P)
+            w.v[e] = __shfl_up_sync(kFullMask, q.v[EPC - P + e], 1);
+        else
+            w.v[e] = q.v[e - P];
+    }
+    if (lane != 0) {
+        *reinterpret_cast<Chunk<T>*>(p - P) = w;
+    } else {
+#pragma unroll
+        for (int e = 0; e < EPC - P; ++e) p[e] = q.v[e];
+    }
+    if (lane == 31) {
+#pragma unroll
+        for (int e = EPC - P; e < EPC; ++e) p[e] = q.v[e];
+    }
+}
+
+template <typename T, bool INCL, bool ALIGNED>
+__global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm) mid_vec_kernel(const ScanArgs a) {
     constexpr int TILE = 16384 / static_cast<int>(sizeof(T));
     constexpr int EPC = 16 / static_cast<int>(sizeof(T));
     constexpr int ROW = kMidThreads * EPC;  // elements per row
@@ -277,27 +275,34 @@ __global__ void __launch_bounds__(kMidThreads, kMidVecCtasPerSm) mid_vec_kernel(
     const uint32_t lane = tid & 31u;
     const uint32_t warp = tid >> 5;
     const uint32_t t = blockIdx.x;
-    const uint64_t gid = grid_id();
+    const uint64_t gid = ptx::grid_id();
     const uint64_t t0 = static_cast<uint64_t>(t) * TILE;
+    // Elements of the input before virtual element `lead` do not exist.
+    const uint32_t lead =
+        ALIGNED ? 0u : static_cast<uint32_t>((reinterpret_cast<uintptr_t>(a.in) & 15u) / sizeof(T));
+    const uint32_t first = t == 0 ? lead : 0u;
     // Elements of this tile; chunk (r, tid) starts at element r * ROW + tid * EPC.
-    const uint32_t cnt = static_cast<uint32_t>(min(static_cast<uint64_t>(TILE), a.n - t0));
-    const bool full = cnt == static_cast<uint32_t>(TILE);
-    const T* src = static_cast<const T*>(a.in) + t0 + tid * EPC;
-    T* dst = static_cast<T*>(a.out) + t0 + tid * EPC;
+    const uint32_t cnt = static_cast<uint32_t>(min(static_cast<uint64_t>(TILE), a.n + lead - t0));
+    const bool full = cnt == static_cast<uint32_t>(TILE) && first == 0;
+    const T* src = static_cast<const T*>(a.in) - lead + t0 + tid * EPC;
+    T* dst = static_cast<T*>(a.out) - lead + t0 + tid * EPC;
+    auto load = [&](int r) -> Chunk<T> {
+        const uint32_t off = r * ROW + tid * EPC;
+        Chunk<T> q;
+        if (full || (off >= first && off + EPC <= cnt)) {
+            q = *reinterpret_cast<const Chunk<T>*>(src + r * ROW);
+        } else {
+#pragma unroll
+            for (int e = 0; e < EPC; ++e) q.v[e] = off + e >= first && off + e < cnt ? src[r * ROW + e] : T(0);
+        }
+        return q;
+    };
 
     T cs[ROWS];
     {
         Chunk<T> q[ROWS];
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) {
-            const uint32_t off = r * ROW + tid * EPC;
-            if (full || off + EPC <= cnt) {
-                q[r] = *reinterpret_cast<const Chunk<T>*>(src + r * ROW);
-            } else {
-#pragma unroll
-                for (int e = 0; e < EPC; ++e) q[r].v[e] = off + e < cnt ? src[r * ROW + e] : T(0);
-            }
-        }
+        for (int r = 0; r < ROWS; ++r) q[r] = load(r);
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
             T x = 0;
@@ -327,50 +332,70 @@ __global__ void __launch_bounds__(kMidThreads, kMidVecCtasPerSm) mid_vec_kernel(
 
     const T base = mid_tile_prefix<T>(a, t, gid, total, lsm, s_pre);
 
-    Chunk<T> q[ROWS];
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-        const uint32_t off = r * ROW + tid * EPC;
-        if (full || off + EPC <= cnt) {
-            q[r] = *reinterpret_cast<const Chunk<T>*>(src + r * ROW);
-        } else {
-#pragma unroll
-            for (int e = 0; e < EPC; ++e) q[r].v[e] = off + e < cnt ? src[r * ROW + e] : T(0);
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < ROWS; ++r) {
-        const uint32_t off = r * ROW + tid * EPC;
+    auto scan_chunk = [&](int r, Chunk<T>& q) {
         T acc = base + s_off[r][tid];
 #pragma unroll
         for (int e = 0; e < EPC; ++e) {
-            const T x = q[r].v[e];
+            const T x = q.v[e];
             if (INCL) {
                 acc += x;
-                q[r].v[e] = acc;
+                q.v[e] = acc;
             } else {
-                q[r].v[e] = acc;
+                q.v[e] = acc;
                 acc += x;
             }
         }
-        if (full || off + EPC <= cnt) {
-            *reinterpret_cast<Chunk<T>*>(dst + r * ROW) = q[r];
-        } else {
+    };
+    if constexpr (ALIGNED) {
+        Chunk<T> q[ROWS];
 #pragma unroll
-            for (int e = 0; e < EPC; ++e)
-                if (off + e < cnt) dst[r * ROW + e] = q[r].v[e];
+        for (int r = 0; r < ROWS; ++r) q[r] = load(r);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            const uint32_t off = r * ROW + tid * EPC;
+            scan_chunk(r, q[r]);
+            if (full || off + EPC <= cnt)
+                *reinterpret_cast<Chunk<T>*>(dst + r * ROW) = q[r];
+            else
+                store_elems(dst + r * ROW, off, 0u, cnt, q[r]);
+        }
+    } else {
+        // Output elements past a 16-byte boundary (of this tile's first chunk,
+        // and so of every chunk). One row at a time, which keeps the kernel
+        // at 32 registers.
+        const uint32_t phase = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(dst) & 15u) / sizeof(T));
+#pragma unroll 1
+        for (int r = 0; r < ROWS; ++r) {
+            const uint32_t off = r * ROW + tid * EPC;
+            T* p = dst + r * ROW;
+            Chunk<T> q = load(r);
+            scan_chunk(r, q);
+            if (phase == 0 && (full || (off >= first && off + EPC <= cnt)))
+                *reinterpret_cast<Chunk<T>*>(p) = q;
+            else if (phase == 0 || !full)
+                store_elems(p, off, first, cnt, q);
+            else if (phase == 1)
+                store_shifted<T, 1>(p, lane, q);
+            else if (EPC == 4 && phase == 2)
+                store_shifted<T, EPC == 4 ? 2 : 1>(p, lane, q);
+            else
+                store_shifted<T, EPC == 4 ? 3 : 1>(p, lane, q);
         }
     }
 }
 
-template <typename T, bool INCL, bool VEC>
+template <typename T, bool INCL, bool ALIGNED>
 cudaError_t launch_mid_v(const ScanArgs& a0, cudaStream_t stream, LaunchInfo* info) {
-    auto kern = VEC ? mid_vec_kernel<T, INCL> : mid_scan_kernel<T, INCL>;
+    constexpr uint64_t TILE = 16384 / sizeof(T);
     ScanArgs a = a0;
+    // Tiles from the input's 16-byte boundary: at most one more than the
+    // plan's (its descriptor regions have kDescPad to spare).
+    const uint64_t lead = ALIGNED ? 0 : (reinterpret_cast<uintptr_t>(a.in) & 15u) / sizeof(T);
+    a.num_tiles = static_cast<uint32_t>((a.n + lead + TILE - 1) / TILE);
     a.desc_stride = a.num_tiles > kGroupTiles && a.num_tiles <= kMidStrideMaxTiles ? kMidDescStride : 1u;
     const int grid = static_cast<int>(a.num_tiles);
     if (info) *info = LaunchInfo{grid, kMidThreads, 0};
-    kern<<<grid, kMidThreads, 0, stream>>>(a);
+    mid_vec_kernel<T, INCL, ALIGNED><<<grid, kMidThreads, 0, stream>>>(a);
     return cudaGetLastError();
 }
 
@@ -379,8 +404,8 @@ cudaError_t launch_mid_t(const ScanArgs& a, cudaStream_t stream, LaunchInfo* inf
     if (((reinterpret_cast<uintptr_t>(a.desc) | reinterpret_cast<uintptr_t>(a.group_desc)) & 15u) != 0 ||
         a.desc == nullptr || a.group_desc == nullptr)
         return cudaErrorInvalidValue;
-    const bool vec = ((reinterpret_cast<uintptr_t>(a.in) | reinterpret_cast<uintptr_t>(a.out)) & 15u) == 0;
-    return vec ? launch_mid_v<T, INCL, true>(a, stream, info) : launch_mid_v<T, INCL, false>(a, stream, info);
+    const bool aligned = ((reinterpret_cast<uintptr_t>(a.in) | reinterpret_cast<uintptr_t>(a.out)) & 15u) == 0;
+    return aligned ? launch_mid_v<T, INCL, true>(a, stream, info) : launch_mid_v<T, INCL, false>(a, stream, info);
 }
 
 }  // namespace
