@@ -175,6 +175,7 @@ gps_status launch_scan(gps_plan_s* p, bool inclusive, const void* in, void* out,
     a.carry_out = carry_out;
     a.wait_budget_ns = p->wait_budget_ns;
     a.stall = p->stall;
+    a.mid_launch = &p->hdr->mid_launch;
     // The persistent kernel for buffers off a 16-byte boundary moves single
     // elements; one tile per CTA is faster at every size (2^25 u32 elements:
     // 64 against 527 us, 2^27: 258 against 2017).
@@ -707,6 +708,15 @@ gps_status gps_plan_check(gps_plan p, gps_stream_t stream) {
             if (err != cudaSuccess) return cuda_fail(err, "clearing device error flags");
         }
         all |= flags;
+    }
+    // A wait that ran out may have left the launch number behind, or CTAs
+    // that read it late: skip past both.
+    if (all != 0 && p->algo == GPS_ALGO_CSDL) {
+        uint64_t number = 0;
+        err = cudaMemcpy(&number, &p->hdr->mid_launch, sizeof(number), cudaMemcpyDeviceToHost);
+        number += 2;
+        if (err == cudaSuccess) err = cudaMemcpy(&p->hdr->mid_launch, &number, sizeof(number), cudaMemcpyHostToDevice);
+        if (err != cudaSuccess) return cuda_fail(err, "advancing the launch number");
     }
     if (all != 0) return fail(GPS_ERR_TIMEOUT, "a device-side wait exceeded its budget (flags 0x%x)", all);
     return GPS_OK;

@@ -47,6 +47,7 @@ struct alignas(128) WsHeader {
     unsigned long long stat_fallbacks;  // predecessor tiles re-reduced
     unsigned long long stat_inserts;    // fallback aggregates that won the CAS
     unsigned long long stat_stalls;     // tiles that were made to stall
+    uint64_t mid_launch;                // launch number of the one-tile-per-CTA kernels
 };
 static_assert(sizeof(WsHeader) == 128, "header is one 128-byte line");
 
@@ -113,6 +114,7 @@ struct ScanArgs {
     void* carry_out;       // optional: receives carry_in + sum of all n inputs
     uint64_t wait_budget_ns;
     StallConfig stall;
+    uint64_t* mid_launch;  // one-tile-per-CTA kernels: WsHeader::mid_launch
 };
 
 // Kernel geometry shared by host and device: RW reduce warps and RW finalize

@@ -18,14 +18,6 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
     return t;
 }
 
-// Id of the running grid: unique among the launches of a CUDA context, graph
-// replays included.
-__device__ __forceinline__ uint64_t grid_id() {
-    uint64_t g;
-    asm volatile("mov.u64 %0, %%gridid;" : "=l"(g));
-    return g;
-}
-
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count)

@@ -15,12 +15,15 @@
 //      groups;
 //   4. publish the inclusive prefix, add the prefix, store.
 // The kernels keep their descriptors in a region of the plan of their own,
-// tagged with the launch's grid id (%gridid: a 64-bit number the driver gives
-// every grid launched in a CUDA context, graph replays included). A
-// descriptor counts only when its tag is the current launch's, so a launch
-// needs neither a clearing memset nor an end-of-launch retirement (the last
-// CTA resetting counters and advancing an epoch): no atomic and no fence on
-// any CTA's path.
+// tagged with the launch's number, which every CTA reads from the plan's
+// header beside its data loads. A descriptor counts only when its tag is the
+// current launch's, so a launch needs no clearing memset. The last tile's CTA
+// advances the number once its own prefix is known: that prefix rests on a
+// descriptor of every tile before it, each written by a CTA that had read the
+// number, so no CTA of this launch can still be about to read it. No atomic
+// and no fence is on any CTA's path. (A number from the driver will not do:
+// %gridid is fixed when a graph is instantiated, the same for all its
+// replays.)
 #include "gps_device.cuh"
 #include "gps_internal.h"
 #include "launch_util.h"
@@ -35,23 +38,22 @@ constexpr int kMidCtasPerSm = 8;
 
 // ------------------------------------------------------------ descriptors
 // One 16-byte word per tile: {lo: the value (u32 or u64), hi: status:2 |
-// grid id:62}. Zeroed memory reads "not ready". 2^62 launches would have to
-// pass in one context before a stale tag could come round again. Tile t's
+// launch number:62}. Zeroed memory reads "not ready". Tile t's
 // word is word t * a.desc_stride of the region: launches of more than one
 // group of tiles give each tile a 128-byte line of its own, since tiles that
 // publish while others read the same line waited up to 3 us for a read.
 // Group descriptors always have a line each (word g * kMidDescStride).
-constexpr uint64_t kGidMask = (1ull << 62) - 1;
+constexpr uint64_t kTagMask = (1ull << 62) - 1;
 
 struct MidDesc {
-    __device__ static ptx::u64x2 pack(uint32_t status, uint64_t gid, uint64_t v) {
+    __device__ static ptx::u64x2 pack(uint32_t status, uint64_t tag, uint64_t v) {
         ptx::u64x2 w;
         w.lo = v;
-        w.hi = (static_cast<uint64_t>(status) << 62) | (gid & kGidMask);
+        w.hi = (static_cast<uint64_t>(status) << 62) | (tag & kTagMask);
         return w;
     }
-    __device__ static uint32_t status(const ptx::u64x2& w, uint64_t gid) {
-        return (w.hi & kGidMask) == (gid & kGidMask) ? static_cast<uint32_t>(w.hi >> 62) : kNotReady;
+    __device__ static uint32_t status(const ptx::u64x2& w, uint64_t tag) {
+        return (w.hi & kTagMask) == (tag & kTagMask) ? static_cast<uint32_t>(w.hi >> 62) : kNotReady;
     }
 };
 
@@ -83,7 +85,7 @@ struct LookbackSmem {
 // Gives up after the wait budget, setting timed_out (then `sum` is 0).
 template <typename T, uint32_t SPIN = 64>
 __device__ bool warp_window(const ScanArgs& a, const ptx::u64x2* d, uint32_t stride, int64_t top, int64_t floor,
-                            uint64_t gid, uint32_t lane, T& sum, bool& timed_out) {
+                            uint64_t tag, uint32_t lane, T& sum, bool& timed_out) {
     const int64_t idx = top - static_cast<int64_t>(lane);
     bool ready = idx < floor, incl = false;
     T v = 0;
@@ -93,7 +95,7 @@ __device__ bool warp_window(const ScanArgs& a, const ptx::u64x2* d, uint32_t str
     while (true) {
         if (!ready) {
             const ptx::u64x2 w = ptx::ld_relaxed_b128(d + idx * stride);
-            const uint32_t st = MidDesc::status(w, gid);
+            const uint32_t st = MidDesc::status(w, tag);
             if (st != kNotReady) {
                 ready = true;
                 v = static_cast<T>(w.lo);
@@ -134,7 +136,7 @@ __device__ bool warp_window(const ScanArgs& a, const ptx::u64x2* d, uint32_t str
 // thread. `total` is the tile's sum, known to every thread. Warp 0 looks
 // back; a barrier hands its result to the CTA.
 template <typename T>
-__device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint64_t gid, T total, LookbackSmem& sm,
+__device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint64_t tag, T total, LookbackSmem& sm,
                                              T* s_pre) {
     ptx::u64x2* d1 = static_cast<ptx::u64x2*>(a.desc);
     ptx::u64x2* d2 = static_cast<ptx::u64x2*>(a.group_desc);
@@ -145,23 +147,25 @@ __device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint
     const bool group_last = (t % kGroupTiles) == kGroupTiles - 1;
     if (t == 0) {
         if (tid == 0) {
-            ptx::st_relaxed_b128(d1, MidDesc::pack(kInclusive, gid, static_cast<uint64_t>(carry + total)));
-            if (a.carry_out != nullptr && a.num_tiles == 1) *static_cast<T*>(a.carry_out) = carry + total;
+            if (a.num_tiles > 1)
+                ptx::st_relaxed_b128(d1, MidDesc::pack(kInclusive, tag, static_cast<uint64_t>(carry + total)));
+            else if (a.carry_out != nullptr)
+                *static_cast<T*>(a.carry_out) = carry + total;
         }
         return carry;
     }
     if (tid < 32) {
         const uint32_t lane = tid;
         if (lane == 0)
-            ptx::st_relaxed_b128(d1 + t * s1, MidDesc::pack(kAggregate, gid, static_cast<uint64_t>(total)));
+            ptx::st_relaxed_b128(d1 + t * s1, MidDesc::pack(kAggregate, tag, static_cast<uint64_t>(total)));
         // The tiles of this group before t; tile 0 is inclusive, so group 0
         // always finds one.
         T in_sum;
         bool timed_out;
         const bool found = warp_window<T>(a, d1, s1, static_cast<int64_t>(t) - 1,
-                                          static_cast<int64_t>(g) * kGroupTiles, gid, lane, in_sum, timed_out);
+                                          static_cast<int64_t>(g) * kGroupTiles, tag, lane, in_sum, timed_out);
         if (lane == 0 && group_last && !timed_out)
-            ptx::st_relaxed_b128(d2 + g * kMidDescStride, MidDesc::pack(found ? kInclusive : kAggregate, gid,
+            ptx::st_relaxed_b128(d2 + g * kMidDescStride, MidDesc::pack(found ? kInclusive : kAggregate, tag,
                                                        static_cast<uint64_t>(in_sum + total)));
         // No inclusive tile in the group before t: the prefix of the group, a
         // decoupled lookback over the group descriptors, 32 per poll.
@@ -170,7 +174,7 @@ __device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint
             int64_t top = static_cast<int64_t>(g) - 1;
             while (true) {
                 T part;
-                const bool gf = warp_window<T>(a, d2, kMidDescStride, top, 0, gid, lane, part, timed_out);
+                const bool gf = warp_window<T>(a, d2, kMidDescStride, top, 0, tag, lane, part, timed_out);
                 if (timed_out) break;
                 gsum += part;
                 if (gf || top < 32) break;  // group 0's descriptor is inclusive
@@ -178,6 +182,7 @@ __device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint
             }
         }
         if (lane == 0) {
+            if (t == a.num_tiles - 1 && !timed_out) ptx::st_relaxed_u64(a.mid_launch, tag + 1);
             s_pre[0] = in_sum + gsum;
             sm.timeout = timed_out ? 1u : 0u;
             sm.found = found ? 1u : 0u;
@@ -190,9 +195,9 @@ __device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint
     }
     const T pre = s_pre[0];
     if (tid == 0) {
-        ptx::st_relaxed_b128(d1 + t * s1, MidDesc::pack(kInclusive, gid, static_cast<uint64_t>(pre + total)));
+        ptx::st_relaxed_b128(d1 + t * s1, MidDesc::pack(kInclusive, tag, static_cast<uint64_t>(pre + total)));
         if (group_last && sm.found == 0)
-            ptx::st_relaxed_b128(d2 + g * kMidDescStride, MidDesc::pack(kInclusive, gid, static_cast<uint64_t>(pre + total)));
+            ptx::st_relaxed_b128(d2 + g * kMidDescStride, MidDesc::pack(kInclusive, tag, static_cast<uint64_t>(pre + total)));
         if (a.carry_out != nullptr && t == a.num_tiles - 1) *static_cast<T*>(a.carry_out) = pre + total;
     }
     return pre;
@@ -275,7 +280,8 @@ __global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm) mid_vec_kernel(con
     const uint32_t lane = tid & 31u;
     const uint32_t warp = tid >> 5;
     const uint32_t t = blockIdx.x;
-    const uint64_t gid = ptx::grid_id();
+    // Only warp 0 uses the launch number; its load overlaps the tile's.
+    const uint64_t tag = threadIdx.x < 32 ? ptx::ld_relaxed_u64(a.mid_launch) : 0;
     const uint64_t t0 = static_cast<uint64_t>(t) * TILE;
     // Elements of the input before virtual element `lead` do not exist.
     const uint32_t lead =
@@ -330,7 +336,7 @@ __global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm) mid_vec_kernel(con
         for (int r = 0; r < ROWS; ++r) s_off[r][tid] = cs[r] + __shfl_sync(kFullMask, xe, r * WARPS + warp);
     }
 
-    const T base = mid_tile_prefix<T>(a, t, gid, total, lsm, s_pre);
+    const T base = mid_tile_prefix<T>(a, t, tag, total, lsm, s_pre);
 
     auto scan_chunk = [&](int r, Chunk<T>& q) {
         T acc = base + s_off[r][tid];
