@@ -62,15 +62,17 @@ struct gps_plan_s {
     // same region after the unit descriptors (so that the epoch-wrap clear
     // covers them).
     void* group_desc16;
-    // Integer chained-scan plans: the 16-byte, launch-tagged descriptors of
-    // the one-tile-per-CTA kernels (mid.cu), one per tile; else null.
+    // Chained-scan plans: the 16-byte, launch-tagged descriptors of the
+    // one-tile-per-CTA kernels (mid.cu; mid_seg.cuh), and one per group of 32
+    // tiles; else null.
     void* desc_mid;
-    void* group_desc_mid;  // and one per group of 32 tiles
+    void* group_desc_mid;
     // Integer scans of at most this many elements run in one CTA (small.cu).
     uint64_t small_max;
     uint64_t mid_max;  // chained-scan plans: largest scan run as one tile per CTA
     // Autotuned launch configuration of the generic kernel per [segmented?]
-    // [size class] (index into gps::kGenericCandidates; -1: not tuned).
+    // [size class] (index into gps::kGenericCandidates, or kTunedMid for one
+    // tile per CTA; -1: not tuned).
     int8_t tuned[2][kSizeClasses];
     uint64_t wait_budget_ns;
     gps::StallConfig stall;
@@ -115,18 +117,30 @@ bool is_float(gps_dtype d) { return d == GPS_DTYPE_F32 || d == GPS_DTYPE_F32_COM
 // reduce-then-scan kernel of their own).
 bool generic_only(gps_dtype d) { return is_float(d) || d == GPS_DTYPE_U32X4; }
 
+// Value of gps_plan_s::tuned when the autotuner found one tile per CTA fastest.
+constexpr int kTunedMid = gps::kNumGenericCandidates;
+
 // Launch configuration of the generic kernel for a scan of n elements: the
 // autotuned one of the size class if there is one, else the default rule.
 gps::GenericConfig generic_config(const gps_plan_s* p, bool segmented, uint64_t n) {
     const int c = p->tuned[segmented ? 1 : 0][size_class(n)];
     if (c >= 0 && c < gps::kNumGenericCandidates) return gps::kGenericCandidates[c];
+    const uint64_t tiles = (n + p->tile_elems - 1) / p->tile_elems;
+    if (tiles <= (c == kTunedMid ? gps::kMidSegMaxTiles : gps::mid_seg_default_tiles(segmented)))
+        return gps::kMidSegConfig;
     return gps::default_generic_config(n, p->tile_elems, p->num_sms);
 }
 
-// Generic kernel (scan_seg.cuh): floating-point scans and batched scans.
-cudaError_t launch_generic(gps_dtype dtype, bool inclusive, const gps::ScanArgs& a, const gps::SegArgs* sg,
-                           const gps::GenericConfig& cfg, int num_sms, cudaStream_t stream, gps::LaunchInfo* info) {
-    switch (dtype) {
+// Generic kernel (scan_seg.cuh, mid_seg.cuh): floating-point scans and batched
+// scans. The launch's descriptors are the plan's for the configuration.
+cudaError_t launch_generic(const gps_plan_s* p, bool inclusive, gps::ScanArgs a, const gps::SegArgs* sg,
+                           const gps::GenericConfig& cfg, cudaStream_t stream, gps::LaunchInfo* info) {
+    const int num_sms = p->num_sms;
+    a.hdr = p->hdr16;
+    a.mid_launch = &p->hdr->mid_launch;
+    a.desc = cfg.unit == 0 ? p->desc_mid : p->desc16;
+    a.group_desc = cfg.unit == 0 ? p->group_desc_mid : p->group_desc16;
+    switch (p->dtype) {
         case GPS_DTYPE_U32: return gps::launch_seg_u32(inclusive, a, sg, cfg, num_sms, stream, info);
         case GPS_DTYPE_U64: return gps::launch_seg_u64(inclusive, a, sg, cfg, num_sms, stream, info);
         case GPS_DTYPE_F32: return gps::launch_seg_f32(inclusive, a, sg, cfg, num_sms, stream, info);
@@ -177,16 +191,12 @@ gps_status launch_scan(gps_plan_s* p, bool inclusive, const void* in, void* out,
     a.stall = p->stall;
     a.mid_launch = &p->hdr->mid_launch;
     // The persistent kernel for buffers off a 16-byte boundary moves single
-    // elements; one tile per CTA is faster at every size (2^25 u32 elements:
-    // 64 against 527 us, 2^27: 258 against 2017).
+    // elements; one tile per CTA is faster at every size (2^27 u32 elements:
+    // 258 against 2017 us).
     const bool unaligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) != 0;
     cudaError_t err;
     if (generic_only(p->dtype)) {
-        a.hdr = p->hdr16;
-        a.desc = p->desc16;
-        a.group_desc = p->group_desc16;
-        err = launch_generic(p->dtype, inclusive, a, nullptr, generic_config(p, false, n), p->num_sms, stream,
-                             &p->last_launch);
+        err = launch_generic(p, inclusive, a, nullptr, generic_config(p, false, n), stream, &p->last_launch);
     } else if (n <= p->small_max && p->stall.mode == 0 && p->stall.fallback_polls == 0) {
         err = gps::launch_small(p->dtype, inclusive, a, stream, &p->last_launch);
     } else if (p->algo == GPS_ALGO_CSDL && (n <= p->mid_max || (unaligned && p->mid_max != 0)) &&
@@ -313,18 +323,21 @@ gps_status gps_plan_create(gps_plan* out_plan, gps_algo algo, gps_dtype dtype, u
     // use the generic kernel's 16-byte descriptors, kept in a region of their
     // own so that the two formats never meet in one slot.
     const uint64_t slots16 = (algo == GPS_ALGO_CSDL && dtype == GPS_DTYPE_U32) ? seg_units + seg_groups : 0;
-    // One-tile-per-CTA kernels of integer chained-scan plans: 16-byte
-    // descriptors tagged with the launch, in a region no other kernel uses.
-    const uint64_t slots_mid = (algo == GPS_ALGO_CSDL && !generic_only(dtype)) ? tiles + gps::kDescPad : 0;
-    const uint64_t groups_mid = slots_mid ? (tiles + 31) / 32 + gps::kDescPad : 0;
+    // One-tile-per-CTA kernels of chained-scan plans: 16-byte descriptors
+    // tagged with the launch, in a region no other kernel uses (for types
+    // without an integer kernel, only as many as the generic one takes).
+    const uint64_t tiles_mid =
+        generic_only(dtype) ? std::min<uint64_t>(tiles, gps::kMidSegMaxTiles) : tiles;
+    const uint64_t slots_mid = algo == GPS_ALGO_CSDL ? tiles_mid + gps::kDescPad : 0;
+    const uint64_t groups_mid = slots_mid ? (tiles_mid + 31) / 32 + gps::kDescPad : 0;
     // [header][carries][descriptors or tile sums]; for u32 chained-scan
     // plans, [256-byte aligned: generic header][16-byte descriptors]; for
-    // integer chained-scan plans, [256-byte aligned: mid-size descriptors].
+    // all chained-scan plans, [256-byte aligned: mid-size descriptors].
     const size_t main_bytes = kHeaderBytes + kCarryBytes + slots * per_tile;
     const size_t region16 = (main_bytes + 255) & ~static_cast<size_t>(255);
     const size_t end16 = slots16 ? region16 + kHeaderBytes + slots16 * 16 : main_bytes;
     const size_t region_mid = (end16 + 255) & ~static_cast<size_t>(255);
-    const uint64_t words_mid = slots_mid ? gps::mid_desc_words(tiles) : 0;
+    const uint64_t words_mid = slots_mid ? gps::mid_desc_words(tiles_mid) : 0;
     p->scratch_bytes = slots_mid ? region_mid + (words_mid + groups_mid * gps::kMidDescStride) * 16 : end16;
     err = cudaMalloc(&p->scratch, p->scratch_bytes);
     if (err != cudaSuccess) {
@@ -450,9 +463,6 @@ gps_status prepare_generic(gps_plan_s* p, gps_scan_kind kind, const void* d_in, 
     a->out = d_out;
     a->n = n;
     a->num_tiles = static_cast<uint32_t>((n + p->tile_elems - 1) / p->tile_elems);
-    a->hdr = p->hdr16;
-    a->desc = p->desc16;
-    a->group_desc = p->group_desc16;
     a->wait_budget_ns = p->wait_budget_ns;
     *sg = gps::SegArgs{d_offsets, static_cast<uint32_t>(num_segments)};
     return GPS_OK;
@@ -467,8 +477,8 @@ gps_status gps_scan_segmented(gps_plan p, gps_scan_kind kind, const void* d_in, 
     gps::SegArgs sg;
     gps_status st = prepare_generic(p, kind, d_in, d_out, n, d_offsets, num_segments, &a, &sg);
     if (st != GPS_OK || n == 0) return st;
-    const cudaError_t err = launch_generic(p->dtype, kind == GPS_SCAN_INCLUSIVE, a, &sg, generic_config(p, true, n),
-                                           p->num_sms, reinterpret_cast<cudaStream_t>(stream), &p->last_launch);
+    const cudaError_t err = launch_generic(p, kind == GPS_SCAN_INCLUSIVE, a, &sg, generic_config(p, true, n),
+                                           reinterpret_cast<cudaStream_t>(stream), &p->last_launch);
     if (err != cudaSuccess) return cuda_fail(err, "batched scan launch");
     return GPS_OK;
 }
@@ -502,13 +512,14 @@ gps_status gps_plan_autotune(gps_plan p, gps_scan_kind kind, const void* d_in, v
     if (err == cudaSuccess) err = cudaEventCreate(&e1);
     int best = -1, rejected = 0;
     float best_ms = 0.0f;
-    for (int c = 0; c < gps::kNumGenericCandidates && err == cudaSuccess; ++c) {
-        const gps::GenericConfig& cfg = gps::kGenericCandidates[c];
+    for (int c = 0; c <= kTunedMid && err == cudaSuccess; ++c) {
+        const gps::GenericConfig cfg = c == kTunedMid ? gps::kMidSegConfig : gps::kGenericCandidates[c];
+        if (c == kTunedMid && a.num_tiles > gps::kMidSegMaxTiles) break;
         if (!generic_config_fits(p->dtype, cfg)) continue;  // this kernel shape does not fit the type
         gps::LaunchInfo info{};
         const gps::SegArgs* sgp = seg ? &sg : nullptr;
         const bool incl = kind == GPS_SCAN_INCLUSIVE;
-        err = launch_generic(p->dtype, incl, a, sgp, cfg, p->num_sms, s, &info);  // warm-up
+        err = launch_generic(p, incl, a, sgp, cfg, s, &info);  // warm-up
         if (err == cudaSuccess && check) {
             err = hash_buffer(d_out, out_bytes, d_hash, s);
             if (err == cudaSuccess) err = cudaMemcpyAsync(&hash, d_hash, sizeof(hash), cudaMemcpyDeviceToHost, s);
@@ -520,7 +531,7 @@ gps_status gps_plan_autotune(gps_plan p, gps_scan_kind kind, const void* d_in, v
         }
         if (err == cudaSuccess) err = cudaEventRecord(e0, s);
         for (int r = 0; r < 3 && err == cudaSuccess; ++r)
-            err = launch_generic(p->dtype, incl, a, sgp, cfg, p->num_sms, s, &info);
+            err = launch_generic(p, incl, a, sgp, cfg, s, &info);
         if (err == cudaSuccess) err = cudaEventRecord(e1, s);
         if (err == cudaSuccess) err = cudaEventSynchronize(e1);
         float ms = 0.0f;
@@ -540,13 +551,11 @@ gps_status gps_plan_autotune(gps_plan p, gps_scan_kind kind, const void* d_in, v
     if (err != cudaSuccess) return cuda_fail(err, "autotuning");
     if (best < 0) return fail(GPS_ERR_CUDA, "autotuning: no launch configuration ran");
     // Leave a correct result in d_out, from the chosen configuration.
-    err = launch_generic(p->dtype, kind == GPS_SCAN_INCLUSIVE, a, seg ? &sg : nullptr, gps::kGenericCandidates[best],
-                         p->num_sms, s, &p->last_launch);
+    err = launch_generic(p, kind == GPS_SCAN_INCLUSIVE, a, seg ? &sg : nullptr,
+                         best == kTunedMid ? gps::kMidSegConfig : gps::kGenericCandidates[best], s, &p->last_launch);
     if (err != cudaSuccess) return cuda_fail(err, "autotuning");
     p->tuned[seg ? 1 : 0][size_class(n)] = static_cast<int8_t>(best);
-    if (out_unit) *out_unit = gps::kGenericCandidates[best].unit;
-    if (out_ctas) *out_ctas = gps::kGenericCandidates[best].ctas_div;
-    if (out_threads_per_row) *out_threads_per_row = gps::kGenericCandidates[best].split;
+    gps_plan_generic_config(p, seg ? 1 : 0, n, out_unit, out_ctas, out_threads_per_row, nullptr);
     st = gps_plan_check(p, stream);
     if (st != GPS_OK) return st;
     if (rejected != 0)
@@ -576,7 +585,10 @@ gps_status gps_plan_set_generic_config(gps_plan p, int segmented, uint64_t n, ui
 gps_status gps_plan_generic_config(gps_plan p, int segmented, uint64_t n, uint32_t* out_unit, uint32_t* out_ctas_div,
                                    uint32_t* out_threads_per_row, int* out_tuned) {
     if (p == nullptr) return fail(GPS_ERR_INVALID_ARGUMENT, "plan is NULL");
-    const gps::GenericConfig cfg = generic_config(p, segmented != 0, n);
+    gps::GenericConfig cfg = generic_config(p, segmented != 0, n);
+    // One tile per CTA has no units: report the default of the kernel with
+    // units, a configuration gps_plan_set_generic_config() takes.
+    if (cfg.unit == 0) cfg = gps::default_generic_config(n, p->tile_elems, p->num_sms);
     if (out_unit) *out_unit = cfg.unit;
     if (out_ctas_div) *out_ctas_div = cfg.ctas_div;
     if (out_threads_per_row) *out_threads_per_row = cfg.split;

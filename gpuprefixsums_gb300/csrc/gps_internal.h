@@ -166,7 +166,8 @@ cudaError_t encode_row_maps(const void* in, void* out, uint64_t n, uint32_t elem
 // 4; the unit is what one CTA takes from the work counter), the CTA count as
 // a fraction of the resident maximum (1 = all, 2 = half), and threads per
 // 128-byte row of a tile (1: 4 reduce and 4 finalize warps, each thread
-// scanning 128 bytes; 2: 8 and 8, each thread scanning 64 bytes).
+// scanning 128 bytes; 2: 8 and 8, each thread scanning 64 bytes). A unit of 0
+// stands for one tile per CTA (mid_seg.cuh).
 struct GenericConfig {
     uint32_t unit;
     uint32_t ctas_div;
@@ -245,6 +246,20 @@ constexpr uint64_t mid_desc_words(uint64_t tiles) {
     const uint64_t strided = ((tiles < kMidStrideMaxTiles ? tiles : kMidStrideMaxTiles) + kDescPad) * kMidDescStride;
     return tiles + kDescPad > strided ? tiles + kDescPad : strided;
 }
+// One-tile-per-CTA form of the generic kernel (mid_seg.cuh): tiles per group
+// of its lookback, and the most tiles it takes.
+constexpr uint32_t kMidSegGroup = 64;
+constexpr uint32_t kMidSegMaxTiles = 4096;
+static_assert(kMidSegGroup >= 32 && kMidSegMaxTiles <= kMidStrideMaxTiles, "within the plan's mid-size descriptors");
+constexpr GenericConfig kMidSegConfig = {0, 1, 1};
+// Untuned scans of up to this many tiles take it; larger ones the kernel with
+// units, whose pipeline then pays. Measured on GB300 (graph replay, us, one tile
+// per CTA against the better unit size): FP32 1024 tiles 12.4 / 15.5, 2048 tiles
+// 20.1 / 18.3; compensated 14.5 / 16.7 and 23.2 / 20.3; batched u32 12.5 / 18.2
+// and 19.9 / 20.9; batched u64 12.9 / 18.4 and 19.5 / 20.7; batched compensated
+// 16.0 / 21.0 and 25.4 / 25.4; structs 1024 tiles 16.5 / 17.3 (single-tile
+// units, the untuned choice there).
+constexpr uint64_t mid_seg_default_tiles(bool segmented) { return segmented ? 2048 : 1024; }
 cudaError_t launch_mid(gps_dtype dtype, bool inclusive, const ScanArgs& a, int num_sms, cudaStream_t stream,
                        LaunchInfo* info);
 

@@ -3,6 +3,7 @@
 // in parallel.
 #pragma once
 #include "launch_util.h"
+#include "mid_seg.cuh"
 #include "scan_seg.cuh"
 
 namespace gps {
@@ -79,6 +80,9 @@ template <class Op, int SPLIT>
 cudaError_t launch_seg_op(bool inclusive, const ScanArgs& a, const SegArgs* sg, const GenericConfig& cfg, int num_sms,
                           cudaStream_t stream, LaunchInfo* info) {
     if (cfg.split != static_cast<uint32_t>(SPLIT)) return cudaErrorInvalidValue;
+    if constexpr (SPLIT == 1) {
+        if (cfg.unit == 0) return launch_mid_seg<Op>(inclusive, a, sg, stream, info);
+    }
     switch (cfg.unit) {
         case 1: return launch_seg_unit<Op, 1, SPLIT>(inclusive, a, sg, cfg, num_sms, stream, info);
         case 4: return launch_seg_unit<Op, 4, SPLIT>(inclusive, a, sg, cfg, num_sms, stream, info);

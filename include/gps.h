@@ -57,9 +57,9 @@ typedef enum gps_dtype {
     GPS_DTYPE_U64 = 1, /* uint64_t, sums wrap mod 2^64 */
     /* float, plain FP32 arithmetic throughout (GPS_ALGO_CSDL only). The
      * floating-point scans sum in an order fixed by n, the segments and the
-     * launch configuration (gps_plan_generic_config), never by timing: two
-     * runs with the same inputs and configuration give bitwise-identical
-     * outputs. */
+     * launch configuration (untuned, autotuned or set by hand; see
+     * gps_plan_generic_config), never by timing: two runs with the same inputs
+     * on plans configured alike give bitwise-identical outputs. */
     GPS_DTYPE_F32 = 2,
     /* float in and out; each partial sum carries a TwoSum error term through
      * the thread, warp and block scans, and the value passed between lookback
@@ -166,9 +166,11 @@ gps_status gps_select_flagged(gps_plan plan, const void* d_in, const uint8_t* d_
  * against the first candidate's (a 64-bit hash computed on the device):
  * a configuration whose result differs is not taken and the call returns
  * GPS_ERR_CUDA after tuning with the others. A shape that does not fit one
- * CTA's shared memory for the element type is skipped. Without tuning a
- * size class uses one thread per row and units of 4 tiles once there are
- * two such units per SM, else 1 tile. d_out is left holding a correct
+ * CTA's shared memory for the element type is skipped. Up to 4096 tiles the
+ * one-tile-per-CTA form of the kernel is a candidate too. Without tuning, scans
+ * of up to 1024 tiles (batched: 2048) take that form; larger ones use one
+ * thread per row and units of 4 tiles once there are two such units per SM,
+ * else 1 tile. d_out is left holding a correct
  * result. Synchronizes `stream`; not allowed while the stream is being
  * captured. The chosen configuration is returned in out_unit /
  * out_ctas_div / out_threads_per_row (any may be NULL).
@@ -181,7 +183,10 @@ gps_status gps_plan_autotune(gps_plan plan, gps_scan_kind kind, const void* d_in
 /* Launch configuration a batched (segmented != 0) or plain generic-kernel
  * scan of n elements would use now: tiles per unit, CTA divisor (1: one CTA
  * per SM, 2: half), threads per row (1 or 2), and whether it comes from
- * gps_plan_autotune() or gps_plan_set_generic_config(). */
+ * gps_plan_autotune() or gps_plan_set_generic_config(). Where the
+ * one-tile-per-CTA form would run (untuned at small sizes, or the autotuner's
+ * choice), which has no such units, this is the untuned configuration of the
+ * kernel with units. */
 gps_status gps_plan_generic_config(gps_plan plan, int segmented, uint64_t n, uint32_t* out_unit,
                                    uint32_t* out_ctas_div, uint32_t* out_threads_per_row, int* out_tuned);
 
