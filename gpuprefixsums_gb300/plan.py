@@ -19,10 +19,28 @@ _DTYPES = {"u32": (_lib.DTYPE_U32, 4, 1), "u64": (_lib.DTYPE_U64, 8, 1), "f32": 
            "f32c": (_lib.DTYPE_F32_COMPENSATED, 4, 1), "u32x4": (_lib.DTYPE_U32X4, 4, 4)}
 
 
+# torch.cuda.current_stream() builds a Stream object: 2.9 us a call on the
+# GB300's host, as long as the launch of a small scan; the handle alone takes
+# 0.1. Set on first use (which initialises CUDA in torch).
+_current_handle = None
+
+
+def _find_current_handle():
+    import torch
+    torch.cuda.current_stream()
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    device = getattr(torch._C, "_cuda_getDevice", None)
+    if raw is None or device is None:
+        return lambda: torch.cuda.current_stream().cuda_stream
+    return lambda: raw(device())
+
+
 def _stream_handle(stream) -> int:
     if stream is None:
-        import torch
-        return torch.cuda.current_stream().cuda_stream
+        global _current_handle
+        if _current_handle is None:
+            _current_handle = _find_current_handle()
+        return _current_handle()
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
@@ -69,14 +87,16 @@ class Plan:
     # -- scans
     def scan_ptr(self, in_ptr: int, out_ptr: int, n: int, inclusive: bool = False, stream=None) -> None:
         kind = _lib.INCLUSIVE if inclusive else _lib.EXCLUSIVE
-        check(lib.gps_scan(self._h, kind, ctypes.c_void_p(in_ptr), ctypes.c_void_p(out_ptr), int(n),
-                           ctypes.c_void_p(_stream_handle(stream))), "gps_scan")
+        status = lib.gps_scan(self._h, kind, in_ptr, out_ptr, int(n), _stream_handle(stream))
+        if status:
+            check(status, "gps_scan")
 
     def length(self, x) -> int:
         """Number of scanned elements in tensor x (structs for u32x4)."""
-        if x.numel() % self.members:
+        words = x.numel()
+        if words % self.members:
             raise ValueError(f"a {self.dtype} tensor holds a multiple of {self.members} words")
-        return x.numel() // self.members
+        return words // self.members
 
     def scan(self, x, out=None, inclusive: bool = False, n: int | None = None, stream=None):
         """Scan the first n elements of CUDA tensor x into out (allocated if None;
@@ -90,8 +110,9 @@ class Plan:
             out = torch.empty_like(x)
         if out.element_size() != self.elem_size or not out.is_contiguous():
             raise ValueError("out must be contiguous with the plan's element size")
-        count = self.length(x) if n is None else int(n)
-        if count > self.length(x) or count > self.length(out):
+        length = self.length(x)
+        count = length if n is None else int(n)
+        if count > length or count > (length if out is x else self.length(out)):
             raise ValueError("n exceeds the tensor length")
         self.scan_ptr(x.data_ptr(), out.data_ptr(), count, inclusive, stream)
         return out
@@ -109,9 +130,10 @@ class Plan:
             import torch
             out = torch.empty_like(x)
         kind = _lib.INCLUSIVE if inclusive else _lib.EXCLUSIVE
-        check(lib.gps_scan_segmented(self._h, kind, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(out.data_ptr()),
-                                     self.length(x), ctypes.c_void_p(offsets.data_ptr()), offsets.numel() - 1,
-                                     ctypes.c_void_p(_stream_handle(stream))), "gps_scan_segmented")
+        status = lib.gps_scan_segmented(self._h, kind, x.data_ptr(), out.data_ptr(), self.length(x),
+                                        offsets.data_ptr(), offsets.numel() - 1, _stream_handle(stream))
+        if status:
+            check(status, "gps_scan_segmented")
         return out
 
     def select(self, x, flags, out=None, num_selected=None, stream=None):
@@ -119,19 +141,20 @@ class Plan:
         (uint8/bool CUDA tensor, same length) is non-zero, in order, into
         out[:count]; count (int64 CUDA tensor of one element) is written on
         the device. Returns (out, num_selected)."""
-        import torch
         if x.element_size() != self.elem_size or not (x.is_cuda and x.is_contiguous()):
             raise ValueError("x must be a contiguous CUDA tensor with the plan's element size")
         if flags.element_size() != 1 or flags.numel() != x.numel() or not (flags.is_cuda and flags.is_contiguous()):
             raise ValueError("flags must be a contiguous one-byte CUDA tensor as long as x")
         if out is None:
+            import torch
             out = torch.empty_like(x)
         if num_selected is None:
+            import torch
             num_selected = torch.zeros(1, dtype=torch.int64, device=x.device)
-        check(lib.gps_select_flagged(self._h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(flags.data_ptr()),
-                                     ctypes.c_void_p(out.data_ptr()), x.numel(),
-                                     ctypes.c_void_p(num_selected.data_ptr()), ctypes.c_void_p(_stream_handle(stream))),
-              "gps_select_flagged")
+        status = lib.gps_select_flagged(self._h, x.data_ptr(), flags.data_ptr(), out.data_ptr(), x.numel(),
+                                        num_selected.data_ptr(), _stream_handle(stream))
+        if status:
+            check(status, "gps_select_flagged")
         return out, num_selected
 
     def autotune(self, x, offsets=None, out=None, inclusive: bool = False, stream=None) -> dict:
