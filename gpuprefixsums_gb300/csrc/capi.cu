@@ -47,7 +47,7 @@ struct gps_plan_s {
     int num_sms;
     uint32_t tile_elems;
     uint64_t capacity_tiles;
-    void* scratch;        // WsHeader, then carry slots, then descriptors / tile sums
+    void* scratch;        // WsHeader, then carry slots, then descriptors / range sums
     size_t scratch_bytes;
     gps::WsHeader* hdr;
     void* carries;        // two elements (host-array scans)
@@ -184,7 +184,6 @@ gps_status launch_scan(gps_plan_s* p, bool inclusive, const void* in, void* out,
     a.num_tiles = static_cast<uint32_t>((n + p->tile_elems - 1) / p->tile_elems);
     a.hdr = p->hdr;
     a.desc = p->area;
-    a.spine = nullptr;
     a.carry_in = carry_in;
     a.carry_out = carry_out;
     a.wait_budget_ns = p->wait_budget_ns;
@@ -309,7 +308,7 @@ gps_status gps_plan_create(gps_plan* out_plan, gps_algo algo, gps_dtype dtype, u
         return cuda_fail(err, "device query");
     }
     // Chained scan: one descriptor per tile plus the lookback padding;
-    // reduce-then-scan: one tile sum per tile.
+    // reduce-then-scan: the range sums of three chunks.
     // Generic-kernel descriptors (packed, or one per line for launches of few
     // units) are followed by the group descriptors of its lookback; both are
     // counted in 16-byte words.
@@ -318,7 +317,7 @@ gps_status gps_plan_create(gps_plan* out_plan, gps_algo algo, gps_dtype dtype, u
     const uint64_t seg_units = gps::seg_desc_words(tiles, seg_dw), seg_groups = gps::seg_group_words(tiles, seg_dw);
     const uint64_t slots = algo == GPS_ALGO_CSDL ? (dtype != GPS_DTYPE_U32 ? (seg_units + seg_groups) / seg_dw
                                                                           : tiles + gps::kDescPad)
-                                                 : tiles;
+                                                 : gps::rts_scratch_elems(p->num_sms);
     // u32 chained-scan plans keep 8-byte descriptors; batched scans of them
     // use the generic kernel's 16-byte descriptors, kept in a region of their
     // own so that the two formats never meet in one slot.
@@ -330,7 +329,7 @@ gps_status gps_plan_create(gps_plan* out_plan, gps_algo algo, gps_dtype dtype, u
         generic_only(dtype) ? std::min<uint64_t>(tiles, gps::kMidSegMaxTiles) : tiles;
     const uint64_t slots_mid = algo == GPS_ALGO_CSDL ? tiles_mid + gps::kDescPad : 0;
     const uint64_t groups_mid = slots_mid ? (tiles_mid + 31) / 32 + gps::kDescPad : 0;
-    // [header][carries][descriptors or tile sums]; for u32 chained-scan
+    // [header][carries][descriptors or range sums]; for u32 chained-scan
     // plans, [256-byte aligned: generic header][16-byte descriptors]; for
     // all chained-scan plans, [256-byte aligned: mid-size descriptors].
     const size_t main_bytes = kHeaderBytes + kCarryBytes + slots * per_tile;
@@ -779,7 +778,7 @@ gps_status gps_plan_geometry(gps_plan p, uint64_t n, uint32_t* tile_elems, uint3
     if (tile_elems) *tile_elems = p->tile_elems;
     if (grid) *grid = static_cast<uint32_t>(p->last_launch.grid);
     const bool small = !generic_only(p->dtype) && n <= p->small_max && p->stall.mode == 0 && p->stall.fallback_polls == 0;
-    if (launches) *launches = n == 0 ? 0u : (small || p->algo == GPS_ALGO_CSDL ? 1u : 3u);
+    if (launches) *launches = n == 0 ? 0u : (small || p->algo == GPS_ALGO_CSDL ? 1u : gps::rts_launches(n, p->tile_elems, p->num_sms));
     return GPS_OK;
 }
 

@@ -22,10 +22,10 @@ constexpr int kCsdlWarps = 4;
 constexpr int kCsdlStages = 12;
 constexpr int kCsdlUnit = 4;  // tiles per lookback unit
 
-template <typename T, bool INCL, bool BULK, bool STALL>
+template <typename T, bool INCL>
 cudaError_t launch_csdl_t(const ScanArgs& a, int num_sms, cudaStream_t stream, LaunchInfo* info) {
     using Shape = TileShape<T, kCsdlWarps>;
-    auto kern = scan_pipeline_kernel<T, kCsdlWarps, kCsdlStages, kCsdlUnit, INCL, BULK, PrefixMode::Lookback, STALL>;
+    auto kern = scan_pipeline_kernel<T, kCsdlWarps, kCsdlStages, kCsdlUnit, INCL>;
     constexpr size_t smem = pipeline_smem_bytes<T, kCsdlWarps, kCsdlStages>();
     int occ = 0;
     cudaError_t err = resident_ctas_per_sm(kern, Shape::kThreads, smem, &occ);
@@ -87,11 +87,9 @@ cudaError_t prepare_csdl_t() {
     if (err == cudaSuccess) {
         using Shape = TileShape<T, kCsdlWarps>;
         constexpr size_t smem = pipeline_smem_bytes<T, kCsdlWarps, kCsdlStages>();
-        err = resident_ctas_per_sm(scan_pipeline_kernel<T, kCsdlWarps, kCsdlStages, kCsdlUnit, false, false,
-                                                        PrefixMode::Lookback, false>, Shape::kThreads, smem, &occ);
+        err = resident_ctas_per_sm(scan_pipeline_kernel<T, kCsdlWarps, kCsdlStages, kCsdlUnit, false>, Shape::kThreads, smem, &occ);
         if (err == cudaSuccess)
-            err = resident_ctas_per_sm(scan_pipeline_kernel<T, kCsdlWarps, kCsdlStages, kCsdlUnit, true, false,
-                                                            PrefixMode::Lookback, false>, Shape::kThreads, smem, &occ);
+            err = resident_ctas_per_sm(scan_pipeline_kernel<T, kCsdlWarps, kCsdlStages, kCsdlUnit, true>, Shape::kThreads, smem, &occ);
     }
     return err;
 }
@@ -110,8 +108,8 @@ cudaError_t dispatch_csdl(bool inclusive, bool stall, const ScanArgs& a, int num
     // The forced-stall test mode wants aligned buffers; the fallback alone
     // (stall mode 0) is a robustness option the ring kernel runs without.
     if (stall && a.stall.mode != 0) return cudaErrorInvalidValue;
-    return inclusive ? launch_csdl_t<T, true, false, false>(a, num_sms, stream, info)
-                     : launch_csdl_t<T, false, false, false>(a, num_sms, stream, info);
+    return inclusive ? launch_csdl_t<T, true>(a, num_sms, stream, info)
+                     : launch_csdl_t<T, false>(a, num_sms, stream, info);
 }
 
 }  // namespace

@@ -67,8 +67,6 @@ struct StallConfig {
     uint32_t pad_;
 };
 
-enum class PrefixMode : int { Lookback = 0, Spine = 1 };
-
 // Fixed-order lookback of the generic kernel (scan_seg.cuh): lookback units
 // per group, and the group descriptors a plan keeps for up to `units` units
 // (one more than the groups, as slack).
@@ -109,7 +107,6 @@ struct ScanArgs {
     // Descriptors of groups: of 32 tiles for the one-tile-per-CTA kernels, of
     // kDetGroupUnits lookback units for the generic kernel.
     void* group_desc;
-    const void* spine;   // inclusive scan of tile sums (reduce-then-scan)
     const void* carry_in;  // optional: one element added to every output
     void* carry_out;       // optional: receives carry_in + sum of all n inputs
     uint64_t wait_budget_ns;
@@ -149,8 +146,12 @@ cudaError_t launch_csdl(gps_dtype dtype, bool inclusive, bool stall_mode, const 
 // Sets up, without launching, every kernel launch_csdl() can pick for this
 // dtype without forced stalls, so that later launches make no set-up call.
 cudaError_t prepare_csdl(gps_dtype dtype);
-cudaError_t launch_rts(gps_dtype dtype, bool inclusive, const ScanArgs& a, void* tile_sums,
+cudaError_t launch_rts(gps_dtype dtype, bool inclusive, const ScanArgs& a, void* scratch,
                        int num_sms, cudaStream_t stream, LaunchInfo* info);
+// Elements of scratch a reduce-then-scan plan keeps, and the kernel launches
+// of a scan of n elements.
+uint64_t rts_scratch_elems(int num_sms);
+uint32_t rts_launches(uint64_t n, uint32_t tile_elems, int num_sms);
 // Tensor maps of the generic kernel: the buffer seen as rows of 128 bytes
 // (32 four-byte or 16 eight-byte elements), boxes of 128 rows (one 16 KB
 // tile), 128-byte swizzle. Rows past the last full row are the kernel's to

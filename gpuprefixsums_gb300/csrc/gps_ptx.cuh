@@ -18,6 +18,15 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
     return t;
 }
 
+// ------------------------------------------------ dependent launches
+// Waits until the kernels this grid depends on have completed and their
+// writes are visible; a no-op in a launch without the attribute.
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Lets the next kernel of the stream start once every CTA of this grid has
+// called this or exited; its own grid_dep_wait() still waits for this grid.
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count)
@@ -77,16 +86,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 }
 
 // ------------------------------------------------------- bulk (TMA) copies
-// global -> shared, completion counted on an mbarrier (bytes).
-__device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, uint32_t bytes,
-                                          uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-            smem_addr(smem_dst)),
-        "l"(gmem_src), "r"(bytes), "r"(smem_addr(bar))
-        : "memory");
-}
-
 // L2 cache policies for bulk copies: keep lines that will be read again,
 // drop lines read for the last time.
 __device__ __forceinline__ uint64_t policy_evict_last() {
@@ -144,13 +143,6 @@ __device__ __forceinline__ void bulk_store_hint(void* gmem_dst, const void* smem
                                                 uint64_t policy) {
     asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;" ::"l"(gmem_dst),
                  "r"(smem_addr(smem_src)), "r"(bytes), "l"(policy)
-                 : "memory");
-}
-
-// shared -> global, tracked as a bulk async-group of the issuing thread.
-__device__ __forceinline__ void bulk_store(void* gmem_dst, const void* smem_src, uint32_t bytes) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gmem_dst),
-                 "r"(smem_addr(smem_src)), "r"(bytes)
                  : "memory");
 }
 
@@ -242,13 +234,20 @@ __device__ __forceinline__ u64x2 atom_cas_b128(u64x2* p, u64x2 cmp, u64x2 val) {
     return old;
 }
 
-// Streaming 16-byte global accesses for the plain (non-bulk) paths.
-__device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
+// 16-byte global accesses past L1, with an L2 cache policy.
+__device__ __forceinline__ uint4 ld_policy_v4(const void* p, uint64_t policy) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p));
+                 : "l"(p), "l"(policy)
+                 : "memory");
     return v;
+}
+
+__device__ __forceinline__ void st_policy_v4(void* p, uint4 v, uint64_t policy) {
+    asm volatile("st.global.L1::no_allocate.L2::cache_hint.v4.u32 [%0], {%1,%2,%3,%4}, %5;" ::"l"(p), "r"(v.x),
+                 "r"(v.y), "r"(v.z), "r"(v.w), "l"(policy)
+                 : "memory");
 }
 
 }  // namespace ptx

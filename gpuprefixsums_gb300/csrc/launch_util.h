@@ -79,6 +79,25 @@ cudaError_t resident_ctas_per_sm(Kernel kern, int threads, size_t smem, int* out
     return cudaSuccess;
 }
 
+// Launches `kern` so that its CTAs may be set up before the kernel ahead of it
+// in the stream has finished; every such kernel calls ptx::grid_dep_wait()
+// before it touches global memory.
+template <typename... Params, typename... Args>
+cudaError_t launch_dependent(void (*kern)(Params...), int grid, int block, size_t smem, cudaStream_t stream,
+                             Args... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(grid));
+    cfg.blockDim = dim3(static_cast<unsigned>(block));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, Params(args)...);
+}
+
 // Persistent grid: as many CTAs as can be resident, but no more than tiles.
 inline int persistent_grid(uint32_t num_tiles, int ctas_per_sm, int num_sms) {
     const uint64_t cap = static_cast<uint64_t>(ctas_per_sm) * static_cast<uint64_t>(num_sms);

@@ -27,12 +27,12 @@
 #include "gps_device.cuh"
 #include "gps_internal.h"
 #include "launch_util.h"
-#include "scan_pipeline.cuh"
+#include "tile_rows.cuh"
 
 namespace gps {
 namespace {
 
-constexpr int kMidThreads = 256;
+constexpr int kMidThreads = kRowThreads;
 // Resident CTAs per SM the kernel is compiled for.
 constexpr int kMidCtasPerSm = 8;
 
@@ -218,57 +218,18 @@ __device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint
 // in one wave. There is no shared-memory staging and no mbarrier to set up,
 // so every CTA issues its loads as soon as it starts.
 //
-// ALIGNED = false takes buffers at any element offset from a 16-byte
-// boundary. Tiles are then counted from the boundary at or below the input
-// ("virtual" index j = i + lead, lead elements of tile 0 lying before the
-// input), so every load but those of the first and last chunk stays a 16-byte
-// one. The output's boundary may lie elsewhere: if virtual element 0 sits
-// `phase` elements past one, an output chunk is the last `phase` elements of
-// the chunk on the left (one shuffle each) and the first of this one, stored
-// as 16 bytes; a warp's two edges, tile 0 and a partial tile store elements.
+// ALIGNED = false takes buffers at any element offset from a 16-byte boundary
+// (tile_rows.cuh), one row at a time after the lookback, which keeps it at 32
+// registers.
 // Bound by the same latency chain as the aligned form. Measured on GB300,
 // 10,000,019 u32 from a view one element past a boundary, into an aligned
 // output: 22.9 us a call, where per-thread element loads and stores (64
 // bytes apart across a warp) took 70.9.
-template <typename T>
-__device__ __forceinline__ void store_elems(T* p, uint32_t off, uint32_t first, uint32_t cnt, const Chunk<T>& q) {
-    constexpr int EPC = 16 / static_cast<int>(sizeof(T));
-#pragma unroll
-    for (int e = 0; e < EPC; ++e)
-        if (off + e >= first && off + e < cnt) p[e] = q.v[e];
-}
-
-// Stores a warp's row of chunks of an interior tile, whose output lies P
-// elements past a 16-byte boundary; p is this lane's first output element.
-template <typename T, int P>
-__device__ __forceinline__ void store_shifted(T* p, uint32_t lane, const Chunk<T>& q) {
-    constexpr int EPC = 16 / static_cast<int>(sizeof(T));
-    Chunk<T> w;
-#pragma unroll
-    for (int e = 0; e < EPC; ++e) {
-        if (e < P)
-            w.v[e] = __shfl_up_sync(kFullMask, q.v[EPC - P + e], 1);
-        else
-            w.v[e] = q.v[e - P];
-    }
-    if (lane != 0) {
-        *reinterpret_cast<Chunk<T>*>(p - P) = w;
-    } else {
-#pragma unroll
-        for (int e = 0; e < EPC - P; ++e) p[e] = q.v[e];
-    }
-    if (lane == 31) {
-#pragma unroll
-        for (int e = EPC - P; e < EPC; ++e) p[e] = q.v[e];
-    }
-}
-
 template <typename T, bool INCL, bool ALIGNED>
 __global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm) mid_vec_kernel(const ScanArgs a) {
-    constexpr int TILE = 16384 / static_cast<int>(sizeof(T));
-    constexpr int EPC = 16 / static_cast<int>(sizeof(T));
-    constexpr int ROW = kMidThreads * EPC;  // elements per row
-    constexpr int ROWS = TILE / ROW;        // 4
+    using Rows = TileRows<T, ALIGNED>;
+    constexpr int EPC = Rows::kEpc;
+    constexpr int ROWS = Rows::kRows;
     constexpr int WARPS = kMidThreads / 32;
     static_assert(ROWS * WARPS == 32, "one warp scans all (row, warp) totals");
     __shared__ T s_tot[ROWS * WARPS];
@@ -282,33 +243,14 @@ __global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm) mid_vec_kernel(con
     const uint32_t t = blockIdx.x;
     // Only warp 0 uses the launch number; its load overlaps the tile's.
     const uint64_t tag = threadIdx.x < 32 ? ptx::ld_relaxed_u64(a.mid_launch) : 0;
-    const uint64_t t0 = static_cast<uint64_t>(t) * TILE;
-    // Elements of the input before virtual element `lead` do not exist.
-    const uint32_t lead =
-        ALIGNED ? 0u : static_cast<uint32_t>((reinterpret_cast<uintptr_t>(a.in) & 15u) / sizeof(T));
-    const uint32_t first = t == 0 ? lead : 0u;
-    // Elements of this tile; chunk (r, tid) starts at element r * ROW + tid * EPC.
-    const uint32_t cnt = static_cast<uint32_t>(min(static_cast<uint64_t>(TILE), a.n + lead - t0));
-    const bool full = cnt == static_cast<uint32_t>(TILE) && first == 0;
-    const T* src = static_cast<const T*>(a.in) - lead + t0 + tid * EPC;
-    T* dst = static_cast<T*>(a.out) - lead + t0 + tid * EPC;
-    auto load = [&](int r) -> Chunk<T> {
-        const uint32_t off = r * ROW + tid * EPC;
-        Chunk<T> q;
-        if (full || (off >= first && off + EPC <= cnt)) {
-            q = *reinterpret_cast<const Chunk<T>*>(src + r * ROW);
-        } else {
-#pragma unroll
-            for (int e = 0; e < EPC; ++e) q.v[e] = off + e >= first && off + e < cnt ? src[r * ROW + e] : T(0);
-        }
-        return q;
-    };
+    const Rows rows(a.in, a.out, a.n, t, tid);
+    constexpr PlainAccess access;
 
     T cs[ROWS];
     {
         Chunk<T> q[ROWS];
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) q[r] = load(r);
+        for (int r = 0; r < ROWS; ++r) q[r] = rows.load(r, access);
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
             T x = 0;
@@ -355,49 +297,28 @@ __global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm) mid_vec_kernel(con
     if constexpr (ALIGNED) {
         Chunk<T> q[ROWS];
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r) q[r] = load(r);
+        for (int r = 0; r < ROWS; ++r) q[r] = rows.load(r, access);
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
-            const uint32_t off = r * ROW + tid * EPC;
             scan_chunk(r, q[r]);
-            if (full || off + EPC <= cnt)
-                *reinterpret_cast<Chunk<T>*>(dst + r * ROW) = q[r];
-            else
-                store_elems(dst + r * ROW, off, 0u, cnt, q[r]);
+            rows.store(r, q[r], lane, access);
         }
     } else {
-        // Output elements past a 16-byte boundary (of this tile's first chunk,
-        // and so of every chunk). One row at a time, which keeps the kernel
-        // at 32 registers.
-        const uint32_t phase = static_cast<uint32_t>((reinterpret_cast<uintptr_t>(dst) & 15u) / sizeof(T));
 #pragma unroll 1
         for (int r = 0; r < ROWS; ++r) {
-            const uint32_t off = r * ROW + tid * EPC;
-            T* p = dst + r * ROW;
-            Chunk<T> q = load(r);
+            Chunk<T> q = rows.load(r, access);
             scan_chunk(r, q);
-            if (phase == 0 && (full || (off >= first && off + EPC <= cnt)))
-                *reinterpret_cast<Chunk<T>*>(p) = q;
-            else if (phase == 0 || !full)
-                store_elems(p, off, first, cnt, q);
-            else if (phase == 1)
-                store_shifted<T, 1>(p, lane, q);
-            else if (EPC == 4 && phase == 2)
-                store_shifted<T, EPC == 4 ? 2 : 1>(p, lane, q);
-            else
-                store_shifted<T, EPC == 4 ? 3 : 1>(p, lane, q);
+            rows.store(r, q, lane, access);
         }
     }
 }
 
 template <typename T, bool INCL, bool ALIGNED>
 cudaError_t launch_mid_v(const ScanArgs& a0, cudaStream_t stream, LaunchInfo* info) {
-    constexpr uint64_t TILE = 16384 / sizeof(T);
     ScanArgs a = a0;
-    // Tiles from the input's 16-byte boundary: at most one more than the
-    // plan's (its descriptor regions have kDescPad to spare).
-    const uint64_t lead = ALIGNED ? 0 : (reinterpret_cast<uintptr_t>(a.in) & 15u) / sizeof(T);
-    a.num_tiles = static_cast<uint32_t>((a.n + lead + TILE - 1) / TILE);
+    // At most one more than the plan's (its descriptor regions have kDescPad
+    // to spare).
+    a.num_tiles = TileRows<T, ALIGNED>::tiles(a.in, a.n);
     a.desc_stride = a.num_tiles > kGroupTiles && a.num_tiles <= kMidStrideMaxTiles ? kMidDescStride : 1u;
     const int grid = static_cast<int>(a.num_tiles);
     if (info) *info = LaunchInfo{grid, kMidThreads, 0};

@@ -1,146 +1,242 @@
-// Reduce-then-scan for u32 and u64: three launches, as in the reference's
-// ReduceThenScanDispatcher::DispatchKernels{Ex,In}clusive
-// (GPUPrefixSumsCUDA/ReduceThenScanDispatcher.cuh:165-187):
-//   1. reduce: one CTA per tile writes the tile's sum
-//      (ReduceThenScan::Reduce, ReduceThenScan.cuh:15-53);
-//   2. spine: one 1024-thread CTA scans the tile sums in place, inclusive
-//      (ReduceThenScan::SpineScan, ReduceThenScan.cuh:56-104);
-//   3. propagate: re-reads every tile, scans it and adds the spine value of
-//      the previous tile (ReduceThenScan::Propagate, ReduceThenScan.cuh:106-161),
-//      here the same bulk-copy pipeline kernel as the chained scan, fed from
-//      the spine instead of the lookback.
-// It reads the input twice (12 bytes per u32 element against 8 for the
-// single-pass scan) and keeps no inter-CTA waits.
+// Reduce-then-scan for u32 and u64, without inter-CTA waits, as in the
+// reference's ReduceThenScanDispatcher::DispatchKernels{Ex,In}clusive
+// (GPUPrefixSumsCUDA/ReduceThenScanDispatcher.cuh:165-187): reduce sums the
+// ranges of the input (ReduceThenScan::Reduce, ReduceThenScan.cuh:15-53), the
+// sums are scanned (ReduceThenScan::SpineScan, :56-104), propagate scans each
+// range from the prefix before it (ReduceThenScan::Propagate, :106-161).
+//
+// Read from HBM twice, the input alone would cost a half more than the
+// single-pass scan. Here it is cut into chunks that stay in L2 (129 MB)
+// between the two readings, and every launch but the first and last does the
+// reduce of one chunk and the propagate of the chunk before:
+//   launch 0      reduce chunk 0
+//   launch j      reduce chunk j, then propagate chunk j - 1
+//   launch K      propagate chunk K - 1
+// A chunk is one range of kRtsTiles 16 KB tiles for every resident CTA, so a
+// launch is one even wave. The spine is too short for a launch of its own:
+// each propagate CTA adds up the sums of the ranges before its own (at most
+// 3 a thread). The launches are dependent launches: a CTA reduces its range
+// of chunk j, which rests on no launch before, while the last CTAs of launch
+// j - 1 still propagate, and only then waits for that launch to finish.
+// Range sums and chunk prefixes therefore have three buffers each: launch
+// j + 1 writes while launch j reads, and launch j - 1 has finished by then.
+//
+// Bound by HBM (25 MB read and 25 written a launch, 7.5 us at the copy rate) and
+// the end of each launch: 9.7 us a launch. Measured on GB300, u32, against
+// three launches over the whole input (reduce, a one-CTA spine over one sum a
+// tile, propagate): 2^20 9.5 -> 5.1 us, 2^24 39 -> 32, 2^26 142 -> 109, 2^28
+// 542 -> 421; a view of 10,000,019 elements off a 16-byte boundary 167 -> 25.
 #include "launch_util.h"
-#include "scan_pipeline.cuh"
+#include "tile_rows.cuh"
 
 namespace gps {
 
 namespace {
 
-constexpr int kRtsWarps = 4;
-constexpr int kRtsStages = 6;
-constexpr int kReduceThreads = 256;
-constexpr int kSpineThreads = 1024;
-constexpr int kSpineItems = 8;
+constexpr int kRtsCtasPerSm = 5;
+// Tiles of a CTA's range in one chunk, at most: 25 MB a chunk. Two chunks wait
+// in L2 at a time, next to what is being written. Measured on GB300, 2^28 u32:
+// 2 tiles 421 us, 1 tile 516 (the end of a launch costs 2 us), 3 tiles 438 and
+// 4 463 (part of the chunk has left L2 by the second reading); 4 or 6 CTAs per
+// SM 438 and 430. Without evict-last loads in the reduce 491.
+constexpr uint32_t kRtsTiles = 2;
 
-template <typename T>
-__global__ void __launch_bounds__(kReduceThreads)
-    rts_reduce_kernel(const T* __restrict__ in, uint64_t n, T* __restrict__ tile_sums, uint32_t num_tiles,
-                      bool vec_ok) {
-    constexpr int TILE = TileShape<T, kRtsWarps>::kTile;
-    constexpr int EPC = 16 / static_cast<int>(sizeof(T));
-    constexpr int CHUNKS_PER_THREAD = TILE / EPC / kReduceThreads;
-    __shared__ T warp_sums[kReduceThreads / 32];
-    const uint32_t t = blockIdx.x;
-    const uint64_t base = static_cast<uint64_t>(t) * TILE;
-    const uint32_t cnt = tile_count<TILE>(n, t);
+struct RtsArgs {
+    const void* in;
+    void* out;
+    uint64_t n;
+    uint32_t tiles;
+    uint32_t range_tiles;  // tiles per range; a chunk is gridDim.x ranges
+    uint32_t chunk;        // this launch reduces it and propagates the one before
+    uint32_t chunks;
+    void* sums;      // [3][gridDim.x] range sums
+    void* prefixes;  // [3] sum of the chunks before
+    const void* carry_in;
+    void* carry_out;
+};
+
+template <typename T, bool INCL, bool ALIGNED>
+__global__ void __launch_bounds__(kRowThreads, kRtsCtasPerSm) rts_kernel(const RtsArgs a) {
+    using Rows = TileRows<T, ALIGNED>;
+    constexpr int ROWS = Rows::kRows;
+    constexpr int WARPS = kRowThreads / 32;
+    static_assert(ROWS * WARPS == 32, "one warp scans all (row, warp) totals");
+    __shared__ T s_tot[2][32];
+    __shared__ T s_pre[2][WARPS];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t ranges = gridDim.x, b = blockIdx.x;
+    T* sums = static_cast<T*>(a.sums);
+    T* prefixes = static_cast<T*>(a.prefixes);
+
+    if (a.chunk == 0) ptx::grid_dep_wait();  // the input's producers
+    // Reduce: one range of chunk a.chunk. L2 keeps what it reads.
     T acc = 0;
-    if (vec_ok && cnt == static_cast<uint32_t>(TILE)) {
-        const Chunk<T>* src = reinterpret_cast<const Chunk<T>*>(in + base);
-        Chunk<T> q[CHUNKS_PER_THREAD];
+    if (a.chunk < a.chunks) {
+        const PolicyAccess pol{ptx::policy_evict_last()};
+        const uint64_t begin = (static_cast<uint64_t>(a.chunk) * ranges + b) * a.range_tiles;
+        const uint64_t end = min(begin + a.range_tiles, static_cast<uint64_t>(a.tiles));
+#pragma unroll 2
+        for (uint64_t t = begin; t < end; ++t) {
+            const Rows rows(a.in, a.out, a.n, static_cast<uint32_t>(t), tid);
+            Chunk<T> q[ROWS];
 #pragma unroll
-        for (int k = 0; k < CHUNKS_PER_THREAD; ++k) {
-            const uint4 r = ptx::ld_stream_v4(src + threadIdx.x + k * kReduceThreads);
-            q[k] = *reinterpret_cast<const Chunk<T>*>(&r);
+            for (int r = 0; r < ROWS; ++r) q[r] = rows.load(r, pol);
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                for (int e = 0; e < Rows::kEpc; ++e) acc += q[r].v[e];
         }
+        acc = warp_sum(acc);
+        if (lane == 0) s_pre[0][warp] = acc;
+        __syncthreads();
+        if (tid == 0) {
+            T x = 0;
 #pragma unroll
-        for (int k = 0; k < CHUNKS_PER_THREAD; ++k)
-#pragma unroll
-            for (int e = 0; e < EPC; ++e) acc += q[k].v[e];
-    } else {
-        for (uint32_t i = threadIdx.x; i < cnt; i += kReduceThreads) acc += in[base + i];
+            for (int w = 0; w < WARPS; ++w) x += s_pre[0][w];
+            sums[(a.chunk % 3) * ranges + b] = x;
+        }
+        __syncthreads();
     }
-    acc = warp_sum(acc);
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    if (lane == 0) warp_sums[warp] = acc;
-    __syncthreads();
-    if (warp == 0) {
-        T x = lane < kReduceThreads / 32 ? warp_sums[lane] : T(0);
-        x = warp_sum(x);
-        if (lane == 0) tile_sums[t] = x;
+    if (a.chunk == 0) {
+        ptx::grid_dep_launch();
+        return;
+    }
+
+    // Propagate: the same range of the chunk before. Its first tile is loaded
+    // and scanned before the wait, which only guards the range sums.
+    const uint32_t c = a.chunk - 1;
+    const PolicyAccess pol{ptx::policy_evict_first()};
+    const uint64_t begin = (static_cast<uint64_t>(c) * ranges + b) * a.range_tiles;
+    const uint64_t end = min(begin + a.range_tiles, static_cast<uint64_t>(a.tiles));
+    T pre = 0;
+    for (uint64_t t = begin; t < end || t == begin; ++t) {
+        const bool live = t < end;  // a range past the end still takes part in the barriers
+        const Rows rows(a.in, a.out, a.n, static_cast<uint32_t>(live ? t : 0), tid);
+        Chunk<T> q[ROWS] = {};
+        if (live) {
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) q[r] = rows.load(r, pol);
+        }
+        T off[ROWS];
+        T* tot = s_tot[t & 1u];
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            T x = 0;
+#pragma unroll
+            for (int e = 0; e < Rows::kEpc; ++e) x += q[r].v[e];
+            const T inc = warp_inclusive_scan(x, lane);
+            if (lane == 31) tot[r * WARPS + warp] = inc;
+            off[r] = inc - x;
+        }
+        if (t == begin) {
+            ptx::grid_dep_wait();
+            ptx::grid_dep_launch();
+            const T* cs = sums + (c % 3) * ranges;
+            T mine = 0, all = 0;
+            for (uint32_t i = tid; i < ranges; i += kRowThreads) {
+                const T x = cs[i];
+                mine += i < b ? x : T(0);
+                all += x;
+            }
+            pre = c != 0 ? prefixes[c % 3] : a.carry_in != nullptr ? *static_cast<const T*>(a.carry_in) : T(0);
+            mine = warp_sum(mine);
+            if (b == 0) all = warp_sum(all);
+            if (lane == 0) {
+                s_pre[0][warp] = mine;
+                s_pre[1][warp] = all;
+            }
+        }
+        __syncthreads();
+        if (t == begin) {
+            if (b == 0 && tid == 0) {
+                T x = pre;
+#pragma unroll
+                for (int w = 0; w < WARPS; ++w) x += s_pre[1][w];
+                prefixes[(c + 1) % 3] = x;
+                if (a.chunk == a.chunks && a.carry_out != nullptr) *static_cast<T*>(a.carry_out) = x;
+            }
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) pre += s_pre[0][w];
+        }
+        if (!live) break;
+        // Every warp scans the 32 (row, warp) totals.
+        const T x = tot[lane];
+        const T xi = warp_inclusive_scan(x, lane);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            T run = pre + off[r] + __shfl_sync(kFullMask, xi - x, r * WARPS + warp);
+#pragma unroll
+            for (int e = 0; e < Rows::kEpc; ++e) {
+                const T y = q[r].v[e];
+                if (INCL) {
+                    run += y;
+                    q[r].v[e] = run;
+                } else {
+                    q[r].v[e] = run;
+                    run += y;
+                }
+            }
+            rows.store(r, q[r], lane, pol);
+        }
+        pre += __shfl_sync(kFullMask, xi, 31);
     }
 }
 
-// Inclusive scan of m tile sums in place by a single CTA, kSpineItems
-// consecutive sums per thread per pass.
-template <typename T>
-__global__ void __launch_bounds__(kSpineThreads) rts_spine_kernel(T* sums, uint32_t m) {
-    __shared__ T warp_tot[kSpineThreads / 32];
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    T carry = 0;
-    for (uint64_t pass = 0; pass < m; pass += static_cast<uint64_t>(kSpineThreads) * kSpineItems) {
-        T v[kSpineItems];
-        T run = 0;
-#pragma unroll
-        for (int i = 0; i < kSpineItems; ++i) {
-            const uint64_t idx = pass + static_cast<uint64_t>(tid) * kSpineItems + i;
-            const T x = idx < m ? sums[idx] : T(0);
-            run += x;
-            v[i] = run;
-        }
-        const T winc = warp_inclusive_scan(run, lane);
-        if (lane == 31) warp_tot[warp] = winc;
-        __syncthreads();
-        if (warp == 0) warp_tot[lane] = warp_inclusive_scan(warp_tot[lane], lane);
-        __syncthreads();
-        const T pre = carry + (warp ? warp_tot[warp - 1] : T(0)) + (winc - run);
-#pragma unroll
-        for (int i = 0; i < kSpineItems; ++i) {
-            const uint64_t idx = pass + static_cast<uint64_t>(tid) * kSpineItems + i;
-            if (idx < m) sums[idx] = pre + v[i];
-        }
-        carry += warp_tot[kSpineThreads / 32 - 1];
-        __syncthreads();
-    }
+// Ranges per chunk, tiles per range and chunks of a scan of `tiles` tiles:
+// the fewest chunks, cut evenly.
+struct RtsShape {
+    uint32_t ranges, range_tiles, chunks;
+};
+RtsShape rts_shape(uint32_t tiles, int num_sms) {
+    const uint32_t ranges = static_cast<uint32_t>(persistent_grid(tiles, kRtsCtasPerSm, num_sms));
+    const uint32_t per_range = (tiles + ranges - 1) / ranges;
+    const uint32_t chunks = (per_range + kRtsTiles - 1) / kRtsTiles;
+    const uint32_t range_tiles = (per_range + chunks - 1) / chunks;
+    return RtsShape{ranges, range_tiles, (per_range + range_tiles - 1) / range_tiles};
 }
 
-template <typename T, bool INCL, bool BULK>
-cudaError_t launch_propagate(const ScanArgs& a, int num_sms, cudaStream_t stream, LaunchInfo* info) {
-    using Shape = TileShape<T, kRtsWarps>;
-    auto kern = scan_pipeline_kernel<T, kRtsWarps, kRtsStages, 1, INCL, BULK, PrefixMode::Spine, false>;
-    constexpr size_t smem = pipeline_smem_bytes<T, kRtsWarps, kRtsStages>();
-    int occ = 0;
-    cudaError_t err = resident_ctas_per_sm(kern, Shape::kThreads, smem, &occ);
-    if (err != cudaSuccess) return err;
-    const int grid = persistent_grid(a.num_tiles, occ, num_sms);
-    if (info) *info = LaunchInfo{grid, Shape::kThreads, smem};
-    kern<<<grid, Shape::kThreads, smem, stream>>>(a);
-    return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t dispatch_rts(bool inclusive, const ScanArgs& a0, void* tile_sums, int num_sms, cudaStream_t stream,
+template <typename T, bool ALIGNED>
+cudaError_t dispatch_rts(bool inclusive, const ScanArgs& s, void* scratch, int num_sms, cudaStream_t stream,
                          LaunchInfo* info) {
-    const bool bulk = ((reinterpret_cast<uintptr_t>(a0.in) | reinterpret_cast<uintptr_t>(a0.out)) & 15u) == 0;
-    const bool in_vec = (reinterpret_cast<uintptr_t>(a0.in) & 15u) == 0;
-    T* sums = static_cast<T*>(tile_sums);
-    rts_reduce_kernel<T><<<a0.num_tiles, kReduceThreads, 0, stream>>>(static_cast<const T*>(a0.in), a0.n, sums,
-                                                                      a0.num_tiles, in_vec);
-    cudaError_t err = cudaGetLastError();
-    if (err != cudaSuccess) return err;
-    rts_spine_kernel<T><<<1, kSpineThreads, 0, stream>>>(sums, a0.num_tiles);
-    err = cudaGetLastError();
-    if (err != cudaSuccess) return err;
-    ScanArgs a = a0;
-    a.spine = sums;
-    if (bulk)
-        return inclusive ? launch_propagate<T, true, true>(a, num_sms, stream, info)
-                         : launch_propagate<T, false, true>(a, num_sms, stream, info);
-    return inclusive ? launch_propagate<T, true, false>(a, num_sms, stream, info)
-                     : launch_propagate<T, false, false>(a, num_sms, stream, info);
+    const uint32_t tiles = TileRows<T, ALIGNED>::tiles(s.in, s.n);
+    const RtsShape sh = rts_shape(tiles, num_sms);
+    T* sums = static_cast<T*>(scratch);
+    RtsArgs a{s.in,      s.out, s.n,       tiles,
+              sh.range_tiles, 0,     sh.chunks, sums,
+              sums + 3ull * static_cast<uint64_t>(kRtsCtasPerSm * num_sms), s.carry_in, s.carry_out};
+    const int grid = static_cast<int>(sh.ranges);
+    if (info) *info = LaunchInfo{grid, kRowThreads, 0};
+    for (; a.chunk <= sh.chunks; ++a.chunk) {
+        const cudaError_t err =
+            inclusive ? launch_dependent(rts_kernel<T, true, ALIGNED>, grid, kRowThreads, 0, stream, a)
+                      : launch_dependent(rts_kernel<T, false, ALIGNED>, grid, kRowThreads, 0, stream, a);
+        if (err != cudaSuccess) return err;
+    }
+    return cudaSuccess;
+}
+
+template <typename T>
+cudaError_t dispatch_rts(bool inclusive, const ScanArgs& a, void* scratch, int num_sms, cudaStream_t stream,
+                         LaunchInfo* info) {
+    const bool aligned = ((reinterpret_cast<uintptr_t>(a.in) | reinterpret_cast<uintptr_t>(a.out)) & 15u) == 0;
+    return aligned ? dispatch_rts<T, true>(inclusive, a, scratch, num_sms, stream, info)
+                   : dispatch_rts<T, false>(inclusive, a, scratch, num_sms, stream, info);
 }
 
 }  // namespace
 
-uint32_t rts_tile_elems(gps_dtype dtype) {
-    return dtype == GPS_DTYPE_U64 ? TileShape<uint64_t, kRtsWarps>::kTile : TileShape<uint32_t, kRtsWarps>::kTile;
+uint32_t rts_tile_elems(gps_dtype dtype) { return 16384u / static_cast<uint32_t>(dtype_size(dtype)); }
+
+uint64_t rts_scratch_elems(int num_sms) { return 3ull * static_cast<uint64_t>(kRtsCtasPerSm * num_sms) + 3; }
+
+uint32_t rts_launches(uint64_t n, uint32_t tile_elems, int num_sms) {
+    return rts_shape(static_cast<uint32_t>((n + tile_elems - 1) / tile_elems), num_sms).chunks + 1;
 }
 
-cudaError_t launch_rts(gps_dtype dtype, bool inclusive, const ScanArgs& a, void* tile_sums, int num_sms,
+cudaError_t launch_rts(gps_dtype dtype, bool inclusive, const ScanArgs& a, void* scratch, int num_sms,
                        cudaStream_t stream, LaunchInfo* info) {
-    if (dtype == GPS_DTYPE_U64) return dispatch_rts<uint64_t>(inclusive, a, tile_sums, num_sms, stream, info);
-    return dispatch_rts<uint32_t>(inclusive, a, tile_sums, num_sms, stream, info);
+    if (dtype == GPS_DTYPE_U64) return dispatch_rts<uint64_t>(inclusive, a, scratch, num_sms, stream, info);
+    return dispatch_rts<uint32_t>(inclusive, a, scratch, num_sms, stream, info);
 }
 
 }  // namespace gps

@@ -1,22 +1,19 @@
-// Persistent, warp-specialised tile-scan kernel for sm_103a.
+// Persistent, warp-specialised ring kernel for buffers off a 16-byte boundary,
+// and the descriptor, warp-scan and lookback code the other kernels share.
 //
 // Each CTA runs a ring of S shared-memory stages, one 16 KB tile each, and
 // four roles:
-//   producer  (1 thread)  takes tile ids (an atomic counter for the chained
-//             scan, a static stride for reduce-then-scan), moves each tile
-//             global -> shared with one bulk copy (cp.async.bulk, completion
-//             on an mbarrier) and, once it is scanned, shared -> global with
-//             one bulk store;
-//   reduce    (RW warps)  sums the landed tile, publishes its aggregate in the
-//             tile descriptor and leaves each thread's offset in shared
+//   producer  (1 thread)  takes unit ids from an atomic counter and recycles
+//             the stages;
+//   reduce    (RW warps)  loads the tile into the stage, sums it, publishes
+//             its unit's aggregate and leaves each thread's offset in shared
 //             memory;
-//   lookback  (1 warp)    resolves the tile's exclusive prefix, in tile order:
+//   lookback  (LW warps)  resolves the unit's exclusive prefix, in order:
 //             decoupled lookback over the descriptors (the reference's
 //             ChainedScanDecoupledLookback.cuh:50-77 does this with a 30-bit
 //             payload; here the payload is the full 32/64-bit value, tagged
-//             with a launch epoch) or the spine of a reduce-then-scan
-//             (ReduceThenScan.cuh:134-136);
-//   finalize  (RW warps)  adds prefix and offsets, writes the tile back.
+//             with a launch epoch);
+//   finalize  (RW warps)  adds prefix and offsets, writes the tile out.
 //
 // Every wait is bounded by the plan's budget (global timer); on expiry the
 // kernel records a flag in the workspace header and winds down without
@@ -395,9 +392,7 @@ __device__ __forceinline__ void rotated_chunk_prefix(const T (&cs)[CHUNKS], uint
 // ------------------------------------------------------------------ kernel
 // CTA layout: warp 0 producer, warps 1..LW lookback (taking alternate units),
 // then RW reduce warps, then RW finalize warps. Reduce and finalize thread i
-// own the same 128 contiguous bytes of a tile, read as eight 16-byte chunks
-// in an order rotated by (i & 7) so that each quarter-warp touches all 32
-// banks once.
+// own the same 128 contiguous bytes of a tile.
 //
 // The lookback unit is G consecutive tiles that one CTA loads into G
 // consecutive stages: one descriptor and one lookback per unit, so the
@@ -410,20 +405,16 @@ __device__ __forceinline__ void rotated_chunk_prefix(const T (&cs)[CHUNKS], uint
 // of their ids having been taken. Lookback warps resolve their CTA's units in
 // order, so every walk ends at the latest at the unit the same warp (or the
 // other lookback warp) resolved before.
-template <typename T, int RW, int S, int G, bool INCL, bool BULK, PrefixMode PM, bool STALL>
+template <typename T, int RW, int S, int G, bool INCL>
 __global__ void __launch_bounds__(TileShape<T, RW>::kThreads, 2) scan_pipeline_kernel(const ScanArgs a) {
     using Shape = TileShape<T, RW>;
     constexpr int TILE = Shape::kTile;
     constexpr int ITEMS = Shape::kItems;
-    constexpr int EPC = 16 / static_cast<int>(sizeof(T));
-    constexpr int CHUNKS = ITEMS / EPC;
     constexpr uint32_t NROLE = Shape::kRoleThreads;
     constexpr uint32_t LW = Shape::kLookbackWarps;
     constexpr uint32_t kWarpReduce = 1 + LW, kWarpFinal = 1 + LW + RW;
     constexpr int SLOTS = S / G;
-    static_assert(CHUNKS == 8, "128 bytes per thread");
     static_assert(S % G == 0 && SLOTS >= 2, "the ring holds at least two units");
-    static_assert(PM == PrefixMode::Lookback || G == 1, "reduce-then-scan works tile by tile");
     using D = DescTraits<T>;
     using word = typename D::word;
 
@@ -449,7 +440,7 @@ __global__ void __launch_bounds__(TileShape<T, RW>::kThreads, 2) scan_pipeline_k
     }
     __syncthreads();
 
-    const uint32_t epoch = (PM == PrefixMode::Lookback) ? ld_volatile_u32(&a.hdr->epoch) : 0u;
+    const uint32_t epoch = ld_volatile_u32(&a.hdr->epoch);
     // Added to every output: the running total of earlier pieces when a long
     // host array is scanned chunk by chunk.
     const T carry = a.carry_in != nullptr ? *static_cast<const T*>(a.carry_in) : T(0);
@@ -457,27 +448,21 @@ __global__ void __launch_bounds__(TileShape<T, RW>::kThreads, 2) scan_pipeline_k
     auto count_of = [&](uint32_t t) -> uint32_t {
         return t < a.num_tiles ? tile_count<TILE>(a.n, t) : 0u;
     };
-    auto bulk_bytes_of = [&](uint32_t t) -> uint32_t {
-        return (count_of(t) * static_cast<uint32_t>(sizeof(T))) & ~15u;
-    };
 
     // ======================================================== producer
     if (warp == 0) {
         if (lane != 0) return;
         bool stop = false;
-        uint64_t k_static = 0;
         // Unit ids are taken one refill ahead (acquire) and checked when the
         // refill is issued (resolve), so the counter's round trip overlaps
         // the wait for the finalize warps. Ids only grow, so once one is past
         // the end every later one is too.
         auto acquire = [&]() -> uint64_t {
             if (stop) return ~0ull;
-            if (PM == PrefixMode::Spine) return blockIdx.x + (k_static++) * gridDim.x;
             return atomicAdd(&a.hdr->tile_counter, 1u);
         };
         auto resolve = [&](uint64_t raw) -> uint32_t {
-            if (stop || raw >= num_units ||
-                (PM == PrefixMode::Lookback && ld_volatile_u32(&a.hdr->error_flags) != 0)) {
+            if (stop || raw >= num_units || ld_volatile_u32(&a.hdr->error_flags) != 0) {
                 stop = true;
                 return kTileEnd;
             }
@@ -489,16 +474,7 @@ __global__ void __launch_bounds__(TileShape<T, RW>::kThreads, 2) scan_pipeline_k
                 const int s = j * G + k;
                 const uint32_t t = u == kTileEnd ? kTileEnd : u * G + k;
                 ctrl->tile_of[s] = t;
-                if (BULK && t != kTileEnd) {
-                    const uint32_t bytes = bulk_bytes_of(t);
-                    ptx::mbar_arrive_expect_tx(&ctrl->full[s], bytes);
-                    if (bytes)
-                        ptx::bulk_load(bufs + static_cast<size_t>(s) * TILE,
-                                       static_cast<const T*>(a.in) + static_cast<uint64_t>(t) * TILE, bytes,
-                                       &ctrl->full[s]);
-                } else {
-                    ptx::mbar_arrive(&ctrl->full[s]);
-                }
+                ptx::mbar_arrive(&ctrl->full[s]);
             }
         };
 #pragma unroll 1
@@ -520,43 +496,27 @@ __global__ void __launch_bounds__(TileShape<T, RW>::kThreads, 2) scan_pipeline_k
                     failed = true;
                     break;
                 }
-                if (BULK) {
-                    const uint32_t t = ctrl->tile_of[s];
-                    const uint32_t bytes = t == kTileEnd ? 0u : bulk_bytes_of(t);
-                    if (bytes)
-                        ptx::bulk_store(static_cast<T*>(a.out) + static_cast<uint64_t>(t) * TILE,
-                                        bufs + static_cast<size_t>(s) * TILE, bytes);
-                }
             }
             if (failed) break;
-            // Refill the slot as soon as its stores have read it out.
-            if (BULK) {
-                ptx::bulk_commit();
-                ptx::bulk_wait_read<0>();
-            }
             issue(j, resolve(upcoming));
             upcoming = acquire();
         }
-        if (BULK) ptx::bulk_wait_all<0>();
-
-        if (PM == PrefixMode::Lookback) {
-            // The last CTA out returns the counters to zero and advances the
-            // epoch, which retires every descriptor of this launch.
+        // The last CTA out returns the counters to zero and advances the
+        // epoch, which retires every descriptor of this launch.
+        __threadfence();
+        const uint32_t prev = atomicAdd(&a.hdr->exit_counter, 1u);
+        if (prev == gridDim.x - 1) {
             __threadfence();
-            const uint32_t prev = atomicAdd(&a.hdr->exit_counter, 1u);
-            if (prev == gridDim.x - 1) {
-                __threadfence();
-                a.hdr->tile_counter = 0;
-                a.hdr->exit_counter = 0;
-                uint32_t e = epoch + 1;
-                if ((e & kEpochMask) == 0) {
-                    word* desc = static_cast<word*>(a.desc);
-                    for (unsigned long long q = 0; q < a.hdr->capacity_tiles; ++q) D::store(desc + q, D::zero());
-                    e += 1;
-                }
-                __threadfence();
-                a.hdr->epoch = e;
+            a.hdr->tile_counter = 0;
+            a.hdr->exit_counter = 0;
+            uint32_t e = epoch + 1;
+            if ((e & kEpochMask) == 0) {
+                word* desc = static_cast<word*>(a.desc);
+                for (unsigned long long q = 0; q < a.hdr->capacity_tiles; ++q) D::store(desc + q, D::zero());
+                e += 1;
             }
+            __threadfence();
+            a.hdr->epoch = e;
         }
         return;
     }
@@ -613,9 +573,7 @@ __global__ void __launch_bounds__(TileShape<T, RW>::kThreads, 2) scan_pipeline_k
             }
             const uint32_t u = t0 / G;
             T pre;
-            if (PM == PrefixMode::Spine) {
-                pre = carry + (t0 == 0 ? T(0) : static_cast<const T*>(a.spine)[t0 - 1]);
-            } else if (u == 0) {
+            if (u == 0) {
                 pre = carry;
             } else {
                 int64_t bound = own_prev;
@@ -635,7 +593,7 @@ __global__ void __launch_bounds__(TileShape<T, RW>::kThreads, 2) scan_pipeline_k
                         }
                     }
                 }
-                pre = lookback<T, TILE * G, STALL>(a, u, epoch, lane, carry, bound, bound_val);
+                pre = lookback<T, TILE * G, false>(a, u, epoch, lane, carry, bound, bound_val);
             }
             // Hand each tile its prefix as soon as its own aggregate is in.
             T run = pre;
@@ -651,13 +609,12 @@ __global__ void __launch_bounds__(TileShape<T, RW>::kThreads, 2) scan_pipeline_k
                 }
                 if (lane == 0) {
                     ctrl->prefix[s] = run;
-                    if (STALL && k == G - 1) __threadfence();
                     ptx::mbar_arrive(&ctrl->prefixed[s]);
                 }
                 run += ctrl->agg[s];
             }
             if (stopped) break;
-            if (PM == PrefixMode::Lookback && u != 0 && lane == 0) D::store(desc + u, D::pack(kInclusive, epoch, run));
+            if (u != 0 && lane == 0) D::store(desc + u, D::pack(kInclusive, epoch, run));
             if (lane == 0 && a.carry_out != nullptr && u == num_units - 1) *static_cast<T*>(a.carry_out) = run;
             own_prev = u;
             own_incl = run;
@@ -670,7 +627,6 @@ __global__ void __launch_bounds__(TileShape<T, RW>::kThreads, 2) scan_pipeline_k
     if (warp < kWarpFinal) {
         const uint32_t r = tid - kWarpReduce * 32;
         const uint32_t rw = warp - kWarpReduce;
-        const uint32_t rot = r & 7u;
         bool running = true;
         for (uint32_t i = 0; running; ++i) {
             const int j = static_cast<int>(i % SLOTS);
@@ -686,31 +642,16 @@ __global__ void __launch_bounds__(TileShape<T, RW>::kThreads, 2) scan_pipeline_k
                 T* sb = bufs + static_cast<size_t>(s) * TILE;
                 const uint32_t cnt = live ? count_of(t) : 0u;
                 T total = 0;
-                if (BULK && cnt == static_cast<uint32_t>(TILE)) {
-#pragma unroll
-                    for (int c8 = 0; c8 < CHUNKS; ++c8) {
-                        const uint32_t c = (c8 + rot) & (CHUNKS - 1);
-                        const Chunk<T> q = *reinterpret_cast<const Chunk<T>*>(sb + r * ITEMS + c * EPC);
-#pragma unroll
-                        for (int e = 0; e < EPC; ++e) total += q.v[e];
-                    }
-                } else if (cnt != 0) {
-                    // Partial tile or unaligned buffers: elements the bulk copy
-                    // did not bring in are read from global memory and parked
-                    // in the stage, so that finalize always reads the stage.
-                    const uint32_t bulk_elems = BULK ? bulk_bytes_of(t) / static_cast<uint32_t>(sizeof(T)) : 0u;
+                if (cnt != 0) {
+                    // Elements are parked in the stage, for finalize.
                     const uint64_t gbase = static_cast<uint64_t>(t) * TILE;
 #pragma unroll 4
                     for (int e = 0; e < ITEMS; ++e) {
                         const uint32_t li = r * ITEMS + e;
                         T x = 0;
                         if (li < cnt) {
-                            if (BULK && li < bulk_elems) {
-                                x = sb[li];
-                            } else {
-                                x = static_cast<const T*>(a.in)[gbase + li];
-                                sb[li] = x;
-                            }
+                            x = static_cast<const T*>(a.in)[gbase + li];
+                            sb[li] = x;
                         }
                         total += x;
                     }
@@ -742,32 +683,12 @@ __global__ void __launch_bounds__(TileShape<T, RW>::kThreads, 2) scan_pipeline_k
                 if (r == 0) {
                     ctrl->agg[s] = agg;
                     unit_agg += agg;
-                    if (PM == PrefixMode::Lookback && k == G - 1) {
+                    if (k == G - 1) {
                         const uint32_t u = t / G;
-                        word* desc = static_cast<word*>(a.desc);
-                        bool publish = true;
-                        if (STALL && unit_stalls(a.stall, u, (a.num_tiles + G - 1) / G)) {
-                            // Withhold the aggregate until the delay ends or a
-                            // successor inserts it (EmulatedDeadlocking.cuh:64-70).
-                            atomicAdd(&a.hdr->stat_stalls, 1ull);
-                            const uint64_t until = ptx::global_timer_ns() + a.stall.delay_ns;
-                            while (true) {
-                                if (D::status(D::load(desc + u), epoch) != kNotReady) {
-                                    publish = false;
-                                    break;
-                                }
-                                if (ptx::global_timer_ns() > until) break;
-                                __nanosleep(200);
-                            }
-                        }
                         // Only unit 0's value is an inclusive prefix, so only
-                        // it holds the carry. A rescuer computes the same
-                        // integer aggregate, so a plain store over an inserted
-                        // one is harmless; rescuers use a CAS so that they
-                        // never overwrite an inclusive prefix.
-                        if (publish)
-                            D::store(desc + u, u == 0 ? D::pack(kInclusive, epoch, carry + unit_agg)
-                                                      : D::pack(kAggregate, epoch, unit_agg));
+                        // it holds the carry.
+                        D::store(static_cast<word*>(a.desc) + u, u == 0 ? D::pack(kInclusive, epoch, carry + unit_agg)
+                                                                        : D::pack(kAggregate, epoch, unit_agg));
                     }
                 }
                 __syncwarp();
@@ -780,7 +701,6 @@ __global__ void __launch_bounds__(TileShape<T, RW>::kThreads, 2) scan_pipeline_k
     // ======================================================== finalize
     {
         const uint32_t f = tid - kWarpFinal * 32;
-        const uint32_t rot = f & 7u;
         bool running = true;
         for (uint32_t i = 0; running; ++i) {
             const int j = static_cast<int>(i % SLOTS);
@@ -800,61 +720,17 @@ __global__ void __launch_bounds__(TileShape<T, RW>::kThreads, 2) scan_pipeline_k
                 T* sb = bufs + static_cast<size_t>(s) * TILE;
                 const uint32_t cnt = count_of(t);
                 const T base = ctrl->prefix[s] + ctrl->offset[s][f];
-                if (BULK && cnt == static_cast<uint32_t>(TILE)) {
-                    T v[ITEMS];
-                    T cs[CHUNKS];
-#pragma unroll
-                    for (int c8 = 0; c8 < CHUNKS; ++c8) {
-                        const uint32_t c = (c8 + rot) & (CHUNKS - 1);
-                        const Chunk<T> q = *reinterpret_cast<const Chunk<T>*>(sb + f * ITEMS + c * EPC);
-                        T x = 0;
-#pragma unroll
-                        for (int e = 0; e < EPC; ++e) {
-                            v[c8 * EPC + e] = q.v[e];
-                            x += q.v[e];
-                        }
-                        cs[c8] = x;
-                    }
-                    T cpre[CHUNKS];
-                    T total;
-                    rotated_chunk_prefix<T, CHUNKS>(cs, rot, cpre, total);
-#pragma unroll
-                    for (int c8 = 0; c8 < CHUNKS; ++c8) {
-                        T run = base + cpre[c8];
-                        Chunk<T> q;
-#pragma unroll
-                        for (int e = 0; e < EPC; ++e) {
-                            const T x = v[c8 * EPC + e];
-                            if (INCL) {
-                                run += x;
-                                q.v[e] = run;
-                            } else {
-                                q.v[e] = run;
-                                run += x;
-                            }
-                        }
-                        const uint32_t c = (c8 + rot) & (CHUNKS - 1);
-                        *reinterpret_cast<Chunk<T>*>(sb + f * ITEMS + c * EPC) = q;
-                    }
-                } else if (cnt != 0) {
-                    const uint32_t bulk_elems = BULK ? bulk_bytes_of(t) / static_cast<uint32_t>(sizeof(T)) : 0u;
-                    const uint64_t gbase = static_cast<uint64_t>(t) * TILE;
-                    T run = base;
+                const uint64_t gbase = static_cast<uint64_t>(t) * TILE;
+                T run = base;
 #pragma unroll 4
-                    for (int e = 0; e < ITEMS; ++e) {
-                        const uint32_t li = f * ITEMS + e;
-                        if (li < cnt) {
-                            const T x = sb[li];
-                            const T y = INCL ? run + x : run;
-                            run += x;
-                            if (BULK && li < bulk_elems)
-                                sb[li] = y;
-                            else
-                                static_cast<T*>(a.out)[gbase + li] = y;
-                        }
+                for (int e = 0; e < ITEMS; ++e) {
+                    const uint32_t li = f * ITEMS + e;
+                    if (li < cnt) {
+                        const T x = sb[li];
+                        static_cast<T*>(a.out)[gbase + li] = INCL ? run + x : run;
+                        run += x;
                     }
                 }
-                if (BULK) ptx::fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) ptx::mbar_arrive(&ctrl->done[s]);
             }

@@ -77,7 +77,9 @@ typedef enum gps_algo {
     /* Single-pass chained scan with decoupled lookback
      * (ChainedScanDecoupledLookback.cuh:79-153). */
     GPS_ALGO_CSDL = 0,
-    /* Reduce -> spine scan -> propagate, three launches
+    /* Reduce, scan of the range sums, propagate, with no waits between CTAs:
+     * one launch more than the input has chunks of 25 MB (gps_plan_geometry),
+     * each after the first propagating one chunk while it reduces the next
      * (ReduceThenScan.cuh:15-161, ReduceThenScanDispatcher.cuh:165-187). */
     GPS_ALGO_RTS = 1
 } gps_algo;
