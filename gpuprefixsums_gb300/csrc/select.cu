@@ -18,22 +18,30 @@
 // written: (sizeof(V) + 1) bytes read and p * sizeof(V) written per element
 // for a selected fraction p.
 //
-// Warps: 0 R-loader (flags), 1 S-loader (values + flags), 2..4 lookback,
-// then 4 reduce and 4 finalize warps. Every wait is bounded by the plan's
-// budget.
+// Warps: 0 R-loader (flags), 1 S-loader (values), 2..4 lookback, then 4
+// reduce warps and two groups of 4 finalize warps, which take alternate tiles.
+// Every wait is bounded by the plan's budget.
+//
+// HBM bounds it now; one finalize group could not compact the tiles as fast
+// as they arrive (one warp per scheduler, each waiting on its own shared-memory
+// stores). Measured on GB300, 2^28 u32, 30% selected: one group 302 us, two
+// groups with 6 units in flight 274, with 8 units and 6 instead of 8 flag
+// stages 264 (6.3 TB/s, 0.95 of the copy rate), 9 or 12 units 265 and 271
+// (fewer flag stages fit); 80% selected 335 / 343 / 334 us.
 #include "launch_util.h"
 #include "scan_pipeline.cuh"
 
 namespace gps {
 namespace {
 
-constexpr int kSelWarps = 4;                 // reduce warps = finalize warps
+constexpr int kSelWarps = 4;                 // reduce warps = finalize warps of a group
+constexpr int kSelGroups = 2;                // finalize groups, taking alternate tiles
 constexpr int kSelRole = kSelWarps * 32;     // threads per role
 constexpr int kSelLookback = 3;
-constexpr int kSelThreads = 32 * (2 + kSelLookback + 2 * kSelWarps);
-constexpr int kSelRS = 8;   // flag stages of the reduce pass
+constexpr int kSelThreads = 32 * (2 + kSelLookback + (1 + kSelGroups) * kSelWarps);
+constexpr int kSelRS = 6;   // flag stages of the reduce pass
 constexpr int kSelSS = 8;   // value stages of the scan pass
-constexpr int kSelQ = 6;    // units in flight
+constexpr int kSelQ = 8;    // units in flight
 constexpr int kSelG = 4;    // tiles per unit
 
 // 16 KB of values per tile: 4096 four-byte or 2048 eight-byte elements.
@@ -67,7 +75,7 @@ struct SelCtrl {
 template <typename V>
 constexpr size_t sel_smem_bytes() {
     constexpr size_t TILE = SelShape<V>::kTile;
-    return kSelRS * TILE + kSelSS * TILE * sizeof(V) + kSelWarps * SelShape<V>::kSlice * sizeof(V) +
+    return kSelRS * TILE + kSelSS * TILE * sizeof(V) + kSelGroups * kSelWarps * SelShape<V>::kSlice * sizeof(V) +
            sizeof(SelCtrl<V>);
 }
 
@@ -101,6 +109,11 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
     constexpr uint32_t kWarpLookback = 2, kWarpReduce = 2 + kSelLookback, kWarpFinal = kWarpReduce + kSelWarps;
     constexpr int RS = kSelRS, SS = kSelSS, Q = kSelQ, G = kSelG;
     static_assert(CHUNKS == 8, "128 bytes of values per thread");
+    static_assert(G % kSelGroups == 0, "a group takes the same tiles of every unit");
+    // With a stage count the groups do not divide, a stage would pass from group
+    // to group and a group would see every other phase of its barrier only,
+    // always with the same parity: it would take a stage before it is loaded.
+    static_assert(SS % kSelGroups == 0, "a stage belongs to one group");
     static_assert(ITEMS <= 32, "one 32-bit mask of flags per thread");
     using Ctrl = SelCtrl<V>;
 
@@ -108,7 +121,7 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
     uint8_t* rflags = smem_raw;
     V* svals = reinterpret_cast<V*>(rflags + static_cast<size_t>(RS) * TILE);
     V* ostage = svals + static_cast<size_t>(SS) * TILE;
-    Ctrl* ctrl = reinterpret_cast<Ctrl*>(ostage + kSelWarps * Sh::kSlice);
+    Ctrl* ctrl = reinterpret_cast<Ctrl*>(ostage + kSelGroups * kSelWarps * Sh::kSlice);
 
     const uint32_t tid = threadIdx.x;
     const uint32_t warp = tid >> 5;
@@ -128,7 +141,7 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
             ptx::mbar_init(&ctrl->uknown[q], 1);
             ptx::mbar_init(&ctrl->ureduced[q], kSelWarps);
             ptx::mbar_init(&ctrl->uprefix[q], 1);
-            ptx::mbar_init(&ctrl->ufree[q], kSelWarps);
+            ptx::mbar_init(&ctrl->ufree[q], kSelGroups * kSelWarps);
         }
         ctrl->end_seq = 0xFFFFFFFFu;
         ptx::fence_mbar_init();
@@ -255,7 +268,8 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
                         break;
                     }
                 }
-                for (int k = 0; k < (end ? 1 : G); ++k, ++sn) {
+                // Every finalize group stops at a stage of its own.
+                for (int k = 0; k < (end ? kSelGroups : G); ++k, ++sn) {
                     const int s = static_cast<int>(sn % SS);
                     if (sn >= SS && !wait1(&ctrl->sfree[s], ((sn - SS) / SS) & 1u, long_budget)) {
                         ok = false;
@@ -264,7 +278,7 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
                     if (end) {
                         ctrl->s_tile[s] = kTileEnd;
                         ptx::mbar_arrive(&ctrl->sfull[s]);
-                        break;
+                        continue;
                     }
                     const uint32_t t = u * G + k;
                     ctrl->s_tile[s] = t;
@@ -398,12 +412,13 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
     // first position comes from one population count: no dependent chain
     // longer than a chunk.
     else {
-        const uint32_t f = tid - kWarpFinal * 32;
-        const uint32_t fw = warp - kWarpFinal;
+        const uint32_t group = (warp - kWarpFinal) / kSelWarps;
+        const uint32_t fw = (warp - kWarpFinal) % kSelWarps;
+        const uint32_t f = fw * 32 + lane;
         const uint32_t rot = f & 7u;
-        V* wst = ostage + fw * Sh::kSlice;  // this warp's staging slice
+        V* wst = ostage + (group * kSelWarps + fw) * Sh::kSlice;  // this warp's staging slice
         uint64_t run = 0;  // the unit's output position
-        for (uint32_t sn = 0;; ++sn) {
+        for (uint32_t sn = group;; sn += kSelGroups) {
             const int s = static_cast<int>(sn % SS);
             const uint32_t i = sn / G;
             const int k = static_cast<int>(sn % G);
@@ -437,7 +452,7 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
             }
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&ctrl->sfree[s]);  // this warp is done with the stage
-            if (k == 0) {
+            if (k == static_cast<int>(group)) {
                 bool pok = wait1(&ctrl->uprefix[q], (i / Q) & 1u, long_budget);
                 pok = __all_sync(kFullMask, pok);
                 if (!pok && lane == 0) raise_error(a.hdr, kErrPipelineTimeout);
@@ -477,7 +492,7 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
             Chunk<V>* dst = reinterpret_cast<Chunk<V>*>(out + head);
             for (uint32_t x = lane; x < body; x += 32u) dst[x] = src[x];
             if (tail + lane < warp_cnt) out[tail + lane] = wst[o + tail + lane];
-            if (k == G - 1 && lane == 0) ptx::mbar_arrive(&ctrl->ufree[q]);
+            if (k + kSelGroups >= G && lane == 0) ptx::mbar_arrive(&ctrl->ufree[q]);
         }
     }
 
