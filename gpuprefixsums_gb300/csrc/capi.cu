@@ -630,7 +630,10 @@ gps_status gps_select_flagged(gps_plan p, const void* d_in, const uint8_t* d_fla
     a.n = n;
     a.num_tiles = static_cast<uint32_t>((n + gps::select_tile_elems(es) - 1) / gps::select_tile_elems(es));
     a.hdr = p->hdr16;
-    a.desc = p->desc16;
+    const bool mid = a.num_tiles <= gps::kMidSelectMaxTiles;
+    a.desc = mid ? p->desc_mid : p->desc16;
+    a.group_desc = p->group_desc_mid;
+    a.mid_launch = &p->hdr->mid_launch;
     a.carry_out = d_num_selected;
     a.wait_budget_ns = p->wait_budget_ns;
     const cudaError_t err = gps::launch_select(es, a, d_flags, p->num_sms, s, &p->last_launch);

@@ -216,6 +216,9 @@ bool seg_u32x4_x2_fits(uint32_t unit);
 // Stream compaction by flag bytes (select.cu): elements per tile for an
 // element size, and the launch. a.carry_out receives the count (uint64).
 uint32_t select_tile_elems(size_t elem_size);
+// Selects of up to this many tiles run one tile per CTA, on the plan's
+// mid-size descriptors.
+constexpr uint32_t kMidSelectMaxTiles = 2048;
 cudaError_t launch_select(size_t elem_size, const ScanArgs& a, const uint8_t* flags, int num_sms, cudaStream_t stream,
                           LaunchInfo* info);
 

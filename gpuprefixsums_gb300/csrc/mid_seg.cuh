@@ -146,6 +146,43 @@ __device__ __forceinline__ bool mid_seg_fold(const ScanArgs& a, const ptx::u64x2
     return true;
 }
 
+// Run by warp 0 of tile t: publishes the tile's aggregate (and its group's, by
+// the group's last tile) and folds the aggregates before it into `pre`. The
+// last tile waits for all groups and advances the launch number. False once
+// the wait budget has run out.
+template <class Op>
+__device__ __forceinline__ bool mid_seg_prefix(const ScanArgs& a, uint32_t t, uint64_t tag, typename Op::C agg,
+                                               bool flag, uint32_t lane, typename Op::C& pre) {
+    using C = typename Op::C;
+    constexpr int KT = static_cast<int>(kMidSegGroup / 32);
+    constexpr int KG = static_cast<int>((kMidSegMaxTiles / kMidSegGroup + 31) / 32);
+    const uint32_t ws = a.desc_stride;
+    ptx::u64x2* d1 = static_cast<ptx::u64x2*>(a.desc);
+    ptx::u64x2* d2 = static_cast<ptx::u64x2*>(a.group_desc);
+    if (lane == 0) mid_seg_store<Op>(d1 + static_cast<uint64_t>(t) * ws, tag, flag, agg);
+    const uint32_t g = t / kMidSegGroup;
+    const uint32_t i0 = g * kMidSegGroup;
+    C in = Op::chain_zero(), gp = Op::chain_zero();
+    bool inf = false, gpf = false, ok = true;
+    // A launch of up to 32 tiles reads one descriptor a lane.
+    if (t != i0) {
+        const ptx::u64x2* dg = d1 + static_cast<uint64_t>(i0) * ws;
+        ok = a.num_tiles <= 32 ? mid_seg_fold<Op, 1>(a, dg, ws, t - i0, tag, lane, in, inf)
+                               : mid_seg_fold<Op, KT>(a, dg, ws, t - i0, tag, lane, in, inf);
+    }
+    if (ok && lane == 0 && t - i0 == kMidSegGroup - 1)
+        mid_seg_store<Op>(d2 + static_cast<uint64_t>(g) * kMidDescStride, tag, inf || flag,
+                          flag ? agg : Op::chain_add(in, agg));
+    const bool last = t == a.num_tiles - 1;
+    if (ok && g != 0 && (!inf || last)) {
+        ok = mid_seg_fold<Op, KG>(a, d2, kMidDescStride, g, tag, lane, gp, gpf);
+        if (!inf) in = t == i0 ? gp : Op::chain_add(gp, in);
+    }
+    if (ok && last && lane == 0) ptx::st_relaxed_u64(a.mid_launch, tag + 1);
+    pre = in;
+    return ok;
+}
+
 template <class Op, bool INCL, bool SEG>
 __global__ void __launch_bounds__(kMidSegThreads, sizeof(typename Op::S) > 8 ? 4 : 6)
     mid_seg_kernel(const ScanArgs a, const SegArgs sg) {
@@ -158,8 +195,6 @@ __global__ void __launch_bounds__(kMidSegThreads, sizeof(typename Op::S) > 8 ? 4
     constexpr int CHUNKS = 4;
     constexpr int WARPS = kMidSegThreads / 32;
     constexpr int kHeadWords = TILE / 32;
-    constexpr int KT = static_cast<int>(kMidSegGroup / 32);
-    constexpr int KG = static_cast<int>((kMidSegMaxTiles / kMidSegGroup + 31) / 32);
     static_assert(ITEMS == CHUNKS * EPC, "four chunks a thread");
 
     __shared__ __align__(16) Chunk<T> s_tile[CHUNKS * kMidSegThreads];
@@ -285,36 +320,11 @@ __global__ void __launch_bounds__(kMidSegThreads, sizeof(typename Op::S) > 8 ? 4
     // 4. Publish and look back.
     if (a.num_tiles > 1) {
         if (warp == 0) {
-            const uint32_t ws = a.desc_stride;
-            ptx::u64x2* d1 = static_cast<ptx::u64x2*>(a.desc);
-            ptx::u64x2* d2 = static_cast<ptx::u64x2*>(a.group_desc);
-            const C agg = Op::to_chain(Op::norm(tot));
-            if (lane == 0) mid_seg_store<Op>(d1 + static_cast<uint64_t>(t) * ws, tag, totf, agg);
-            const uint32_t g = t / kMidSegGroup;
-            const uint32_t i0 = g * kMidSegGroup;
-            C in = Op::chain_zero(), gp = Op::chain_zero();
-            bool inf = false, gpf = false;
-            // A launch of up to 32 tiles reads one descriptor a lane.
-            bool ok = true;
-            if (t != i0) {
-                const ptx::u64x2* dg = d1 + static_cast<uint64_t>(i0) * ws;
-                ok = a.num_tiles <= 32 ? mid_seg_fold<Op, 1>(a, dg, ws, t - i0, tag, lane, in, inf)
-                                       : mid_seg_fold<Op, KT>(a, dg, ws, t - i0, tag, lane, in, inf);
-            }
-            if (ok && lane == 0 && t - i0 == kMidSegGroup - 1)
-                mid_seg_store<Op>(d2 + static_cast<uint64_t>(g) * kMidDescStride, tag, inf || totf,
-                                  totf ? agg : Op::chain_add(in, agg));
-            // The last tile waits for all groups, so that it may advance the
-            // launch number.
-            const bool last = t == a.num_tiles - 1;
-            if (ok && g != 0 && (!inf || last)) {
-                ok = mid_seg_fold<Op, KG>(a, d2, kMidDescStride, g, tag, lane, gp, gpf);
-                if (!inf) in = t == i0 ? gp : Op::chain_add(gp, in);
-            }
+            C before;
+            const bool ok = mid_seg_prefix<Op>(a, t, tag, Op::to_chain(Op::norm(tot)), totf, lane, before);
             if (lane == 0) {
-                if (ok && last) ptx::st_relaxed_u64(a.mid_launch, tag + 1);
                 if (!ok) raise_error(a.hdr, kErrLookbackTimeout);
-                s_pre = in;
+                s_pre = before;
             }
         }
         __syncthreads();

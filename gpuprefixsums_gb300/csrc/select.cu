@@ -29,7 +29,7 @@
 // stages 264 (6.3 TB/s, 0.95 of the copy rate), 9 or 12 units 265 and 271
 // (fewer flag stages fit); 80% selected 335 / 343 / 334 us.
 #include "launch_util.h"
-#include "scan_pipeline.cuh"
+#include "mid_seg.cuh"
 
 namespace gps {
 namespace {
@@ -519,6 +519,128 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
     }
 }
 
+// ------------------------------------------------------ small and mid sizes
+// One tile of 16 KB of values per CTA of 256 threads, as in mid_seg.cuh: the
+// persistent kernel's pipeline takes 9 us whatever the size, and its units of
+// 4 tiles leave most SMs idle below 600 tiles. Flags and values are loaded
+// together; each thread turns the flags of its 64 bytes of values into a mask,
+// the block scans the counts, and while warp 0 publishes the tile's count and
+// folds the counts before it (mid_seg.cuh's fixed-order lookback), the values
+// are compacted in shared memory. Then the run goes out, coalesced.
+// Latency bounds it: one HBM read, two L2 round trips, a store. Measured on
+// GB300, graph replay, u32, 30% selected, against the persistent kernel:
+// 2^16 elements 2.7 against 7.1 us, 2^20 5.6 / 8.8, 2^22 11.4 / 14.2, 2^23 17.9 /
+// 19.0 (90% selected: 21.0 / 24.0), 2^24 32.3 / 28.4.
+constexpr int kMidSelThreads = kMidSegThreads;
+
+template <typename V>
+__global__ void __launch_bounds__(kMidSelThreads, 6) mid_select_kernel(const ScanArgs a, const SelArgs sa) {
+    constexpr int TILE = 16384 / static_cast<int>(sizeof(V));
+    constexpr int EPC = 16 / static_cast<int>(sizeof(V));
+    constexpr int ITEMS = TILE / kMidSelThreads;
+    constexpr int CHUNKS = 4;
+    constexpr int WARPS = kMidSelThreads / 32;
+    constexpr int FW = ITEMS / 4;  // flag words per thread
+    static_assert(ITEMS == CHUNKS * EPC, "four chunks a thread");
+    __shared__ __align__(16) Chunk<V> s_tile[CHUNKS * kMidSelThreads];
+    __shared__ uint32_t s_wtot[WARPS];
+    __shared__ uint64_t s_pre;
+
+    const uint32_t tid = threadIdx.x;
+    const uint32_t lane = tid & 31u;
+    const uint32_t warp = tid >> 5;
+    const uint32_t t = blockIdx.x;
+    ptx::grid_dep_launch();
+    ptx::grid_dep_wait();
+    const uint64_t tag = threadIdx.x < 32 ? ptx::ld_relaxed_u64(a.mid_launch) : 0;
+    const uint64_t t0 = static_cast<uint64_t>(t) * TILE;
+    const uint32_t cnt = static_cast<uint32_t>(min(static_cast<uint64_t>(TILE), a.n - t0));
+    auto slot = [](uint32_t c) -> uint32_t { return c ^ ((c >> 3) & 3u); };
+
+    const uint8_t* fl = sa.flags + t0 + tid * ITEMS;
+    uint32_t w[FW] = {};
+    if ((tid + 1) * ITEMS <= cnt) {
+        if constexpr (FW == 4) {
+            const uint4 q = *reinterpret_cast<const uint4*>(fl);
+            w[0] = q.x, w[1] = q.y, w[2] = q.z, w[FW - 1] = q.w;
+        } else {
+            const uint2 q = *reinterpret_cast<const uint2*>(fl);
+            w[0] = q.x, w[FW - 1] = q.y;
+        }
+    } else {
+        for (uint32_t i = tid * ITEMS; i < cnt; ++i) {
+            const uint32_t b = i - tid * ITEMS;
+            if (fl[b] != 0) {
+#pragma unroll
+                for (int j = 0; j < FW; ++j)
+                    if (b / 4 == static_cast<uint32_t>(j)) w[j] |= 1u << (8 * (b & 3u));
+            }
+        }
+    }
+    const V* src = static_cast<const V*>(a.in) + t0;
+    Chunk<V> q[CHUNKS];
+#pragma unroll
+    for (int r = 0; r < CHUNKS; ++r) {
+        const uint32_t off = (r * kMidSelThreads + tid) * EPC;
+        if (off + EPC <= cnt) {
+            q[r] = *reinterpret_cast<const Chunk<V>*>(src + off);
+        } else {
+#pragma unroll
+            for (int e = 0; e < EPC; ++e) q[r].v[e] = off + e < cnt ? src[off + e] : V(0);
+        }
+    }
+    const uint32_t mask = nonzero_byte_mask<FW>(w);
+    const uint32_t mine = static_cast<uint32_t>(__popc(mask));
+    const uint32_t inc = warp_inclusive_scan(mine, lane);
+    if (lane == 31) s_wtot[warp] = inc;
+#pragma unroll
+    for (int r = 0; r < CHUNKS; ++r) s_tile[slot(r * kMidSelThreads + tid)] = q[r];
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+#pragma unroll
+    for (int k = 0; k < WARPS; ++k) {
+        const uint32_t x = s_wtot[k];
+        before += static_cast<uint32_t>(k) < warp ? x : 0u;
+        total += x;
+    }
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c) q[c] = s_tile[slot(tid * CHUNKS + c)];
+    __syncthreads();
+
+    // Compact into the tile's own space, at the positions within the tile.
+    V* run = reinterpret_cast<V*>(s_tile);
+    uint32_t pos = before + inc - mine;
+#pragma unroll
+    for (int c = 0; c < CHUNKS; ++c)
+#pragma unroll
+        for (int e = 0; e < EPC; ++e)
+            if ((mask >> (c * EPC + e)) & 1u) run[pos++] = q[c].v[e];
+
+    if (warp == 0) {
+        uint64_t pre = 0;
+        const bool last = t == a.num_tiles - 1;
+        const bool ok = a.num_tiles == 1 || mid_seg_prefix<OpU64>(a, t, tag, total, false, lane, pre);
+        if (lane == 0) {
+            if (!ok) raise_error(a.hdr, kErrLookbackTimeout);
+            if (last) *static_cast<uint64_t*>(a.carry_out) = pre + total;
+            s_pre = ok ? pre : ~0ull;
+        }
+    }
+    __syncthreads();
+    if (s_pre == ~0ull) return;
+    V* out = static_cast<V*>(a.out) + s_pre;
+    for (uint32_t i = tid; i < total; i += kMidSelThreads) out[i] = run[i];
+}
+
+template <typename V>
+cudaError_t launch_mid_select(const ScanArgs& a0, const SelArgs& sa, cudaStream_t stream, LaunchInfo* info) {
+    ScanArgs a = a0;
+    a.desc_stride = a.num_tiles > 32 ? kMidDescStride : 1u;
+    const int grid = static_cast<int>(a.num_tiles);
+    if (info) *info = LaunchInfo{grid, kMidSelThreads, 0};
+    return launch_dependent(mid_select_kernel<V>, grid, kMidSelThreads, 0, stream, a, sa);
+}
+
 template <typename V>
 cudaError_t launch_select_t(const ScanArgs& a, const SelArgs& sa, int num_sms, cudaStream_t stream,
                             LaunchInfo* info) {
@@ -542,6 +664,9 @@ uint32_t select_tile_elems(size_t elem_size) { return elem_size == 8 ? 2048u : 4
 cudaError_t launch_select(size_t elem_size, const ScanArgs& a, const uint8_t* flags, int num_sms, cudaStream_t stream,
                           LaunchInfo* info) {
     const SelArgs sa{flags};
+    if (a.num_tiles <= kMidSelectMaxTiles)
+        return elem_size == 8 ? launch_mid_select<uint64_t>(a, sa, stream, info)
+                              : launch_mid_select<uint32_t>(a, sa, stream, info);
     return elem_size == 8 ? launch_select_t<uint64_t>(a, sa, num_sms, stream, info)
                           : launch_select_t<uint32_t>(a, sa, num_sms, stream, info);
 }
