@@ -64,8 +64,7 @@ cudaError_t launch_l2_t(const ScanArgs& a, int num_sms, cudaStream_t stream, Lau
     const uint32_t units = (a.num_tiles + kL2Unit - 1) / kL2Unit;
     const int grid = persistent_grid(units, occ, num_sms);
     if (info) *info = LaunchInfo{grid, threads, smem};
-    kern<<<grid, threads, smem, stream>>>(a);
-    return cudaGetLastError();
+    return launch_dependent(kern, grid, threads, smem, stream, a);
 }
 
 // Sets up (shared-memory opt-in, occupancy) the four kernels a chained scan

@@ -111,6 +111,8 @@ __global__ void __launch_bounds__(L2Shape<T, RW>::kThreads, 1) scan_l2_kernel(co
         ctrl->end_seq = 0xFFFFFFFFu;
         ptx::fence_mbar_init();
     }
+    ptx::grid_dep_launch();
+    ptx::grid_dep_wait();
     __syncthreads();
 
     const uint32_t epoch = ld_volatile_u32(&a.hdr->epoch);

@@ -340,6 +340,7 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
     // The 128-byte swizzle repeats every 1024 bytes: stages must start on a
     // 1024-byte boundary. (A misaligned window is reported, not used.)
     if ((ptx::smem_addr(smem_raw) & 1023u) != 0) {
+        ptx::grid_dep_wait();
         if (tid == 0) raise_error(a.hdr, kErrPipelineTimeout);
         return;
     }
@@ -375,6 +376,8 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
         ctrl->end_seq = 0xFFFFFFFFu;
         ptx::fence_mbar_init();
     }
+    ptx::grid_dep_launch();
+    ptx::grid_dep_wait();
     if constexpr (SEG)
         for (uint32_t j = tid; j < nsample; j += blockDim.x) ctrl->sample[j] = sg.offsets[min(j * stride, nseg)];
     __syncthreads();

@@ -59,8 +59,7 @@ cudaError_t launch_seg_t(const ScanArgs& a, const SegArgs& sg, const GenericConf
     if (info) *info = LaunchInfo{grid, threads, smem};
     ScanArgs b = a;
     b.desc_stride = units <= kSegStrideMaxUnits ? kSegDescStride : 0u;
-    kern<<<grid, threads, smem, stream>>>(b, sg, maps.in, maps.out);
-    return cudaGetLastError();
+    return launch_dependent(kern, grid, threads, smem, stream, b, sg, maps.in, maps.out);
     }
 }
 

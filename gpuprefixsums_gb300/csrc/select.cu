@@ -146,6 +146,8 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
         ctrl->end_seq = 0xFFFFFFFFu;
         ptx::fence_mbar_init();
     }
+    ptx::grid_dep_launch();
+    ptx::grid_dep_wait();
     __syncthreads();
 
     const uint32_t epoch = ld_volatile_u32(&a.hdr->epoch);
@@ -653,8 +655,7 @@ cudaError_t launch_select_t(const ScanArgs& a, const SelArgs& sa, int num_sms, c
     const uint32_t units = (a.num_tiles + kSelG - 1) / kSelG;
     const int grid = persistent_grid(units, occ, num_sms);
     if (info) *info = LaunchInfo{grid, kSelThreads, smem};
-    kern<<<grid, kSelThreads, smem, stream>>>(a, sa);
-    return cudaGetLastError();
+    return launch_dependent(kern, grid, kSelThreads, smem, stream, a, sa);
 }
 
 }  // namespace

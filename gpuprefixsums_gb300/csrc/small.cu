@@ -10,6 +10,8 @@
 // loads are issued before the current chunk is scanned.
 #include "gps_device.cuh"
 #include "gps_internal.h"
+#include "gps_ptx.cuh"
+#include "launch_util.h"
 
 namespace gps {
 namespace {
@@ -42,6 +44,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     constexpr int ITEMS = kSmallItems<T>;
     constexpr int CHUNK = kSmallThreads * ITEMS;
     __shared__ gps_device::BlockScanStorage<kSmallThreads, T> st;
+    ptx::grid_dep_launch();
+    ptx::grid_dep_wait();
     T carry = carry_in != nullptr ? *carry_in : T(0);
     T v[ITEMS], nxt[ITEMS];
     load_chunk<T, VEC>(in, n, 0, v);
@@ -84,11 +88,8 @@ cudaError_t launch_small_t(const ScanArgs& a, cudaStream_t stream, LaunchInfo* i
     const T* cin = static_cast<const T*>(a.carry_in);
     T* cout = static_cast<T*>(a.carry_out);
     if (info) *info = LaunchInfo{1, kSmallThreads, 0};
-    if (vec)
-        small_scan_kernel<T, INCL, true><<<1, kSmallThreads, 0, stream>>>(in, out, a.n, cin, cout);
-    else
-        small_scan_kernel<T, INCL, false><<<1, kSmallThreads, 0, stream>>>(in, out, a.n, cin, cout);
-    return cudaGetLastError();
+    return vec ? launch_dependent(small_scan_kernel<T, INCL, true>, 1, kSmallThreads, 0, stream, in, out, a.n, cin, cout)
+               : launch_dependent(small_scan_kernel<T, INCL, false>, 1, kSmallThreads, 0, stream, in, out, a.n, cin, cout);
 }
 
 }  // namespace
