@@ -203,6 +203,10 @@ gps_status launch_scan(gps_plan_s* p, bool inclusive, const void* in, void* out,
         a.desc = p->desc_mid;
         a.group_desc = p->group_desc_mid;
         err = gps::launch_mid(p->dtype, inclusive, a, p->num_sms, stream, &p->last_launch);
+    } else if (p->algo == GPS_ALGO_CSDL && !unaligned && p->stall.mode == 0 && p->stall.fallback_polls == 0 &&
+               carry_in == nullptr && carry_out == nullptr &&
+               gps::integer_scan_takes_generic(p->dtype, n, a.num_tiles, p->num_sms)) {
+        err = launch_generic(p, inclusive, a, nullptr, gps::kGenericCandidates[0], stream, &p->last_launch);
     } else if (p->algo == GPS_ALGO_CSDL) {
         err = gps::launch_csdl(p->dtype, inclusive, p->stall.mode != 0 || p->stall.fallback_polls != 0, a, p->num_sms,
                                stream, &p->last_launch);
@@ -247,6 +251,19 @@ size_t dtype_size(gps_dtype dtype) { return dtype == GPS_DTYPE_U64 ? 8 : dtype =
 GenericConfig default_generic_config(uint64_t n, uint32_t tile_elems, int num_sms) {
     const uint64_t units4 = (n + 4ull * tile_elems - 1) / (4ull * tile_elems);
     return units4 >= 2ull * static_cast<uint64_t>(num_sms) ? GenericConfig{4, 1, 1} : GenericConfig{1, 1, 1};
+}
+// Plain integer scans above the mid size run on the generic kernel too, in units
+// of 4 tiles: its reduce warps need no warp scan and no barrier per tile (the
+// aggregator warp scans a unit's row sums once), and its fixed-order lookback
+// has one descriptor per cache line at these sizes. Measured on GB300 against
+// scan_l2_kernel, graph replay: u32 2^24 27.5 / 33.4 us, 2^25 47.6 / 53.4, 2^26
+// 88.9 / 92.0, 2^27 170.9 / 171.9, 2^28 333.1 / 330.7 (so u32 stops at 512 MB);
+// u64 2^23 28.1 / 32.1, 2^25 89.8 / 94.9, 2^27 335.5 / 345.1. Below two units
+// per SM its pipeline does not fill. The tensor maps count rows of 128 bytes in
+// 32 bits.
+bool integer_scan_takes_generic(gps_dtype dtype, uint64_t n, uint32_t tiles, int num_sms) {
+    if (tiles < 8ull * static_cast<uint64_t>(num_sms)) return false;
+    return dtype == GPS_DTYPE_U32 ? n <= (1ull << 27) : n <= (1ull << 34);
 }
 void record_error(const char* msg) { g_last_error = msg; }
 }  // namespace gps
@@ -435,7 +452,7 @@ gps_status prepare_generic(gps_plan_s* p, gps_scan_kind kind, const void* d_in, 
     if (p->algo != GPS_ALGO_CSDL)
         return fail(GPS_ERR_UNSUPPORTED, "batched scans run on chained-scan plans (GPS_ALGO_CSDL)");
     if (d_offsets == nullptr && !generic_only(p->dtype))
-        return fail(GPS_ERR_UNSUPPORTED, "integer plans use the generic kernel for batched scans only");
+        return fail(GPS_ERR_UNSUPPORTED, "plain integer scans have no launch configuration to tune");
     if (n == 0) return GPS_OK;
     if (d_offsets != nullptr && num_segments == 0)
         return fail(GPS_ERR_INVALID_ARGUMENT, "%llu elements but no segments", static_cast<unsigned long long>(n));

@@ -180,6 +180,8 @@ constexpr int kNumGenericCandidates = 8;
 // Untuned choice: units of 4 tiles once there are at least two such units
 // per SM, else single-tile units (more CTAs busy on small inputs).
 GenericConfig default_generic_config(uint64_t n, uint32_t tile_elems, int num_sms);
+// Whether a plain u32 or u64 scan above the mid size runs on the generic kernel.
+bool integer_scan_takes_generic(gps_dtype dtype, uint64_t n, uint32_t tiles, int num_sms);
 
 // Generic single-pass scan (scan_seg.cuh), one per scan operation; `sg` null
 // for a plain scan. Buffers must be 16-byte aligned; descriptors are 16 bytes.
@@ -229,12 +231,10 @@ cudaError_t launch_small(gps_dtype dtype, bool inclusive, const ScanArgs& a, cud
 
 // Integer chained scans up to mid size, one 16 KB tile per CTA (mid.cu); the
 // default upper size of a plan, in bytes of input. Measured on GB300 (graph
-// replay; descriptors one per line): one tile per CTA is faster than the
-// persistent kernel up to 64 MB (u32: 31.8 against 34.4 us at 2^24; u64:
-// 32.1 against 32.8 us at 2^23), slower from 96 MB (u32: 43.7 against 44.6
-// us at 3 x 2^23 at best, 56.5 against 53.7 at 2^25; u64: 44.5 against 43.2
-// at 3 x 2^22).
-constexpr size_t kMidMaxBytes = 64ull << 20;
+// replay) against the persistent kernel that takes over (the generic one):
+// u32 2^22 9.7 against 13.7 us, 2^23 16.6 / 17.8, 10 x 2^20 20.4 / 20.3, 3 x 2^22 24.2 / 22.1, 2^24 31.4 /
+// 27.5; u64 2^23 32.4 / 28.1.
+constexpr size_t kMidMaxBytes = 40ull << 20;
 // Tile descriptors of the one-tile-per-CTA kernels sit one per 128-byte line
 // (a stride of 8 words) when a launch has more than one group of 32 tiles
 // and at most kMidStrideMaxTiles tiles, else packed. Sharing lines between

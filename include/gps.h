@@ -253,11 +253,11 @@ gps_status gps_plan_set_fallback(gps_plan plan, uint32_t fallback_polls);
 gps_status gps_plan_set_small_max(gps_plan plan, uint64_t max_n);
 
 /* Integer scans on a GPS_ALGO_CSDL plan above the one-CTA size and of at
- * most max_n elements (default: 64 MB of input, 2^24 u32 or 2^23 u64) run
+ * most max_n elements (default: 40 MB of input) run
  * as one 16 KB tile per CTA -- a single-pass chained scan without
- * the persistent kernel's pipeline, whose latency dominates at these sizes;
- * larger ones run on the persistent L2-buffered kernel. 0 sends them all to
- * the persistent kernel. Forced-stall and fallback modes always use the
+ * the persistent kernels' pipeline, whose latency dominates at these sizes;
+ * larger ones run on a persistent L2-buffered kernel. 0 sends them all to
+ * the persistent kernels. Forced-stall and fallback modes always use the
  * persistent kernel. Buffers that are not 16-byte aligned take it at every
  * size unless max_n is 0. The kernel takes its tile ids from the block index and
  * relies on the hardware starting lower-numbered blocks first, as CUB's
