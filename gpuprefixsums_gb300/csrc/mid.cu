@@ -33,8 +33,10 @@ namespace gps {
 namespace {
 
 constexpr int kMidThreads = kRowThreads;
-// Resident CTAs per SM the kernel is compiled for.
-constexpr int kMidCtasPerSm = 8;
+// Resident CTAs per SM the kernel is compiled for: 40 registers a thread with
+// the tile held in registers, 32 without.
+template <bool HELD>
+constexpr int kMidCtasPerSm = HELD ? 6 : 8;
 
 // ------------------------------------------------------------ descriptors
 // One 16-byte word per tile: {lo: the value (u32 or u64), hi: status:2 |
@@ -210,23 +212,26 @@ __device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint
 // chunks of row r before tid: the four chunk sums are warp-scanned together,
 // the warp totals go through shared memory in row-major order (row r, warp
 // w at r * 8 + w), and one warp scan of those 32 totals gives every (row,
-// warp) its offset -- one barrier for the whole block scan. Chunks are read
-// twice: for the sums, and after the lookback to scan and store them (the
-// second read hits this SM's L1). Neither tile data nor chunk offsets stay in
-// registers across the lookback, which keeps the kernel at 32 registers and
-// eight CTAs per SM: on 152 SMs up to 1216 tiles (2^22 u32 elements fit) run
-// in one wave. There is no shared-memory staging and no mbarrier to set up,
-// so every CTA issues its loads as soon as it starts.
+// warp) its offset -- one barrier for the whole block scan; the chunk offsets
+// wait in shared memory during the lookback. HELD keeps the tile in registers
+// across the lookback: 40 registers, six CTAs per SM. Otherwise its chunks are
+// read again after it (from L1 or L2): 32 registers, eight CTAs per SM, so that
+// up to 1216 tiles (2^22 u32 elements fit on 152 SMs) run in one wave. Which is
+// faster turns on the number of waves: up to one wave of the HELD form it is
+// ahead (graph replay, u32: 1000 elements 1.43 against 1.62 us, 2^16 2.74 / 2.91,
+// 2^20 5.67 / 5.92, 2^21 7.1 / 7.4), beyond it the other (2^22 11.0 / 9.7, 2^23
+// 17.8 / 16.7). There is no shared-memory staging and no mbarrier to set up, so
+// every CTA issues its loads as soon as it starts.
 //
 // ALIGNED = false takes buffers at any element offset from a 16-byte boundary
 // (tile_rows.cuh), one row at a time after the lookback, which keeps it at 32
 // registers.
 // Bound by the same latency chain as the aligned form. Measured on GB300,
 // 10,000,019 u32 from a view one element past a boundary, into an aligned
-// output: 22.9 us a call, where per-thread element loads and stores (64
+// output: 21.3 us a call, where per-thread element loads and stores (64
 // bytes apart across a warp) took 70.9.
-template <typename T, bool INCL, bool ALIGNED>
-__global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm) mid_vec_kernel(const ScanArgs a) {
+template <typename T, bool INCL, bool ALIGNED, bool HELD>
+__global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm<HELD>) mid_vec_kernel(const ScanArgs a) {
     using Rows = TileRows<T, ALIGNED>;
     constexpr int EPC = Rows::kEpc;
     constexpr int ROWS = Rows::kRows;
@@ -249,10 +254,15 @@ __global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm) mid_vec_kernel(con
     constexpr PlainAccess access;
 
     T cs[ROWS];
+    Chunk<T> held[HELD ? ROWS : 1];
     {
         Chunk<T> q[ROWS];
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) q[r] = rows.load(r, access);
+        if constexpr (HELD) {
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) held[r] = q[r];
+        }
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
             T x = 0;
@@ -296,7 +306,13 @@ __global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm) mid_vec_kernel(con
             }
         }
     };
-    if constexpr (ALIGNED) {
+    if constexpr (HELD) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            scan_chunk(r, held[r]);
+            rows.store(r, held[r], lane, access);
+        }
+    } else if constexpr (ALIGNED) {
         Chunk<T> q[ROWS];
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) q[r] = rows.load(r, access);
@@ -316,7 +332,7 @@ __global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm) mid_vec_kernel(con
 }
 
 template <typename T, bool INCL, bool ALIGNED>
-cudaError_t launch_mid_v(const ScanArgs& a0, cudaStream_t stream, LaunchInfo* info) {
+cudaError_t launch_mid_v(const ScanArgs& a0, int num_sms, cudaStream_t stream, LaunchInfo* info) {
     ScanArgs a = a0;
     // At most one more than the plan's (its descriptor regions have kDescPad
     // to spare).
@@ -328,25 +344,31 @@ cudaError_t launch_mid_v(const ScanArgs& a0, cudaStream_t stream, LaunchInfo* in
     // program that scans one small array after another waits for one launch
     // less each time (2^20 u32: 6.3 -> 5.5 us a call, 32 captured scans of 2^16:
     // 102 -> 89 us).
-    return launch_dependent(mid_vec_kernel<T, INCL, ALIGNED>, grid, kMidThreads, 0, stream, a);
+    // The form that holds its tile, while the launch is one wave of it.
+    return a.num_tiles <= static_cast<uint32_t>(kMidCtasPerSm<true> * num_sms)
+               ? launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, true>, grid, kMidThreads, 0, stream, a)
+               : launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, false>, grid, kMidThreads, 0, stream, a);
 }
 
 template <typename T, bool INCL>
-cudaError_t launch_mid_t(const ScanArgs& a, cudaStream_t stream, LaunchInfo* info) {
+cudaError_t launch_mid_t(const ScanArgs& a, int num_sms, cudaStream_t stream, LaunchInfo* info) {
     if (((reinterpret_cast<uintptr_t>(a.desc) | reinterpret_cast<uintptr_t>(a.group_desc)) & 15u) != 0 ||
         a.desc == nullptr || a.group_desc == nullptr)
         return cudaErrorInvalidValue;
     const bool aligned = ((reinterpret_cast<uintptr_t>(a.in) | reinterpret_cast<uintptr_t>(a.out)) & 15u) == 0;
-    return aligned ? launch_mid_v<T, INCL, true>(a, stream, info) : launch_mid_v<T, INCL, false>(a, stream, info);
+    return aligned ? launch_mid_v<T, INCL, true>(a, num_sms, stream, info)
+                   : launch_mid_v<T, INCL, false>(a, num_sms, stream, info);
 }
 
 }  // namespace
 
-cudaError_t launch_mid(gps_dtype dtype, bool inclusive, const ScanArgs& a, int /*num_sms*/, cudaStream_t stream,
+cudaError_t launch_mid(gps_dtype dtype, bool inclusive, const ScanArgs& a, int num_sms, cudaStream_t stream,
                        LaunchInfo* info) {
     if (dtype == GPS_DTYPE_U64)
-        return inclusive ? launch_mid_t<uint64_t, true>(a, stream, info) : launch_mid_t<uint64_t, false>(a, stream, info);
-    return inclusive ? launch_mid_t<uint32_t, true>(a, stream, info) : launch_mid_t<uint32_t, false>(a, stream, info);
+        return inclusive ? launch_mid_t<uint64_t, true>(a, num_sms, stream, info)
+                         : launch_mid_t<uint64_t, false>(a, num_sms, stream, info);
+    return inclusive ? launch_mid_t<uint32_t, true>(a, num_sms, stream, info)
+                         : launch_mid_t<uint32_t, false>(a, num_sms, stream, info);
 }
 
 }  // namespace gps
