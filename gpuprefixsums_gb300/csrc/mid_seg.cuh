@@ -61,14 +61,15 @@ __device__ __forceinline__ void mid_seg_store(ptx::u64x2* d, uint64_t tag, bool 
     }
 }
 
-// False until every word of the descriptor carries this launch's id.
+// False unless every word of the descriptor carries this launch's number.
 template <class Op>
-__device__ __forceinline__ bool mid_seg_load(const ptx::u64x2* d, uint64_t tag, bool& flag, typename Op::C& c) {
+__device__ __forceinline__ bool mid_seg_decode(const ptx::u64x2 (&d)[Op::kDescWords], uint64_t tag, bool& flag,
+                                               typename Op::C& c) {
     uint64_t words[Op::kDescWords];
     bool ok = true;
 #pragma unroll
     for (int w = 0; w < Op::kDescWords; ++w) {
-        const ptx::u64x2 x = ptx::ld_relaxed_b128(d + w);
+        const ptx::u64x2 x = d[w];
         ok = ok && (x.hi >> 63) != 0 && (x.hi & kMidSegTagMask) == (tag & kMidSegTagMask);
         flag = ((x.hi >> 62) & 1u) != 0;
         words[w] = x.lo;
@@ -96,16 +97,23 @@ __device__ __forceinline__ bool mid_seg_fold(const ScanArgs& a, const ptx::u64x2
     uint32_t polls = 0, backoff = 32;
     uint64_t deadline = 0;
     while (true) {
+        // All loads of a poll are issued before the first is looked at.
+        ptx::u64x2 x[K][Op::kDescWords];
+#pragma unroll
+        for (int j = 0; j < K; ++j)
+#pragma unroll
+            for (int w = 0; w < Op::kDescWords; ++w) {
+                x[j][w] = ptx::u64x2{0, 0};
+                if (!((ready >> j) & 1u)) x[j][w] = ptx::ld_relaxed_b128(d + static_cast<uint64_t>(lane * K + j) * ws + w);
+            }
 #pragma unroll
         for (int j = 0; j < K; ++j) {
-            if (!((ready >> j) & 1u)) {
-                bool hf = false;
-                C cv;
-                if (mid_seg_load<Op>(d + static_cast<uint64_t>(lane * K + j) * ws, tag, hf, cv)) {
-                    v[j] = cv;
-                    f[j] = hf;
-                    ready |= 1u << j;
-                }
+            bool hf = false;
+            C cv;
+            if (!((ready >> j) & 1u) && mid_seg_decode<Op>(x[j], tag, hf, cv)) {
+                v[j] = cv;
+                f[j] = hf;
+                ready |= 1u << j;
             }
         }
         if (__all_sync(kFullMask, ready == (1u << K) - 1u)) break;
