@@ -205,7 +205,7 @@ gps_status launch_scan(gps_plan_s* p, bool inclusive, const void* in, void* out,
         err = gps::launch_mid(p->dtype, inclusive, a, p->num_sms, stream, &p->last_launch);
     } else if (p->algo == GPS_ALGO_CSDL && !unaligned && p->stall.mode == 0 && p->stall.fallback_polls == 0 &&
                carry_in == nullptr && carry_out == nullptr &&
-               gps::integer_scan_takes_generic(p->dtype, n, a.num_tiles, p->num_sms)) {
+               gps::integer_scan_takes_generic(n, a.num_tiles, p->num_sms)) {
         err = launch_generic(p, inclusive, a, nullptr, gps::kGenericCandidates[0], stream, &p->last_launch);
     } else if (p->algo == GPS_ALGO_CSDL) {
         err = gps::launch_csdl(p->dtype, inclusive, p->stall.mode != 0 || p->stall.fallback_polls != 0, a, p->num_sms,
@@ -255,15 +255,12 @@ GenericConfig default_generic_config(uint64_t n, uint32_t tile_elems, int num_sm
 // Plain integer scans above the mid size run on the generic kernel too, in units
 // of 4 tiles: its reduce warps need no warp scan and no barrier per tile (the
 // aggregator warp scans a unit's row sums once), and its fixed-order lookback
-// has one descriptor per cache line at these sizes. Measured on GB300 against
-// scan_l2_kernel, graph replay: u32 2^24 27.5 / 33.4 us, 2^25 47.6 / 53.4, 2^26
-// 88.9 / 92.0, 2^27 170.9 / 171.9, 2^28 333.1 / 330.7 (so u32 stops at 512 MB);
-// u64 2^23 28.1 / 32.1, 2^25 89.8 / 94.9, 2^27 335.5 / 345.1. Below two units
-// per SM its pipeline does not fill. The tensor maps count rows of 128 bytes in
-// 32 bits.
-bool integer_scan_takes_generic(gps_dtype dtype, uint64_t n, uint32_t tiles, int num_sms) {
-    if (tiles < 8ull * static_cast<uint64_t>(num_sms)) return false;
-    return dtype == GPS_DTYPE_U32 ? n <= (1ull << 27) : n <= (1ull << 34);
+// reads 128 descriptors a poll, not 512. Measured on GB300 against
+// scan_l2_kernel, graph replay: u32 2^24 26.3 / 33.4 us, 2^25 46.5 / 53.4, 2^26
+// 86.2 / 92.0, 2^28 320 / 330; u64 2^27 322 / 345. Below two units per SM its
+// pipeline does not fill. The tensor maps count rows of 128 bytes in 32 bits.
+bool integer_scan_takes_generic(uint64_t n, uint32_t tiles, int num_sms) {
+    return tiles >= 8ull * static_cast<uint64_t>(num_sms) && n <= (1ull << 34);
 }
 void record_error(const char* msg) { g_last_error = msg; }
 }  // namespace gps

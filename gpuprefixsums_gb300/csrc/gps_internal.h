@@ -181,7 +181,7 @@ constexpr int kNumGenericCandidates = 8;
 // per SM, else single-tile units (more CTAs busy on small inputs).
 GenericConfig default_generic_config(uint64_t n, uint32_t tile_elems, int num_sms);
 // Whether a plain u32 or u64 scan above the mid size runs on the generic kernel.
-bool integer_scan_takes_generic(gps_dtype dtype, uint64_t n, uint32_t tiles, int num_sms);
+bool integer_scan_takes_generic(uint64_t n, uint32_t tiles, int num_sms);
 
 // Generic single-pass scan (scan_seg.cuh), one per scan operation; `sg` null
 // for a plain scan. Buffers must be 16-byte aligned; descriptors are 16 bytes.
