@@ -112,6 +112,7 @@ struct ScanArgs {
     uint64_t wait_budget_ns;
     StallConfig stall;
     uint64_t* mid_launch;  // one-tile-per-CTA kernels: WsHeader::mid_launch
+    uint32_t units_in_flight;  // generic kernel: per CTA, set by its launcher
 };
 
 // Kernel geometry shared by host and device: RW reduce warps and RW finalize

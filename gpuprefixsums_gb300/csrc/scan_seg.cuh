@@ -218,10 +218,11 @@ __device__ typename Op::C seg_lookback(const ScanArgs& a, uint32_t u, uint32_t e
     };
     // 1. The in-group aggregates. Plain scans issue all loads of a poll before
     // they look at the first (2^26 FP32 88.2 -> 85.8 us, 2^27 u64 334 -> 322);
-    // segmented ones are slower that way (4096 u32 segments 375 -> 393 us, a longer
-    // back-off 385 at best) and look at one descriptor after the other.
+    // segmented ones and structs are slower that way (4096 u32 segments 375 -> 393
+    // us, a longer back-off 385 at best; 2^24 structs 88.7 -> 96.9) and look at one
+    // descriptor after the other.
     while (true) {
-        if constexpr (SEG) {
+        if constexpr (SEG || Op::kDescWords > 1) {
 #pragma unroll
             for (int j = 0; j < K; ++j) {
                 bool hf = false;
@@ -411,9 +412,19 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
     }
     ptx::grid_dep_launch();
     ptx::grid_dep_wait();
-    if constexpr (SEG)
-        for (uint32_t j = tid; j < nsample; j += blockDim.x) ctrl->sample[j] = sg.offsets[min(j * stride, nseg)];
     __syncthreads();
+    // The reduce and finalize warps, idle until the first tile lands, read the
+    // samples for the head warp; the loaders do not wait for them (2^26 u32 in 500
+    // segments 91.1 -> 87.4 us, 100,000 segments 103 -> 97; read by the head warp
+    // alone 97 and 111).
+    constexpr uint32_t kSampleThreads = 2 * NROLE;
+    if constexpr (SEG) {
+        if (warp >= kWarpReduce) {
+            for (uint32_t j = tid - kWarpReduce * 32; j < nsample; j += kSampleThreads)
+                ctrl->sample[j] = sg.offsets[min(j * stride, nseg)];
+            ptx::named_bar_arrive(1, kSampleThreads + 32);
+        }
+    }
 
     const uint32_t epoch = ld_volatile_u32(&a.hdr->epoch);
     const uint64_t budget = a.wait_budget_ns;
@@ -501,7 +512,10 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
             bool ok = true;
             for (uint32_t i = 0; ok; ++i) {
                 const int q = static_cast<int>(i % Q);
-                if (i >= Q && !wait1(&ctrl->ufree[q], ((i - Q) / Q) & 1u, long_budget)) break;
+                // At most a.units_in_flight (<= Q) units between claim and output.
+                if (i >= a.units_in_flight &&
+                    !wait1(&ctrl->ufree[(i - a.units_in_flight) % Q], ((i - a.units_in_flight) / Q) & 1u, long_budget))
+                    break;
                 // The unit id is taken only now, when its loads follow, and
                 // the unit's full rows are prefetched into L2 (see
                 // scan_l2.cuh; measured on GB300: +3-4% for the integer and
@@ -655,6 +669,7 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
         if constexpr (!SEG) {
             return;
         } else {
+            ptx::named_bar_sync(1, kSampleThreads + 32);
             // For each unit of this CTA, marks the elements where a segment
             // starts: the offsets o with tile_start <= o < tile_end, found by a
             // search in the shared samples, then one coalesced read of the
@@ -743,7 +758,12 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
             }
             const uint32_t u = ctrl->unit_of[q];
             if (u == kTileEnd) break;
-            const C pre = u == 0 ? Op::chain_zero() : seg_lookback<Op, SEG>(a, u, epoch, lane);
+            // Compensated batches, whose units take longest to aggregate, look back
+            // once their own is in: until then most polls are in vain (121.2 ->
+            // 118.4 us for 2^26 elements; the other types lose up to 1% that way).
+            constexpr bool kLate = SEG && sizeof(S) > sizeof(T);
+            C pre = Op::chain_zero();
+            if (!kLate && u != 0) pre = seg_lookback<Op, SEG>(a, u, epoch, lane);
             uint32_t state = 0;
             if (lane == 0) {
                 const uint64_t deadline = ptx::global_timer_ns() + long_budget;
@@ -764,6 +784,7 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
                 if (lane == 0 && state == 2) raise_error(a.hdr, kErrPipelineTimeout);
                 break;
             }
+            if (kLate && u != 0) pre = seg_lookback<Op, SEG>(a, u, epoch, lane);
             const C agg = ctrl->uagg[q];
             const bool flag = ctrl->uflag[q] != 0;
             const C incl = flag ? agg : Op::chain_add(pre, agg);

@@ -8,8 +8,7 @@
 
 namespace gps {
 
-// 4 reduce + 4 finalize warps over 16 KB tiles, 6 units in flight per CTA.
-// Stages: as many as fit in 227 KB of shared memory next to the control
+// 4 reduce + 4 finalize warps over 16 KB tiles. Stages: as many as fit in 227 KB of shared memory next to the control
 // block (whose per-thread prefixes and head bitmaps grow with the state size
 // and the unit), taken as 4 reduce-pass + 9 scan-pass stages when 13 fit
 // (measured on GB300: 4 + 9 beats 5 + 8 by 3-8% on the batched workloads),
@@ -19,21 +18,31 @@ namespace gps {
 // took batched FP32 from 6.17 down to 4.79. The unit (1 or 4 tiles) and the
 // CTA count come from the plan's launch configuration (GenericConfig).
 constexpr int kSegWarps = 4;
-constexpr int kSegQueue = 6;
+// Units in flight per CTA: each waits in L2 (64 KB, or 16 KB in single-tile
+// units) between the two passes, 152 x 6 x 64 KB at most. Measured on GB300:
+// batched scans (5 against 6; 4096 u32 segments 359 / 366 us, 2^27 u64 337 / 345, 2^24
+// compensated 39.0 / 39.4) and structs (2^24 88.7 / 94.0: the smaller control
+// block makes room for a fourth reduce-pass stage) take 5. Plain scans of 512 MB and
+// more take 5 of the 6 there is room for (2^28 u32 317 / 322, 2^27 163 / 165; 2^26
+// FP32 88.0 / 87.3, compensated 93.1 / 92.7); 4 or 3 are slower everywhere but for
+// compensated batches (2^28 u32 333 and 385).
+template <class Op, bool SEG>
+constexpr int kSegQueue = SEG || sizeof(typename Op::S) == 16 ? 5 : 6;
+constexpr uint64_t kSegDeepBytes = 512ull << 20;
 constexpr size_t kMaxSmem = 232448;
 
 template <class Op, int G, bool SEG, int SPLIT>
 struct SegStages {
     static constexpr int RW = kSegWarps * SPLIT;  // warps per role
-    static constexpr bool k13 = seg_smem_bytes<Op, RW, 4, 9, kSegQueue, G, SEG>() <= kMaxSmem;
-    static constexpr bool k12 = seg_smem_bytes<Op, RW, 4, 8, kSegQueue, G, SEG>() <= kMaxSmem;
-    static constexpr bool k11 = seg_smem_bytes<Op, RW, 3, 8, kSegQueue, G, SEG>() <= kMaxSmem;
-    static constexpr bool k10 = seg_smem_bytes<Op, RW, 3, 7, kSegQueue, G, SEG>() <= kMaxSmem;
+    static constexpr bool k13 = seg_smem_bytes<Op, RW, 4, 9, kSegQueue<Op, SEG>, G, SEG>() <= kMaxSmem;
+    static constexpr bool k12 = seg_smem_bytes<Op, RW, 4, 8, kSegQueue<Op, SEG>, G, SEG>() <= kMaxSmem;
+    static constexpr bool k11 = seg_smem_bytes<Op, RW, 3, 8, kSegQueue<Op, SEG>, G, SEG>() <= kMaxSmem;
+    static constexpr bool k10 = seg_smem_bytes<Op, RW, 3, 7, kSegQueue<Op, SEG>, G, SEG>() <= kMaxSmem;
     static constexpr int RS = (k13 || k12 || k11) ? 4 : 3;
     static constexpr int SS = k13 ? 9 : k12 ? 8 : (k11 || k10) ? 7 : 6;
     // Two threads per row double the per-thread prefixes: some types do not
     // fit 9 stages then, and that shape is not offered for them.
-    static constexpr bool kFits = seg_smem_bytes<Op, RW, RS, SS, kSegQueue, G, SEG>() <= kMaxSmem;
+    static constexpr bool kFits = seg_smem_bytes<Op, RW, RS, SS, kSegQueue<Op, SEG>, G, SEG>() <= kMaxSmem;
     static_assert(kFits || SPLIT > 1, "227 KB per CTA");
 };
 
@@ -44,8 +53,8 @@ cudaError_t launch_seg_t(const ScanArgs& a, const SegArgs& sg, const GenericConf
     if constexpr (!St::kFits) {
         return cudaErrorNotSupported;
     } else {
-    auto kern = scan_seg_kernel<Op, St::RW, St::RS, St::SS, kSegQueue, UNIT, INCL, SEG>;
-    constexpr size_t smem = seg_smem_bytes<Op, St::RW, St::RS, St::SS, kSegQueue, UNIT, SEG>();
+    auto kern = scan_seg_kernel<Op, St::RW, St::RS, St::SS, kSegQueue<Op, SEG>, UNIT, INCL, SEG>;
+    constexpr size_t smem = seg_smem_bytes<Op, St::RW, St::RS, St::SS, kSegQueue<Op, SEG>, UNIT, SEG>();
     constexpr int threads = SegShape<Op, St::RW>::kThreads;
     RowMaps maps;
     cudaError_t err = encode_row_maps(a.in, a.out, a.n, static_cast<uint32_t>(sizeof(typename Op::T)), &maps);
@@ -58,6 +67,8 @@ cudaError_t launch_seg_t(const ScanArgs& a, const SegArgs& sg, const GenericConf
     const int grid = persistent_grid(units, 1, ctas);
     if (info) *info = LaunchInfo{grid, threads, smem};
     ScanArgs b = a;
+    b.units_in_flight = kSegQueue<Op, SEG>;
+    if (b.units_in_flight > 5 && a.n * sizeof(typename Op::T) >= kSegDeepBytes) b.units_in_flight = 5;
     b.desc_stride = units <= kSegStrideMaxUnits ? kSegDescStride : 0u;
     return launch_dependent(kern, grid, threads, smem, stream, b, sg, maps.in, maps.out);
     }
