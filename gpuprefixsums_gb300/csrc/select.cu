@@ -26,8 +26,10 @@
 // as they arrive (one warp per scheduler, each waiting on its own shared-memory
 // stores). Measured on GB300, 2^28 u32, 30% selected: one group 302 us, two
 // groups with 6 units in flight 274, with 8 units and 6 instead of 8 flag
-// stages 264 (6.3 TB/s, 0.95 of the copy rate), 9 or 12 units 265 and 271
-// (fewer flag stages fit); 80% selected 335 / 343 / 334 us.
+// stages 264, 9 or 12 units 265 and 271 (fewer flag stages fit); 80% selected
+// 335 / 343 / 334 us. With lookback windows of 32 descriptors, one load a lane,
+// instead of 256: 260 us (6.4 TB/s, 0.96 of the copy rate), 80% selected 330, 2^24
+// 25.5 against 27.1.
 #include "launch_util.h"
 #include "mid_seg.cuh"
 
@@ -316,7 +318,7 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
             const uint32_t u = ctrl->unit_of[q];
             if (u == kTileEnd) break;
             const uint64_t pre =
-                u == 0 ? 0ull : lookback<uint64_t, TILE * G, false>(a, u, epoch, lane, 0ull, own_prev, own_incl);
+                u == 0 ? 0ull : lookback<uint64_t, TILE * G, false, 0, 16>(a, u, epoch, lane, 0ull, own_prev, own_incl);
             uint32_t state = 0;  // 0 reduced, 1 reduce warps stopped, 2 timeout
             if (lane == 0) {
                 const uint64_t deadline = ptx::global_timer_ns() + long_budget;
