@@ -70,8 +70,8 @@ struct StallConfig {
 // Fixed-order lookback of the generic kernel (scan_seg.cuh): lookback units
 // per group, and the group descriptors a plan keeps for up to `units` units
 // (one more than the groups, as slack).
-constexpr uint32_t kDetGroupUnits = 128;
-constexpr uint64_t det_group_slots(uint64_t units) { return (units + kDetGroupUnits - 1) / kDetGroupUnits + 1; }
+constexpr uint32_t det_group_units(int unit_tiles) { return unit_tiles == 1 ? 128u : 64u; }
+constexpr uint64_t det_group_slots(uint64_t units) { return (units + 63) / 64 + 1; }
 
 // The generic kernel's unit and group descriptors sit one per 128-byte line
 // (a stride of 8 words) when a launch has at most kSegStrideMaxUnits
@@ -105,7 +105,7 @@ struct ScanArgs {
     WsHeader* hdr;       // plan state (counters, epoch, error flags)
     void* desc;          // tile descriptors (lookback)
     // Descriptors of groups: of 32 tiles for the one-tile-per-CTA kernels, of
-    // kDetGroupUnits lookback units for the generic kernel.
+    // det_group_units() lookback units for the generic kernel.
     void* group_desc;
     const void* carry_in;  // optional: one element added to every output
     void* carry_out;       // optional: receives carry_in + sum of all n inputs

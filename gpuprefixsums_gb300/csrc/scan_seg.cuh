@@ -155,7 +155,7 @@ __device__ __forceinline__ uint32_t desc_load(const ptx::u64x2* desc, uint64_t u
 // Lookback of the generic kernel, in a fixed order. A decoupled lookback
 // that sums whichever predecessors' descriptors it finds ready makes the
 // rounding of a floating-point prefix depend on timing; here the units form
-// groups of G = kDetGroupUnits, a unit's descriptor holds its aggregate only
+// groups of G = det_group_units(), a unit's descriptor holds its aggregate only
 // (it is never upgraded to an inclusive prefix), and the prefix of unit u in
 // group g is
 //     P(g) + fold(aggregates of units G*g .. u-1),
@@ -170,24 +170,28 @@ __device__ __forceinline__ uint32_t desc_load(const ptx::u64x2* desc, uint64_t u
 // group one at a time, one L2 round trip per G units, which stays off the
 // critical path while G units take longer to stream than that round trip.
 // Measured on GB300 against the lookback that stops at the nearest
-// inclusive prefix (windows of 256 descriptors, back-off up to 1 us): 2^28
+// inclusive prefix (windows of 256 descriptors, back-off up to 1 us), in groups of
+// 128: 2^28
 // FP32 in 333 against 342 us, compensated 344 against 355 us, 4096 batched
 // u32 segments (305 M elements) in 381 against 395 us, compensated FP32
 // 506 against 564 us (units of 4 tiles). Groups of 256 units took 348, 357,
 // 390 and 502 us. A back-off of up to 1 us instead of 128 ns while waiting
 // took 338, 349, 380 and 502 us, and 656 against 555 us for 2^28 FP32 in
-// single-tile units, where a group streams in about a microsecond.
-static_assert(kDetGroupUnits % 32 == 0 && kDetGroupUnits <= 32 * 32, "whole lanes of at most 32 units");
+// single-tile units, where a group streams in about a microsecond. Units of 4
+// tiles now take groups of 64 (two descriptors a lane; a group is 4 MB): batched
+// 2^28 u32 315 against 320 us, 2^24 structs 87.2 / 89.3, compensated 2^26 91.6 / 92.4,
+// the others alike; single-tile units stay at 128 (2 MB).
 
-template <class Op, bool SEG>
+template <class Op, bool SEG, uint32_t GROUP>
 __device__ typename Op::C seg_lookback(const ScanArgs& a, uint32_t u, uint32_t epoch, uint32_t lane) {
     using C = typename Op::C;
     const uint32_t ws = desc_words<Op>(a);
-    constexpr int K = static_cast<int>(kDetGroupUnits / 32);  // units per lane
+    static_assert(GROUP % 32 == 0 && GROUP <= 32 * 32, "whole lanes of at most 32 units");
+    constexpr int K = static_cast<int>(GROUP / 32);  // units per lane
     const ptx::u64x2* desc = static_cast<const ptx::u64x2*>(a.desc);
     const ptx::u64x2* gdesc = static_cast<const ptx::u64x2*>(a.group_desc);
-    const uint32_t g = u / kDetGroupUnits;
-    const uint32_t i0 = g * kDetGroupUnits;
+    const uint32_t g = u / GROUP;
+    const uint32_t i0 = g * GROUP;
     const uint32_t cnt = u - i0;  // in-group predecessors
     C v[K];
     bool f[K];
@@ -763,7 +767,7 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
             // 118.4 us for 2^26 elements; the other types lose up to 1% that way).
             constexpr bool kLate = SEG && sizeof(S) > sizeof(T);
             C pre = Op::chain_zero();
-            if (!kLate && u != 0) pre = seg_lookback<Op, SEG>(a, u, epoch, lane);
+            if (!kLate && u != 0) pre = seg_lookback<Op, SEG, det_group_units(G)>(a, u, epoch, lane);
             uint32_t state = 0;
             if (lane == 0) {
                 const uint64_t deadline = ptx::global_timer_ns() + long_budget;
@@ -784,14 +788,15 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
                 if (lane == 0 && state == 2) raise_error(a.hdr, kErrPipelineTimeout);
                 break;
             }
-            if (kLate && u != 0) pre = seg_lookback<Op, SEG>(a, u, epoch, lane);
+            if (kLate && u != 0) pre = seg_lookback<Op, SEG, det_group_units(G)>(a, u, epoch, lane);
             const C agg = ctrl->uagg[q];
             const bool flag = ctrl->uflag[q] != 0;
             const C incl = flag ? agg : Op::chain_add(pre, agg);
             if (lane == 0) {
                 // The last unit of a group passes the group prefix on.
-                if ((u % kDetGroupUnits) == kDetGroupUnits - 1)
-                    desc_store<Op>(static_cast<ptx::u64x2*>(a.group_desc), u / kDetGroupUnits, desc_words<Op>(a),
+                constexpr uint32_t kGroup = det_group_units(G);
+                if ((u % kGroup) == kGroup - 1)
+                    desc_store<Op>(static_cast<ptx::u64x2*>(a.group_desc), u / kGroup, desc_words<Op>(a),
                                    kInclusive, false,
                                    epoch, incl);
                 ctrl->upre[q] = pre;
