@@ -70,7 +70,9 @@ struct StallConfig {
 // Fixed-order lookback of the generic kernel (scan_seg.cuh): lookback units
 // per group, and the group descriptors a plan keeps for up to `units` units
 // (one more than the groups, as slack).
-constexpr uint32_t det_group_units(int unit_tiles) { return unit_tiles == 1 ? 128u : 64u; }
+constexpr uint32_t det_group_units(int unit_tiles, bool long_groups) {
+    return unit_tiles == 1 || long_groups ? 128u : 64u;
+}
 constexpr uint64_t det_group_slots(uint64_t units) { return (units + 63) / 64 + 1; }
 
 // The generic kernel's unit and group descriptors sit one per 128-byte line

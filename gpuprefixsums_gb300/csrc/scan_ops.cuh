@@ -6,6 +6,8 @@
 //      for the compensated FP32 scan),
 //   C  value carried between lookback units in the tile descriptors (the
 //      element type, or FP64 for the compensated FP32 scan),
+//   kLongGroups  whether the lookback keeps its longer groups (fewer roundings
+//      in the chain of group prefixes),
 // and the associative combine of S and of C. Integer scans wrap mod 2^w.
 #pragma once
 #include <cstdint>
@@ -38,6 +40,7 @@ struct OpInt {
     using T = U;
     using S = U;
     using C = U;
+    static constexpr bool kLongGroups = false;
     static constexpr bool kPackedRowSum = false;
     __device__ static S zero() { return 0; }
     __device__ static S lift(T x) { return x; }
@@ -69,6 +72,7 @@ struct OpF32 {
     using T = float;
     using S = float;
     using C = float;
+    static constexpr bool kLongGroups = true;
     static constexpr bool kPackedRowSum = false;
     __device__ static S zero() { return 0.0f; }
     __device__ static S lift(T x) { return x; }
@@ -135,6 +139,7 @@ struct OpF32C {
     using C = double;
     // The reduce pass sums a row as two half-chains (even and odd items) in
     // packed FP32x2 TwoSums: half the instructions of one chain.
+    static constexpr bool kLongGroups = false;
     static constexpr bool kPackedRowSum = true;
     __device__ static S zero() { return F2{0.0f, 0.0f}; }
     __device__ static S lift(T x) { return F2{x, 0.0f}; }
@@ -218,6 +223,7 @@ struct OpU32x4 {
     using T = uint4;
     using S = uint4;
     using C = uint4;
+    static constexpr bool kLongGroups = false;
     static constexpr bool kPackedRowSum = false;
     static constexpr int kDescWords = 2;
     __device__ static S zero() { return make_uint4(0u, 0u, 0u, 0u); }
