@@ -22,10 +22,14 @@
 // j + 1 writes while launch j reads, and launch j - 1 has finished by then.
 //
 // Bound by HBM (25 MB read and 25 written a launch, 7.5 us at the copy rate) and
-// the end of each launch: 9.7 us a launch. Measured on GB300, u32, against
-// three launches over the whole input (reduce, a one-CTA spine over one sum a
-// tile, propagate): 2^20 9.5 -> 5.1 us, 2^24 39 -> 32, 2^26 142 -> 109, 2^28
-// 542 -> 421; a view of 10,000,019 elements off a 16-byte boundary 167 -> 25.
+// the end of each launch: 8.8 us a launch. While the launch ahead drains, no
+// output can be written: the last tile of the range to reduce is therefore asked
+// for only then, into shared memory, and added at the end (2^28 u32 421 -> 384 us;
+// all of the range that way 422; one chunk more between the two readings, without
+// the wait, 569). Measured on GB300, u32, against three launches over the whole
+// input (reduce, a one-CTA spine over one sum a tile, propagate): 2^20 9.5 -> 5.1
+// us, 2^24 39 -> 31, 2^26 142 -> 102, 2^28 542 -> 384; a view of 10,000,019 elements
+// off a 16-byte boundary 167 -> 25.
 #include "launch_util.h"
 #include "tile_rows.cuh"
 
@@ -36,9 +40,10 @@ namespace {
 constexpr int kRtsCtasPerSm = 5;
 // Tiles of a CTA's range in one chunk, at most: 25 MB a chunk. Two chunks wait
 // in L2 at a time, next to what is being written. Measured on GB300, 2^28 u32:
-// 2 tiles 421 us, 1 tile 516 (the end of a launch costs 2 us), 3 tiles 438 and
-// 4 463 (part of the chunk has left L2 by the second reading); 4 or 6 CTAs per
-// SM 438 and 430. Without evict-last loads in the reduce 491.
+// 2 tiles 384 us, 3 tiles 419 and 4 459 (part of the chunk has left L2 by the
+// second reading), 1 tile 516 before the late tile (the end of a launch costs 2
+// us); 4 or 6 CTAs per SM 393 and 387. Without evict-last loads in the reduce 491
+// against 421.
 constexpr uint32_t kRtsTiles = 2;
 
 struct RtsArgs {
@@ -53,6 +58,8 @@ struct RtsArgs {
     void* prefixes;  // [3] sum of the chunks before
     const void* carry_in;
     void* carry_out;
+    WsHeader* hdr;
+    uint64_t wait_budget_ns;
 };
 
 template <typename T, bool INCL, bool ALIGNED>
@@ -63,20 +70,49 @@ __global__ void __launch_bounds__(kRowThreads, kRtsCtasPerSm) rts_kernel(const R
     static_assert(ROWS * WARPS == 32, "one warp scans all (row, warp) totals");
     __shared__ T s_tot[2][32];
     __shared__ T s_pre[2][WARPS];
+    __shared__ uint64_t s_bar;
+    extern __shared__ __align__(128) uint8_t s_raw[];  // one tile, where a launch has a reduce and a propagate part
+    T* s_stage = reinterpret_cast<T*>(s_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t ranges = gridDim.x, b = blockIdx.x;
     T* sums = static_cast<T*>(a.sums);
     T* prefixes = static_cast<T*>(a.prefixes);
 
     if (a.chunk == 0) ptx::grid_dep_wait();  // the input's producers
-    // Reduce: one range of chunk a.chunk. L2 keeps what it reads.
+    // Reduce: one range of chunk a.chunk. L2 keeps what it reads. The last tile
+    // of the range is only asked for before the wait below, into shared memory,
+    // and added at the end: it keeps HBM busy while the launch ahead drains.
+    const uint64_t r_begin = (static_cast<uint64_t>(a.chunk) * ranges + b) * a.range_tiles;
+    uint64_t r_end = a.chunk < a.chunks ? min(r_begin + a.range_tiles, static_cast<uint64_t>(a.tiles)) : 0;
+    bool deferred = false;
+    if (a.chunk != 0 && r_begin < r_end) {
+        const Rows rows(a.in, a.out, a.n, static_cast<uint32_t>(r_end - 1), 0);
+        deferred = rows.full;
+        if (deferred) {
+            --r_end;
+            if (tid == 0) {
+                ptx::mbar_init(&s_bar, 1);
+                ptx::fence_mbar_init();
+            }
+        }
+    }
     T acc = 0;
+    auto publish_sum = [&]() {
+        acc = warp_sum(acc);
+        __syncthreads();
+        if (lane == 0) s_pre[0][warp] = acc;
+        __syncthreads();
+        if (tid == 0) {
+            T x = 0;
+#pragma unroll
+            for (int w = 0; w < WARPS; ++w) x += s_pre[0][w];
+            sums[(a.chunk % 3) * ranges + b] = x;
+        }
+    };
     if (a.chunk < a.chunks) {
         const PolicyAccess pol{ptx::policy_evict_last()};
-        const uint64_t begin = (static_cast<uint64_t>(a.chunk) * ranges + b) * a.range_tiles;
-        const uint64_t end = min(begin + a.range_tiles, static_cast<uint64_t>(a.tiles));
 #pragma unroll 2
-        for (uint64_t t = begin; t < end; ++t) {
+        for (uint64_t t = r_begin; t < r_end; ++t) {
             const Rows rows(a.in, a.out, a.n, static_cast<uint32_t>(t), tid);
             Chunk<T> q[ROWS];
 #pragma unroll
@@ -86,15 +122,7 @@ __global__ void __launch_bounds__(kRowThreads, kRtsCtasPerSm) rts_kernel(const R
 #pragma unroll
                 for (int e = 0; e < Rows::kEpc; ++e) acc += q[r].v[e];
         }
-        acc = warp_sum(acc);
-        if (lane == 0) s_pre[0][warp] = acc;
-        __syncthreads();
-        if (tid == 0) {
-            T x = 0;
-#pragma unroll
-            for (int w = 0; w < WARPS; ++w) x += s_pre[0][w];
-            sums[(a.chunk % 3) * ranges + b] = x;
-        }
+        if (!deferred) publish_sum();
         __syncthreads();
     }
     if (a.chunk == 0) {
@@ -129,6 +157,11 @@ __global__ void __launch_bounds__(kRowThreads, kRtsCtasPerSm) rts_kernel(const R
             off[r] = inc - x;
         }
         if (t == begin) {
+            if (deferred && tid == 0) {
+                const Rows last(a.in, a.out, a.n, static_cast<uint32_t>(r_end), 0);
+                ptx::mbar_arrive_expect_tx(&s_bar, 16384u);
+                ptx::bulk_load_hint(s_stage, last.src, 16384u, &s_bar, ptx::policy_evict_last());
+            }
             ptx::grid_dep_wait();
             ptx::grid_dep_launch();
             const T* cs = sums + (c % 3) * ranges;
@@ -180,6 +213,18 @@ __global__ void __launch_bounds__(kRowThreads, kRtsCtasPerSm) rts_kernel(const R
         }
         pre += __shfl_sync(kFullMask, xi, 31);
     }
+    if (deferred) {
+        if (!ptx::mbar_try_wait(&s_bar, 0) &&
+            !ptx::mbar_wait_bounded(&s_bar, 0, ptx::global_timer_ns() + a.wait_budget_ns))
+            raise_error(a.hdr, kErrPipelineTimeout);
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            const Chunk<T> q = reinterpret_cast<const Chunk<T>*>(s_stage)[r * kRowThreads + tid];
+#pragma unroll
+            for (int e = 0; e < Rows::kEpc; ++e) acc += q.v[e];
+        }
+        publish_sum();
+    }
 }
 
 // Ranges per chunk, tiles per range and chunks of a scan of `tiles` tiles:
@@ -203,13 +248,14 @@ cudaError_t dispatch_rts(bool inclusive, const ScanArgs& s, void* scratch, int n
     T* sums = static_cast<T*>(scratch);
     RtsArgs a{s.in,      s.out, s.n,       tiles,
               sh.range_tiles, 0,     sh.chunks, sums,
-              sums + 3ull * static_cast<uint64_t>(kRtsCtasPerSm * num_sms), s.carry_in, s.carry_out};
+              sums + 3ull * static_cast<uint64_t>(kRtsCtasPerSm * num_sms), s.carry_in, s.carry_out, s.hdr, s.wait_budget_ns};
     const int grid = static_cast<int>(sh.ranges);
-    if (info) *info = LaunchInfo{grid, kRowThreads, 0};
+    const size_t smem = sh.chunks > 1 ? 16384 : 0;
+    if (info) *info = LaunchInfo{grid, kRowThreads, smem};
     for (; a.chunk <= sh.chunks; ++a.chunk) {
         const cudaError_t err =
-            inclusive ? launch_dependent(rts_kernel<T, true, ALIGNED>, grid, kRowThreads, 0, stream, a)
-                      : launch_dependent(rts_kernel<T, false, ALIGNED>, grid, kRowThreads, 0, stream, a);
+            inclusive ? launch_dependent(rts_kernel<T, true, ALIGNED>, grid, kRowThreads, smem, stream, a)
+                      : launch_dependent(rts_kernel<T, false, ALIGNED>, grid, kRowThreads, smem, stream, a);
         if (err != cudaSuccess) return err;
     }
     return cudaSuccess;
