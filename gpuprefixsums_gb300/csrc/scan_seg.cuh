@@ -333,16 +333,24 @@ constexpr size_t seg_smem_bytes() {
            sizeof(SegCtrl<Op, RW, RS, SS, Q, G, SEG>);
 }
 
-template <class Op, int RW>
+template <class Op, int RW, bool SEG>
 struct SegShape {
     static constexpr int kLookbackWarps = 3;
+    // Groups of RW finalize warps, each with stages of its own: two for segmented
+    // scans and for states of 8 bytes, one for the rest. A single group is one warp
+    // per scheduler, each waiting on its own chain. Measured on GB300, one group
+    // against two: compensated FP32 2^26 91.7 / 85.9 us, in 500 segments 117 / 108, in
+    // 20,000 151 / 131; batched 2^28 u32 317 / 310, 2^26 u64 174 / 162, 2^24 structs
+    // 103 / 99; plain 2^24 u64 48.7 / 46.3, but 2^28 u32 318.1 / 319.5 (three groups:
+    // compensated batches 117 / 143).
+    static constexpr int kFinalGroups = RW == 4 && (SEG || sizeof(typename Op::S) == 8) ? 2 : 1;
     // R-loader, S-loader, storer, head warp, lookback warps, aggregator,
     // reduce warps, finalize warps.
-    static constexpr int kThreads = 32 * (5 + kLookbackWarps + 2 * RW);
+    static constexpr int kThreads = 32 * (5 + kLookbackWarps + (1 + kFinalGroups) * RW);
 };
 
 template <class Op, int RW, int RS, int SS, int Q, int G, bool INCL, bool SEG>
-__global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
+__global__ void __launch_bounds__(SegShape<Op, RW, SEG>::kThreads, 1)
     scan_seg_kernel(const ScanArgs a, const SegArgs sg, const __grid_constant__ CUtensorMap tin,
                     const __grid_constant__ CUtensorMap tout) {
     using T = typename Op::T;
@@ -358,8 +366,9 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
     constexpr int CHUNKS = ITEMS / EPC;
     constexpr uint32_t NROLE = RW * 32;
     constexpr uint32_t ROWS = 128;  // rows per tile
-    constexpr uint32_t LW = SegShape<Op, RW>::kLookbackWarps;
+    constexpr uint32_t LW = SegShape<Op, RW, SEG>::kLookbackWarps;
     constexpr uint32_t kWarpLookback = 4, kWarpAgg = 4 + LW, kWarpReduce = 5 + LW, kWarpFinal = 5 + LW + RW;
+    constexpr uint32_t FG = SegShape<Op, RW, SEG>::kFinalGroups;
     constexpr uint32_t kLaneEntries = G * RW;  // aggregator entries per lane
     auto entry_at = [](uint32_t j) -> uint32_t { return j + j / kLaneEntries; };
     constexpr int kHeadWords = TILE / 32;
@@ -411,7 +420,7 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
             ptx::mbar_init(&ctrl->ustates[q], 1);
             ptx::mbar_init(&ctrl->ureduced[q], 1);
             ptx::mbar_init(&ctrl->uprefix[q], 1);
-            ptx::mbar_init(&ctrl->ufree[q], RW);
+            ptx::mbar_init(&ctrl->ufree[q], FG == 1 ? RW : RW * G);
         }
         ctrl->end_seq = 0xFFFFFFFFu;
         ptx::fence_mbar_init();
@@ -419,13 +428,13 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
     ptx::grid_dep_launch();
     ptx::grid_dep_wait();
     __syncthreads();
-    // The reduce and finalize warps, idle until the first tile lands, read the
+    // The reduce warps and RW finalize warps, idle until the first tile lands, read the
     // samples for the head warp; the loaders do not wait for them (2^26 u32 in 500
     // segments 91.1 -> 87.4 us, 100,000 segments 103 -> 97; read by the head warp
     // alone 97 and 111).
     constexpr uint32_t kSampleThreads = 2 * NROLE;
     if constexpr (SEG) {
-        if (warp >= kWarpReduce) {
+        if (warp >= kWarpReduce && warp < kWarpFinal + RW) {
             for (uint32_t j = tid - kWarpReduce * 32; j < nsample; j += kSampleThreads)
                 ctrl->sample[j] = sg.offsets[min(j * stride, nseg)];
             ptx::named_bar_arrive(1, kSampleThreads + 32);
@@ -602,7 +611,9 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
                         break;
                     }
                 }
-                for (int k = 0; k < (end ? 1 : G); ++k, ++sn) {
+                // At the end, a stage of every finalize group says so (two in a row
+                // may belong to one group where SS is odd).
+                for (int k = 0; k < (end ? (FG == 1 ? 1 : static_cast<int>(FG) + 1) : G); ++k, ++sn) {
                     const int s = static_cast<int>(sn % SS);
                     if (sn >= SS && !wait1(&ctrl->sfree[s], ((sn - SS) / SS) & 1u, long_budget)) {
                         ok = false;
@@ -611,7 +622,7 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
                     if (end) {
                         ctrl->s_tile[s] = kTileEnd;
                         ptx::mbar_arrive(&ctrl->sfull[s]);
-                        break;
+                        continue;
                     }
                     const uint32_t t = u * G + k;
                     ctrl->s_tile[s] = t;
@@ -927,10 +938,15 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
     }
     // ======================================================== finalize
     else {
-        const uint32_t f = tid - kWarpFinal * 32;
+        // Stage s belongs to group s % FG, so that every wait of a group on a
+        // stage's barriers is for the phase after its last one.
+        const uint32_t group = (warp - kWarpFinal) / RW;
+        const uint32_t f = tid - (kWarpFinal + group * RW) * 32;
         S run = Op::zero();  // the unit's prefix from the lookback
+        uint32_t unit_seen = 0xFFFFFFFFu;
         for (uint32_t sn = 0;; ++sn) {
             const int s = static_cast<int>(sn % SS);
+            if (FG > 1 && static_cast<uint32_t>(s) % FG != group) continue;
             const uint32_t i = sn / G;
             const int k = static_cast<int>(sn % G);
             const int q = static_cast<int>(i % Q);
@@ -956,7 +972,8 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
             constexpr bool kRolled = sizeof(S) > sizeof(T);
             T v[ITEMS];
             if constexpr (!kRolled) load_row(sb, t, f, v);
-            if (k == 0) {
+            if (FG == 1 ? k == 0 : i != unit_seen) {
+                unit_seen = i;
                 // The unit's prefix (which also orders this warp after the
                 // head warp's bits), and the per-thread states (ustates).
                 bool pok = ptx::mbar_try_wait(&ctrl->uprefix[q], (i / Q) & 1u) ||
@@ -1021,7 +1038,7 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
             __syncwarp();
             if (lane == 0) {
                 ptx::mbar_arrive(&ctrl->sdone[s]);
-                if (k == G - 1) ptx::mbar_arrive(&ctrl->ufree[q]);
+                if (FG > 1 || k == G - 1) ptx::mbar_arrive(&ctrl->ufree[q]);
             }
         }
     }

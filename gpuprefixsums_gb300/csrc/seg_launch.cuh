@@ -19,15 +19,16 @@ namespace gps {
 // CTA count come from the plan's launch configuration (GenericConfig).
 constexpr int kSegWarps = 4;
 // Units in flight per CTA: each waits in L2 (64 KB, or 16 KB in single-tile
-// units) between the two passes, 152 x 6 x 64 KB at most. Measured on GB300:
-// batched scans (5 against 6; 4096 u32 segments 359 / 366 us, 2^27 u64 337 / 345, 2^24
-// compensated 39.0 / 39.4) and structs (2^24 88.7 / 94.0: the smaller control
-// block makes room for a fourth reduce-pass stage) take 5. Plain scans of 512 MB and
-// more take 5 of the 6 there is room for (2^28 u32 317 / 322, 2^27 163 / 165; 2^26
-// FP32 88.0 / 87.3, compensated 93.1 / 92.7); 4 or 3 are slower everywhere but for
-// compensated batches (2^28 u32 333 and 385).
+// units) between the two passes, 152 x 6 x 64 KB at most. A smaller queue also
+// leaves shared memory for stages. Measured on GB300: batched scans take 5 (2^27
+// u64 with 4 / 5 / 6: 321 / 313 / 316 us, 4096 u32 segments 355 / 352 / 352), compensated
+// and struct batches 4 (2^24 compensated 35.5 / 36.4 / 37.4, structs 92.8 / 99.4 / 99.9),
+// plain structs 5 (2^24 98 / 107 for 5 / 6), the rest 6 -- of which plain scans of
+// 512 MB and more use 5 (2^28 u32 317 / 322, 2^27 163 / 165; 2^26 FP32 88.0 / 87.3); 4 or 3
+// are slower there (2^28 u32 333 and 385).
 template <class Op, bool SEG>
-constexpr int kSegQueue = SEG || sizeof(typename Op::S) == 16 ? 5 : 6;
+constexpr int kSegQueue = SEG ? (sizeof(typename Op::S) > sizeof(typename Op::T) || sizeof(typename Op::S) == 16 ? 4 : 5)
+                              : (sizeof(typename Op::S) == 16 ? 5 : 6);
 constexpr uint64_t kSegDeepBytes = 512ull << 20;
 constexpr size_t kMaxSmem = 232448;
 
@@ -55,7 +56,7 @@ cudaError_t launch_seg_t(const ScanArgs& a, const SegArgs& sg, const GenericConf
     } else {
     auto kern = scan_seg_kernel<Op, St::RW, St::RS, St::SS, kSegQueue<Op, SEG>, UNIT, INCL, SEG>;
     constexpr size_t smem = seg_smem_bytes<Op, St::RW, St::RS, St::SS, kSegQueue<Op, SEG>, UNIT, SEG>();
-    constexpr int threads = SegShape<Op, St::RW>::kThreads;
+    constexpr int threads = SegShape<Op, St::RW, SEG>::kThreads;
     RowMaps maps;
     cudaError_t err = encode_row_maps(a.in, a.out, a.n, static_cast<uint32_t>(sizeof(typename Op::T)), &maps);
     if (err != cudaSuccess) return err;
