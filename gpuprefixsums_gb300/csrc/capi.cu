@@ -126,7 +126,7 @@ gps::GenericConfig generic_config(const gps_plan_s* p, bool segmented, uint64_t 
     const int c = p->tuned[segmented ? 1 : 0][size_class(n)];
     if (c >= 0 && c < gps::kNumGenericCandidates) return gps::kGenericCandidates[c];
     const uint64_t tiles = (n + p->tile_elems - 1) / p->tile_elems;
-    if (tiles <= (c == kTunedMid ? gps::kMidSegMaxTiles : gps::mid_seg_default_tiles(segmented)))
+    if (tiles <= (c == kTunedMid ? gps::kMidSegMaxTiles : gps::mid_seg_default_tiles(p->dtype)))
         return gps::kMidSegConfig;
     return gps::default_generic_config(n, p->tile_elems, p->num_sms);
 }
@@ -250,7 +250,7 @@ namespace gps {
 size_t dtype_size(gps_dtype dtype) { return dtype == GPS_DTYPE_U64 ? 8 : dtype == GPS_DTYPE_U32X4 ? 16 : 4; }
 GenericConfig default_generic_config(uint64_t n, uint32_t tile_elems, int num_sms) {
     const uint64_t units4 = (n + 4ull * tile_elems - 1) / (4ull * tile_elems);
-    return units4 >= 2ull * static_cast<uint64_t>(num_sms) ? GenericConfig{4, 1, 1} : GenericConfig{1, 1, 1};
+    return units4 >= static_cast<uint64_t>(num_sms) ? GenericConfig{4, 1, 1} : GenericConfig{1, 1, 1};
 }
 // Plain integer scans above the mid size run on the generic kernel too, in units
 // of 4 tiles: its reduce warps need no warp scan and no barrier per tile (the
@@ -314,7 +314,7 @@ gps_status gps_plan_create(gps_plan* out_plan, gps_algo algo, gps_dtype dtype, u
     // 2.7 against 4.5 us at 16384 u32). Reduce-then-scan plans keep the
     // one-CTA kernel for small inputs.
     p->small_max = algo == GPS_ALGO_CSDL ? 0 : gps::small_scan_max_elems(dtype);
-    p->mid_max = algo == GPS_ALGO_CSDL && !generic_only(dtype) ? gps::kMidMaxBytes / gps::dtype_size(dtype) : 0;
+    p->mid_max = algo == GPS_ALGO_CSDL && !generic_only(dtype) ? gps::mid_max_bytes(dtype) / gps::dtype_size(dtype) : 0;
     cudaError_t err = cudaGetDevice(&p->device);
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device);
     if (err != cudaSuccess) {

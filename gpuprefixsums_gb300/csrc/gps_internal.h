@@ -180,8 +180,10 @@ struct GenericConfig {
 constexpr GenericConfig kGenericCandidates[] = {{4, 1, 1}, {1, 1, 1}, {4, 2, 1}, {1, 2, 1},
                                                 {4, 1, 2}, {1, 1, 2}, {4, 2, 2}, {1, 2, 2}};
 constexpr int kNumGenericCandidates = 8;
-// Untuned choice: units of 4 tiles once there are at least two such units
-// per SM, else single-tile units (more CTAs busy on small inputs).
+// Untuned choice: units of 4 tiles once there is one such unit per SM, else
+// single-tile units (more CTAs busy on small inputs). Measured on GB300, 640 tiles
+// (160 units of 4): FP32 11.2 us either way, batched u32 11.7 against 13.1 with
+// single-tile units; 1024 tiles 13.5 / 13.7 and 13.5 / 16.3.
 GenericConfig default_generic_config(uint64_t n, uint32_t tile_elems, int num_sms);
 // Whether a plain u32 or u64 scan above the mid size runs on the generic kernel.
 bool integer_scan_takes_generic(uint64_t n, uint32_t tiles, int num_sms);
@@ -222,8 +224,9 @@ bool seg_u32x4_x2_fits(uint32_t unit);
 // element size, and the launch. a.carry_out receives the count (uint64).
 uint32_t select_tile_elems(size_t elem_size);
 // Selects of up to this many tiles run one tile per CTA, on the plan's
-// mid-size descriptors.
-constexpr uint32_t kMidSelectMaxTiles = 2048;
+// mid-size descriptors (2048 tiles of u32 16.9 us against 17.5 on the persistent
+// kernel, 2560 19.3 / 19.3, 3072 22.9 / 21.3).
+constexpr uint32_t kMidSelectMaxTiles = 2560;
 cudaError_t launch_select(size_t elem_size, const ScanArgs& a, const uint8_t* flags, int num_sms, cudaStream_t stream,
                           LaunchInfo* info);
 
@@ -235,9 +238,9 @@ cudaError_t launch_small(gps_dtype dtype, bool inclusive, const ScanArgs& a, cud
 // Integer chained scans up to mid size, one 16 KB tile per CTA (mid.cu); the
 // default upper size of a plan, in bytes of input. Measured on GB300 (graph
 // replay) against the persistent kernel that takes over (the generic one):
-// u32 2^22 9.7 against 13.7 us, 2^23 16.6 / 17.8, 10 x 2^20 20.4 / 20.3, 3 x 2^22 24.2 / 22.1, 2^24 31.4 /
-// 27.5; u64 2^23 32.4 / 28.1.
-constexpr size_t kMidMaxBytes = 40ull << 20;
+// u32 2^22 9.7 against 13.7 us, 2^23 16.7 / 17.9, 2300 tiles 17.9 / 19.0, 2560 20.5 /
+// 19.5, 2^24 31.4 / 26; u64 1800 tiles 16.1 / 15.9, 2048 17.6 / 16.6.
+constexpr size_t mid_max_bytes(gps_dtype dtype) { return dtype == GPS_DTYPE_U64 ? 28ull << 20 : 38ull << 20; }
 // Tile descriptors of the one-tile-per-CTA kernels sit one per 128-byte line
 // (a stride of 8 words) when a launch has more than one group of 32 tiles
 // and at most kMidStrideMaxTiles tiles, else packed. Sharing lines between
@@ -260,13 +263,23 @@ constexpr uint32_t kMidSegMaxTiles = 4096;
 static_assert(kMidSegGroup >= 32 && kMidSegMaxTiles <= kMidStrideMaxTiles, "within the plan's mid-size descriptors");
 constexpr GenericConfig kMidSegConfig = {0, 1, 1};
 // Untuned scans of up to this many tiles take it; larger ones the kernel with
-// units, whose pipeline then pays. Measured on GB300 (graph replay, us, one tile
-// per CTA against the better unit size): FP32 1024 tiles 12.4 / 15.5, 2048 tiles
-// 20.1 / 18.3; compensated 14.5 / 16.7 and 23.2 / 20.3; batched u32 12.5 / 18.2
-// and 19.9 / 20.9; batched u64 12.9 / 18.4 and 19.5 / 20.7; batched compensated
-// 16.0 / 21.0 and 25.4 / 25.4; structs 1024 tiles 16.5 / 17.3 (single-tile
-// units, the untuned choice there).
-constexpr uint64_t mid_seg_default_tiles(bool segmented) { return segmented ? 2048 : 1024; }
+// units, whose pipeline then pays. The wider the running state, the fewer CTAs
+// an SM holds and the longer each takes. Measured on GB300 (graph replay, us, one
+// tile per CTA against units of 4 tiles): FP32 1536 tiles 14.5 / 16.0, 2048 18.7 /
+// 16.9; batched u32 15.2 / 15.6 and 18.7 / 17.8; compensated 1024 tiles 13.8 / 14.4,
+// 1280 16.0 / 15.2; batched u64 13.1 / 13.5 and 14.5 / 14.3; batched compensated 15.2 /
+// 15.4 and 17.0 / 16.4; structs 640 tiles 10.8 / 11.8, 768 12.9 / 11.9, batched 11.6 /
+// 12.0 and 12.8 / 12.5.
+constexpr uint64_t mid_seg_default_tiles(gps_dtype dtype) {
+    switch (dtype) {
+        case GPS_DTYPE_U32:
+        case GPS_DTYPE_F32: return 1664;
+        case GPS_DTYPE_U64:
+        case GPS_DTYPE_F32_COMPENSATED: return 1216;
+        case GPS_DTYPE_U32X4: break;
+    }
+    return 704;
+}
 cudaError_t launch_mid(gps_dtype dtype, bool inclusive, const ScanArgs& a, int num_sms, cudaStream_t stream,
                        LaunchInfo* info);
 

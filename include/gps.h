@@ -170,9 +170,9 @@ gps_status gps_select_flagged(gps_plan plan, const void* d_in, const uint8_t* d_
  * GPS_ERR_CUDA after tuning with the others. A shape that does not fit one
  * CTA's shared memory for the element type is skipped. Up to 4096 tiles the
  * one-tile-per-CTA form of the kernel is a candidate too. Without tuning, scans
- * of up to 1024 tiles (batched: 2048) take that form; larger ones use one
- * thread per row and units of 4 tiles once there are two such units per SM,
- * else 1 tile. d_out is left holding a correct
+ * of up to 1664 tiles (u32, f32), 1216 (u64, compensated f32) or 704 (structs)
+ * take that form; larger ones use one thread per row and units of 4 tiles once
+ * there is one such unit per SM, else 1 tile. d_out is left holding a correct
  * result. Synchronizes `stream`; not allowed while the stream is being
  * captured. The chosen configuration is returned in out_unit /
  * out_ctas_div / out_threads_per_row (any may be NULL).
@@ -253,7 +253,7 @@ gps_status gps_plan_set_fallback(gps_plan plan, uint32_t fallback_polls);
 gps_status gps_plan_set_small_max(gps_plan plan, uint64_t max_n);
 
 /* Integer scans on a GPS_ALGO_CSDL plan above the one-CTA size and of at
- * most max_n elements (default: 40 MB of input) run
+ * most max_n elements (default: 38 MB of u32 or 28 MB of u64) run
  * as one 16 KB tile per CTA -- a single-pass chained scan without
  * the persistent kernels' pipeline, whose latency dominates at these sizes;
  * larger ones run on a persistent L2-buffered kernel. 0 sends them all to

@@ -1,9 +1,8 @@
 """Small and mid sizes of the batched, floating-point and struct scans (one
 tile per CTA, mid_seg.cuh) against the oracle.
 
-Sizes sit on the edges of the 16 KB tile, of the groups of 32 tiles the
-lookback folds, of the 32 groups (1024 tiles) one fold round of a lane covers,
-and of the default size limit. Integer results are bit-exact. Floating-point
+Sizes sit on the edges of the 16 KB tile, of the groups of 64 tiles the
+lookback folds, and of the default size limits. Integer results are bit-exact. Floating-point
 results are held to the bounds of the library's other scans: compensated FP32,
 relative error <= 1e-6 (rounding the exact prefix to FP32 costs 2^-24) and
 normwise <= 1e-7; plain FP32, normwise <= 1e-5; both repeat bit for bit.
@@ -37,7 +36,7 @@ def _lengths(rng, n, style):
 def test_batched_integers(cuda, dtype, style):
     tile = 16384 // np.dtype(NP[dtype]).itemsize
     sizes = [1, 3, tile - 1, tile, tile + 1, 31 * tile + 7, 32 * tile, 32 * tile + 1, 33 * tile + 5, 64 * tile,
-             100 * tile + 9, 1024 * tile, 1025 * tile - 3]
+             65 * tile, 100 * tile + 9, 1216 * tile, 1217 * tile - 3, 1665 * tile - 1]
     with Plan("csdl", dtype, max_n=max(sizes)) as plan:
         for n in sizes:
             rng = np.random.default_rng(n)
@@ -57,7 +56,7 @@ def test_batched_integers(cuda, dtype, style):
 @pytest.mark.parametrize("inclusive", [False, True])
 @pytest.mark.parametrize("dt", ["f32", "f32c"])
 def test_floating_point(cuda, dt, inclusive):
-    sizes = [1, 4095, 4097, 32 * 4096 + 1, 65 * 4096 - 2, 1024 * 4096 - 1, 1025 * 4096]
+    sizes = [1, 4095, 4097, 32 * 4096 + 1, 65 * 4096 - 2, 129 * 4096, 1216 * 4096 - 1, 1217 * 4096, 1665 * 4096 - 7]
     with Plan("csdl", dt, max_n=max(sizes)) as plan:
         for n in sizes:
             x = fp_input("mixed", n, seed=n)
@@ -94,7 +93,7 @@ def test_an_infinity_stays_inside_its_segment(cuda, dt):
 
 @pytest.mark.parametrize("inclusive", [False, True])
 def test_structs_plain_and_batched(cuda, inclusive):
-    sizes = [1, 1023, 1025, 33 * 1024 + 1, 1024 * 1024, 1025 * 1024 + 3]
+    sizes = [1, 1023, 1025, 33 * 1024 + 1, 65 * 1024, 704 * 1024, 705 * 1024 + 3]
     with Plan("csdl", "u32x4", max_n=max(sizes)) as plan:
         for n in sizes:
             rng = np.random.default_rng(n)
