@@ -191,8 +191,22 @@ __device__ __forceinline__ bool mid_seg_prefix(const ScanArgs& a, uint32_t t, ui
     return ok;
 }
 
-template <class Op, bool INCL, bool SEG>
-__global__ void __launch_bounds__(kMidSegThreads, sizeof(typename Op::S) > 8 ? 4 : 6)
+// CTAS: resident CTAs per SM the kernel is compiled for. Few leave it more
+// registers, the faster form while a launch fits one wave of them; larger
+// launches want more tiles in flight: the smallest of 4, 6 and 8 that takes the
+// launch in one wave (segmented scans at most 6, structs always 4). Measured on
+// GB300 (graph replay, us, 4 / 6 / 8 CTAs): FP32 256 tiles 5.64 / 5.80 / 6.43, 1024
+// tiles 12.1 / 11.1 / 10.5; compensated 1024 tiles 15.0 / 13.8 / 12.8; batched compensated
+// 551 tiles 9.9 / 10.9 / 11.3, 1024 tiles 15.5 / 15.2 / 15.1; batched u64 512 tiles 7.9 / 9.1 /
+// 9.4; select 800 tiles 9.1 / 7.8 / 8.7, 2048 tiles 17.3 / 16.9 / 15.8.
+inline int mid_seg_ctas(uint32_t tiles, int num_sms, int most) {
+    for (int c = 4; c < most; c += 2)
+        if (tiles <= static_cast<uint32_t>(c * num_sms)) return c;
+    return most;
+}
+
+template <class Op, bool INCL, bool SEG, int CTAS>
+__global__ void __launch_bounds__(kMidSegThreads, CTAS)
     mid_seg_kernel(const ScanArgs a, const SegArgs sg) {
     using T = typename Op::T;
     using S = typename Op::S;
@@ -377,7 +391,7 @@ __global__ void __launch_bounds__(kMidSegThreads, sizeof(typename Op::S) > 8 ? 4
 }
 
 template <class Op>
-cudaError_t launch_mid_seg(bool inclusive, const ScanArgs& a0, const SegArgs* sg, cudaStream_t stream,
+cudaError_t launch_mid_seg(bool inclusive, const ScanArgs& a0, const SegArgs* sg, int num_sms, cudaStream_t stream,
                            LaunchInfo* info) {
     if (((reinterpret_cast<uintptr_t>(a0.desc) | reinterpret_cast<uintptr_t>(a0.group_desc)) & 15u) != 0 ||
         a0.desc == nullptr || a0.group_desc == nullptr || a0.num_tiles > kMidSegMaxTiles)
@@ -392,9 +406,24 @@ cudaError_t launch_mid_seg(bool inclusive, const ScanArgs& a0, const SegArgs* sg
     auto launch = [&](void (*kern)(ScanArgs, SegArgs), const SegArgs& s) {
         return launch_dependent(kern, grid, kMidSegThreads, 0, stream, a, s);
     };
-    if (sg != nullptr)
-        return inclusive ? launch(mid_seg_kernel<Op, true, true>, *sg) : launch(mid_seg_kernel<Op, false, true>, *sg);
-    return inclusive ? launch(mid_seg_kernel<Op, true, false>, none) : launch(mid_seg_kernel<Op, false, false>, none);
+    constexpr int kMost = sizeof(typename Op::S) > 8 ? 4 : 8;
+    constexpr int k6 = kMost < 6 ? kMost : 6;
+    const int ctas = mid_seg_ctas(a.num_tiles, num_sms, sg != nullptr ? k6 : kMost);
+    if (sg != nullptr) {
+        if (ctas == 4)
+            return inclusive ? launch(mid_seg_kernel<Op, true, true, 4>, *sg)
+                             : launch(mid_seg_kernel<Op, false, true, 4>, *sg);
+        return inclusive ? launch(mid_seg_kernel<Op, true, true, k6>, *sg)
+                         : launch(mid_seg_kernel<Op, false, true, k6>, *sg);
+    }
+    if (ctas == 4)
+        return inclusive ? launch(mid_seg_kernel<Op, true, false, 4>, none)
+                         : launch(mid_seg_kernel<Op, false, false, 4>, none);
+    if (ctas == 6)
+        return inclusive ? launch(mid_seg_kernel<Op, true, false, k6>, none)
+                         : launch(mid_seg_kernel<Op, false, false, k6>, none);
+    return inclusive ? launch(mid_seg_kernel<Op, true, false, kMost>, none)
+                     : launch(mid_seg_kernel<Op, false, false, kMost>, none);
 }
 
 }  // namespace gps

@@ -92,7 +92,7 @@ cudaError_t launch_seg_op(bool inclusive, const ScanArgs& a, const SegArgs* sg, 
                           cudaStream_t stream, LaunchInfo* info) {
     if (cfg.split != static_cast<uint32_t>(SPLIT)) return cudaErrorInvalidValue;
     if constexpr (SPLIT == 1) {
-        if (cfg.unit == 0) return launch_mid_seg<Op>(inclusive, a, sg, stream, info);
+        if (cfg.unit == 0) return launch_mid_seg<Op>(inclusive, a, sg, num_sms, stream, info);
     }
     switch (cfg.unit) {
         case 1: return launch_seg_unit<Op, 1, SPLIT>(inclusive, a, sg, cfg, num_sms, stream, info);

@@ -537,8 +537,8 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
 // 19.0 (90% selected: 21.0 / 24.0), 2^24 32.3 / 28.4.
 constexpr int kMidSelThreads = kMidSegThreads;
 
-template <typename V>
-__global__ void __launch_bounds__(kMidSelThreads, 6) mid_select_kernel(const ScanArgs a, const SelArgs sa) {
+template <typename V, int CTAS>
+__global__ void __launch_bounds__(kMidSelThreads, CTAS) mid_select_kernel(const ScanArgs a, const SelArgs sa) {
     constexpr int TILE = 16384 / static_cast<int>(sizeof(V));
     constexpr int EPC = 16 / static_cast<int>(sizeof(V));
     constexpr int ITEMS = TILE / kMidSelThreads;
@@ -637,12 +637,17 @@ __global__ void __launch_bounds__(kMidSelThreads, 6) mid_select_kernel(const Sca
 }
 
 template <typename V>
-cudaError_t launch_mid_select(const ScanArgs& a0, const SelArgs& sa, cudaStream_t stream, LaunchInfo* info) {
+cudaError_t launch_mid_select(const ScanArgs& a0, const SelArgs& sa, int num_sms, cudaStream_t stream,
+                              LaunchInfo* info) {
     ScanArgs a = a0;
     a.desc_stride = a.num_tiles > 32 ? kMidDescStride : 1u;
     const int grid = static_cast<int>(a.num_tiles);
     if (info) *info = LaunchInfo{grid, kMidSelThreads, 0};
-    return launch_dependent(mid_select_kernel<V>, grid, kMidSelThreads, 0, stream, a, sa);
+    switch (mid_seg_ctas(a.num_tiles, num_sms, 8)) {
+        case 4: return launch_dependent(mid_select_kernel<V, 4>, grid, kMidSelThreads, 0, stream, a, sa);
+        case 6: return launch_dependent(mid_select_kernel<V, 6>, grid, kMidSelThreads, 0, stream, a, sa);
+    }
+    return launch_dependent(mid_select_kernel<V, 8>, grid, kMidSelThreads, 0, stream, a, sa);
 }
 
 template <typename V>
@@ -668,8 +673,8 @@ cudaError_t launch_select(size_t elem_size, const ScanArgs& a, const uint8_t* fl
                           LaunchInfo* info) {
     const SelArgs sa{flags};
     if (a.num_tiles <= kMidSelectMaxTiles)
-        return elem_size == 8 ? launch_mid_select<uint64_t>(a, sa, stream, info)
-                              : launch_mid_select<uint32_t>(a, sa, stream, info);
+        return elem_size == 8 ? launch_mid_select<uint64_t>(a, sa, num_sms, stream, info)
+                              : launch_mid_select<uint32_t>(a, sa, num_sms, stream, info);
     return elem_size == 8 ? launch_select_t<uint64_t>(a, sa, num_sms, stream, info)
                           : launch_select_t<uint32_t>(a, sa, num_sms, stream, info);
 }
