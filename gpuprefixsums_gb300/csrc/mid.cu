@@ -33,10 +33,9 @@ namespace gps {
 namespace {
 
 constexpr int kMidThreads = kRowThreads;
-// Resident CTAs per SM the kernel is compiled for: 40 registers a thread with
-// the tile held in registers, 32 without.
-template <bool HELD>
-constexpr int kMidCtasPerSm = HELD ? 6 : 8;
+// Resident CTAs per SM of the form that does not hold its tile in registers
+// (32 registers a thread).
+constexpr int kMidCtasPerSm = 8;
 
 // ------------------------------------------------------------ descriptors
 // One 16-byte word per tile: {lo: the value (u32 or u64), hi: status:2 |
@@ -214,13 +213,14 @@ __device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint
 // w at r * 8 + w), and one warp scan of those 32 totals gives every (row,
 // warp) its offset -- one barrier for the whole block scan; the chunk offsets
 // wait in shared memory during the lookback. HELD keeps the tile in registers
-// across the lookback: 40 registers, six CTAs per SM. Otherwise its chunks are
+// across the lookback, and is the CTAs per SM it is compiled for: four (64
+// registers) or six (40). With 0 its chunks are
 // read again after it (from L1 or L2): 32 registers, eight CTAs per SM, so that
 // up to 1216 tiles (2^22 u32 elements fit on 152 SMs) run in one wave. Which is
 // faster turns on the number of waves: up to one wave of the HELD form it is
 // ahead (graph replay, u32: 1000 elements 1.43 against 1.62 us, 2^16 2.74 / 2.91,
 // 2^20 5.67 / 5.92, 2^21 7.1 / 7.4), beyond it the other (2^22 11.0 / 9.7, 2^23
-// 17.8 / 16.7). There is no shared-memory staging and no mbarrier to set up, so
+// 17.8 / 16.7; with four CTAs instead of six, 500 tiles 6.7 / 7.1). There is no shared-memory staging and no mbarrier to set up, so
 // every CTA issues its loads as soon as it starts.
 //
 // ALIGNED = false takes buffers at any element offset from a 16-byte boundary
@@ -230,8 +230,8 @@ __device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint
 // 10,000,019 u32 from a view one element past a boundary, into an aligned
 // output: 21.3 us a call, where per-thread element loads and stores (64
 // bytes apart across a warp) took 70.9.
-template <typename T, bool INCL, bool ALIGNED, bool HELD>
-__global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm<HELD>) mid_vec_kernel(const ScanArgs a) {
+template <typename T, bool INCL, bool ALIGNED, int HELD>
+__global__ void __launch_bounds__(kMidThreads, HELD ? HELD : kMidCtasPerSm) mid_vec_kernel(const ScanArgs a) {
     using Rows = TileRows<T, ALIGNED>;
     constexpr int EPC = Rows::kEpc;
     constexpr int ROWS = Rows::kRows;
@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm<HELD>) mid_vec_kern
         Chunk<T> q[ROWS];
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) q[r] = rows.load(r, access);
-        if constexpr (HELD) {
+        if constexpr (HELD != 0) {
 #pragma unroll
             for (int r = 0; r < ROWS; ++r) held[r] = q[r];
         }
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(kMidThreads, kMidCtasPerSm<HELD>) mid_vec_kern
             }
         }
     };
-    if constexpr (HELD) {
+    if constexpr (HELD != 0) {
 #pragma unroll
         for (int r = 0; r < ROWS; ++r) {
             scan_chunk(r, held[r]);
@@ -344,10 +344,12 @@ cudaError_t launch_mid_v(const ScanArgs& a0, int num_sms, cudaStream_t stream, L
     // program that scans one small array after another waits for one launch
     // less each time (2^20 u32: 6.3 -> 5.5 us a call, 32 captured scans of 2^16:
     // 102 -> 89 us).
-    // The form that holds its tile, while the launch is one wave of it.
-    return a.num_tiles <= static_cast<uint32_t>(kMidCtasPerSm<true> * num_sms)
-               ? launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, true>, grid, kMidThreads, 0, stream, a)
-               : launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, false>, grid, kMidThreads, 0, stream, a);
+    // The forms that hold their tile, while the launch is one wave of them.
+    if (a.num_tiles <= static_cast<uint32_t>(4 * num_sms))
+        return launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, 4>, grid, kMidThreads, 0, stream, a);
+    if (a.num_tiles <= static_cast<uint32_t>(6 * num_sms))
+        return launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, 6>, grid, kMidThreads, 0, stream, a);
+    return launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, 0>, grid, kMidThreads, 0, stream, a);
 }
 
 template <typename T, bool INCL>
