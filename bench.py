@@ -52,7 +52,7 @@ import tempfile
 import time
 
 ROOT = os.path.dirname(os.path.abspath(__file__))
-PROFILE_TRAFFIC = os.path.join(ROOT, "profiles", "scan_l2_kernel_u32_exclusive_2pow28.md")
+PROFILE_TRAFFIC = os.path.join(ROOT, "profiles", "scan_seg_kernel_u32_exclusive_2pow28.md")
 METRIC = "scan GB/s (u32 exclusive, n=2^28, chained scan), % of D2D-copy roofline"
 
 
@@ -451,8 +451,8 @@ def run_sweep(stream, d_in, d_out):
     second power of two) on the benchmark's buffers, beside CUB DeviceScan on
     the same buffers, and u64 at n = 2^27. GPU time per scan from CUDA-graph
     replay. Inputs below about 2^24 elements stay in L2 between launches.
-    The plan's defaults pick the kernel: one tile per CTA up to 64 MB, the
-    persistent L2-buffered kernel above."""
+    The plan's defaults pick the kernel: one tile per CTA up to 38 MB (28 MB
+    of u64), the persistent generic kernel above."""
     import torch
 
     from gpuprefixsums_gb300 import Plan

@@ -5,6 +5,11 @@
 // (ChainedScanDecoupledLookbackDispatcher.cuh:177-195). The reference clears
 // its descriptors and bump counter with two cudaMemsets per call; here the
 // kernel leaves its workspace ready for the next launch itself.
+//
+// These two kernels take what the one-tile-per-CTA kernels (mid.cu) and the
+// generic one (seg_*.cu) leave: forced stalls and the fallback, carries from
+// chunk to chunk, fewer than two units per SM when a plan lowers its mid-size
+// limit, more than 2^34 elements, and the allocation-free entry point.
 #include "launch_util.h"
 #include "scan_l2.cuh"
 #include "scan_pipeline.cuh"

@@ -81,7 +81,8 @@ cudaError_t resident_ctas_per_sm(Kernel kern, int threads, size_t smem, int* out
 
 // Launches `kern` so that its CTAs may be set up before the kernel ahead of it
 // in the stream has finished; every such kernel calls ptx::grid_dep_wait()
-// before it touches global memory.
+// before it touches global memory that the kernels ahead may write or read (the
+// launches of one reduce-then-scan overlap more, see rts.cu).
 template <typename... Params, typename... Args>
 cudaError_t launch_dependent(void (*kern)(Params...), int grid, int block, size_t smem, cudaStream_t stream,
                              Args... args) {

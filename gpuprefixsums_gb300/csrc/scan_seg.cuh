@@ -7,18 +7,19 @@
 // element carries a "segment head" bit; states combine with the segmented
 // operator
 //     (a, fa) . (b, fb) = (fb ? b : a + b, fa | fb),
-// which is associative, so the same decoupled lookback works: a unit whose
-// tiles contain a head publishes the sum since its last head together with a
-// head flag, and such a descriptor ends a lookback walk just like an
-// inclusive prefix. Short segments therefore resolve inside their unit, long
-// ones walk back to the unit where they start. The reference has no batched
+// which is associative, so the same lookback works: a unit whose tiles contain
+// a head publishes the sum since its last head together with a head flag, and
+// nothing before such a unit counts for the units after it. Short segments
+// therefore resolve inside their group of units, long ones take the chain of
+// group prefixes. The reference has no batched
 // or floating-point scan; this kernel covers those rows of the design
 // (dtype per launch: u32, u64, plain FP32, compensated FP32, and structs of
 // four u32 members).
 //
 // Warps: 0 R-loader, 1 S-loader, 2 storer, 3 head warp (segment heads of each
 // unit, from the offsets), then LW lookback warps, the aggregator warp, RW
-// reduce warps and RW finalize warps; see scan_l2.cuh for the two passes.
+// reduce warps and one or two groups of RW finalize warps (kFinalGroups); see
+// scan_l2.cuh for the two passes.
 // Unlike scan_l2.cuh, the reduce warps only aggregate their rows: once per
 // unit the aggregator warp scans those aggregates, publishes the unit's
 // aggregate and hands every finalize thread its state within the unit, so
