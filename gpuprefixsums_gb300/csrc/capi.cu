@@ -134,12 +134,14 @@ gps::GenericConfig generic_config(const gps_plan_s* p, bool segmented, uint64_t 
 // Generic kernel (scan_seg.cuh, mid_seg.cuh): floating-point scans and batched
 // scans. The launch's descriptors are the plan's for the configuration.
 cudaError_t launch_generic(const gps_plan_s* p, bool inclusive, gps::ScanArgs a, const gps::SegArgs* sg,
-                           const gps::GenericConfig& cfg, cudaStream_t stream, gps::LaunchInfo* info) {
+                           const gps::GenericConfig& cfg, cudaStream_t stream, gps::LaunchInfo* info,
+                           bool unaligned = false) {
     const int num_sms = p->num_sms;
     a.hdr = p->hdr16;
     a.mid_launch = &p->hdr->mid_launch;
     a.desc = cfg.unit == 0 ? p->desc_mid : p->desc16;
     a.group_desc = cfg.unit == 0 ? p->group_desc_mid : p->group_desc16;
+    if (unaligned) return gps::launch_seg_view(p->dtype, inclusive, a, num_sms, stream, info);
     switch (p->dtype) {
         case GPS_DTYPE_U32: return gps::launch_seg_u32(inclusive, a, sg, cfg, num_sms, stream, info);
         case GPS_DTYPE_U64: return gps::launch_seg_u64(inclusive, a, sg, cfg, num_sms, stream, info);
@@ -189,24 +191,26 @@ gps_status launch_scan(gps_plan_s* p, bool inclusive, const void* in, void* out,
     a.wait_budget_ns = p->wait_budget_ns;
     a.stall = p->stall;
     a.mid_launch = &p->hdr->mid_launch;
-    // The persistent kernel for buffers off a 16-byte boundary moves single
-    // elements; one tile per CTA is faster at every size (2^27 u32 elements:
-    // 258 against 2017 us).
+    // Buffers off a 16-byte boundary take the same kernels as others, but where the
+    // generic one does not apply: csdl.cu's for them moves single elements, so one tile per
+    // CTA takes every size that is left (2^27 u32 elements: 258 against 2017 us;
+    // generic kernel 160). One limit serves both: at 9.5 M u32 off a boundary one tile
+    // per CTA takes 19.5 us and the generic kernel 19.1, at 2.5 M u64 13.4 and 14.0.
     const bool unaligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) != 0;
     cudaError_t err;
     if (generic_only(p->dtype)) {
         err = launch_generic(p, inclusive, a, nullptr, generic_config(p, false, n), stream, &p->last_launch);
     } else if (n <= p->small_max && p->stall.mode == 0 && p->stall.fallback_polls == 0) {
         err = gps::launch_small(p->dtype, inclusive, a, stream, &p->last_launch);
+    } else if (p->algo == GPS_ALGO_CSDL && p->stall.mode == 0 && p->stall.fallback_polls == 0 && n > p->mid_max &&
+               carry_in == nullptr && carry_out == nullptr &&
+               gps::integer_scan_takes_generic(n, a.num_tiles, p->num_sms)) {
+        err = launch_generic(p, inclusive, a, nullptr, gps::kGenericCandidates[0], stream, &p->last_launch, unaligned);
     } else if (p->algo == GPS_ALGO_CSDL && (n <= p->mid_max || (unaligned && p->mid_max != 0)) &&
                p->stall.mode == 0 && p->stall.fallback_polls == 0) {
         a.desc = p->desc_mid;
         a.group_desc = p->group_desc_mid;
         err = gps::launch_mid(p->dtype, inclusive, a, p->num_sms, stream, &p->last_launch);
-    } else if (p->algo == GPS_ALGO_CSDL && !unaligned && p->stall.mode == 0 && p->stall.fallback_polls == 0 &&
-               carry_in == nullptr && carry_out == nullptr &&
-               gps::integer_scan_takes_generic(n, a.num_tiles, p->num_sms)) {
-        err = launch_generic(p, inclusive, a, nullptr, gps::kGenericCandidates[0], stream, &p->last_launch);
     } else if (p->algo == GPS_ALGO_CSDL) {
         err = gps::launch_csdl(p->dtype, inclusive, p->stall.mode != 0 || p->stall.fallback_polls != 0, a, p->num_sms,
                                stream, &p->last_launch);

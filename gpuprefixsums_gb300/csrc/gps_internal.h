@@ -115,6 +115,10 @@ struct ScanArgs {
     StallConfig stall;
     uint64_t* mid_launch;  // one-tile-per-CTA kernels: WsHeader::mid_launch
     uint32_t units_in_flight;  // generic kernel: per CTA, set by its launcher
+    // Generic kernel on buffers off a 16-byte boundary (its launcher sets them):
+    // elements before the input in its first 16 bytes, and how many elements
+    // further the outputs sit from their boundary.
+    uint32_t view_lead, view_shift;
 };
 
 // Kernel geometry shared by host and device: RW reduce warps and RW finalize
@@ -164,7 +168,8 @@ struct RowMaps {
     CUtensorMap in;
     CUtensorMap out;
 };
-cudaError_t encode_row_maps(const void* in, void* out, uint64_t n, uint32_t elem_size, RowMaps* maps);
+// (of n elements of input and out_n of output).
+cudaError_t encode_row_maps(const void* in, void* out, uint64_t n, uint64_t out_n, uint32_t elem_size, RowMaps* maps);
 
 // Launch configuration of the generic kernel: tiles per lookback unit (1 or
 // 4; the unit is what one CTA takes from the work counter), the CTA count as
@@ -200,6 +205,10 @@ cudaError_t launch_seg_f32c(bool inclusive, const ScanArgs& a, const SegArgs* sg
                             int num_sms, cudaStream_t stream, LaunchInfo* info);
 cudaError_t launch_seg_u32x4(bool inclusive, const ScanArgs& a, const SegArgs* sg, const GenericConfig& cfg,
                              int num_sms, cudaStream_t stream, LaunchInfo* info);
+// Plain u32 and u64 scans of buffers off a 16-byte boundary, in units of 4 tiles
+// (seg_view.cu).
+cudaError_t launch_seg_view(gps_dtype dtype, bool inclusive, const ScanArgs& a, int num_sms, cudaStream_t stream,
+                            LaunchInfo* info);
 // The same with two threads per row (cfg.split == 2), in translation units of
 // their own (seg_*_x2.cu); cudaErrorNotSupported when that kernel shape does
 // not fit one CTA's shared memory for the type.

@@ -296,8 +296,18 @@ __device__ typename Op::C seg_lookback(const ScanArgs& a, uint32_t u, uint32_t e
     return Op::chain_add(gp, c);
 }
 
-template <class Op, int RW, int RS, int SS, int Q, int G, bool SEG>
-struct SegCtrl {
+// Views only: the last chunk of every warp's rows (from the reduce pass) and of
+// the tile before each unit.
+template <typename T, int RW, int Q, int G, bool VIEW>
+struct SegEdges {};
+template <typename T, int RW, int Q, int G>
+struct SegEdges<T, RW, Q, G, true> {
+    Chunk<T> edge[Q][G][RW];
+    Chunk<T> uedge[Q];
+};
+
+template <class Op, int RW, int RS, int SS, int Q, int G, bool SEG, bool VIEW = false>
+struct SegCtrl : SegEdges<typename Op::T, RW, Q, G, VIEW> {
     using S = typename Op::S;
     using C = typename Op::C;
     static constexpr int kHeadWords = 16384 / static_cast<int>(sizeof(typename Op::T)) / 32;
@@ -328,13 +338,13 @@ struct SegCtrl {
     uint32_t sample[SEG ? 1024 : 1];             // offsets[j * sample_stride], to start head searches
 };
 
-template <class Op, int RW, int RS, int SS, int Q, int G, bool SEG>
+template <class Op, int RW, int RS, int SS, int Q, int G, bool SEG, bool VIEW = false>
 constexpr size_t seg_smem_bytes() {
     return static_cast<size_t>(RS + SS) * 16384 +
-           sizeof(SegCtrl<Op, RW, RS, SS, Q, G, SEG>);
+           sizeof(SegCtrl<Op, RW, RS, SS, Q, G, SEG, VIEW>);
 }
 
-template <class Op, int RW, bool SEG>
+template <class Op, int RW, bool SEG, bool VIEW = false>
 struct SegShape {
     static constexpr int kLookbackWarps = 3;
     // Groups of RW finalize warps, each with stages of its own: two for segmented
@@ -342,16 +352,29 @@ struct SegShape {
     // per scheduler, each waiting on its own chain. Measured on GB300, one group
     // against two: compensated FP32 2^26 91.7 / 85.9 us, in 500 segments 117 / 108, in
     // 20,000 151 / 131; batched 2^28 u32 317 / 310, 2^26 u64 174 / 162, 2^24 structs
-    // 103 / 99; plain 2^24 u64 48.7 / 46.3, but 2^28 u32 318.1 / 319.5 (three groups:
-    // compensated batches 117 / 143).
-    static constexpr int kFinalGroups = RW == 4 && (SEG || sizeof(typename Op::S) == 8) ? 2 : 1;
+    // 103 / 99; plain 2^24 u64 48.7 / 46.3, u32 off a boundary 2^27 176 / 160, but aligned
+    // 2^28 u32 318.1 / 319.5 (three groups: compensated batches 117 / 143).
+    static constexpr int kFinalGroups = RW == 4 && (SEG || VIEW || sizeof(typename Op::S) == 8) ? 2 : 1;
     // R-loader, S-loader, storer, head warp, lookback warps, aggregator,
     // reduce warps, finalize warps.
     static constexpr int kThreads = 32 * (5 + kLookbackWarps + (1 + kFinalGroups) * RW);
 };
 
-template <class Op, int RW, int RS, int SS, int Q, int G, bool INCL, bool SEG>
-__global__ void __launch_bounds__(SegShape<Op, RW, SEG>::kThreads, 1)
+// VIEW: integer scans of buffers off a 16-byte boundary. The arguments describe
+// the input from the boundary at or below it (a.in; a.n counts its a.view_lead
+// elements before the input too, which are taken as zeros), so that it moves in
+// the same TMA boxes. Virtual element j's result goes to a.out[j + a.view_shift],
+// a.out on a boundary too: each finalize thread moves its row of results up by
+// view_shift (0 to 3) elements, and the first ones are results of the elements
+// before its row, which follow from its prefix and those elements (an integer sum
+// can be taken back). Those come from the lane below, from the reduce pass where a
+// warp's rows begin and, once per unit, from memory. Tile 0, whose
+// first row lies partly before the output, is stored by plain stores.
+// HBM bounds it as it does aligned scans. Measured on GB300, graph replay, one tile per
+// CTA (mid.cu) against this: u32 2^24 33 / 27-30 us, 2^25 70.6 / 47, 2^27 258 / 160 (aligned
+// 26, 46, 162); u64 2^24 73 / 48. With one finalize group, u32 2^25 53, 2^27 176.
+template <class Op, int RW, int RS, int SS, int Q, int G, bool INCL, bool SEG, bool VIEW = false>
+__global__ void __launch_bounds__(SegShape<Op, RW, SEG, VIEW>::kThreads, 1)
     scan_seg_kernel(const ScanArgs a, const SegArgs sg, const __grid_constant__ CUtensorMap tin,
                     const __grid_constant__ CUtensorMap tout) {
     using T = typename Op::T;
@@ -367,16 +390,17 @@ __global__ void __launch_bounds__(SegShape<Op, RW, SEG>::kThreads, 1)
     constexpr int CHUNKS = ITEMS / EPC;
     constexpr uint32_t NROLE = RW * 32;
     constexpr uint32_t ROWS = 128;  // rows per tile
-    constexpr uint32_t LW = SegShape<Op, RW, SEG>::kLookbackWarps;
+    constexpr uint32_t LW = SegShape<Op, RW, SEG, VIEW>::kLookbackWarps;
     constexpr uint32_t kWarpLookback = 4, kWarpAgg = 4 + LW, kWarpReduce = 5 + LW, kWarpFinal = 5 + LW + RW;
-    constexpr uint32_t FG = SegShape<Op, RW, SEG>::kFinalGroups;
+    constexpr uint32_t FG = SegShape<Op, RW, SEG, VIEW>::kFinalGroups;
     constexpr uint32_t kLaneEntries = G * RW;  // aggregator entries per lane
     auto entry_at = [](uint32_t j) -> uint32_t { return j + j / kLaneEntries; };
     constexpr int kHeadWords = TILE / 32;
     static_assert((SPLIT == 1 || SPLIT == 2) && RW % 4 == 0, "4 or 8 warps per role");
     static_assert(NROLE / SPLIT == ROWS, "a tile is one box of 128 rows of 128 bytes");
     static_assert(Q > LW, "every lookback warp needs its own queue entry");
-    using Ctrl = SegCtrl<Op, RW, RS, SS, Q, G, SEG>;
+    static_assert(!VIEW || (SPLIT == 1 && !SEG && sizeof(S) == sizeof(T)), "views: plain integer scans");
+    using Ctrl = SegCtrl<Op, RW, RS, SS, Q, G, SEG, VIEW>;
 
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     T* rbuf = reinterpret_cast<T*>(smem_raw);
@@ -399,6 +423,10 @@ __global__ void __launch_bounds__(SegShape<Op, RW, SEG>::kThreads, 1)
     constexpr uint32_t ROW = 128 / sizeof(T);
     const uint64_t rows_full = a.n / ROW;
     const uint32_t tail = static_cast<uint32_t>(a.n % ROW);
+    // Output elements [out_first, out_n) and full rows of the output.
+    const uint64_t out_n = VIEW ? a.n + a.view_shift : a.n;
+    const uint64_t out_first = VIEW ? a.view_lead + a.view_shift : 0u;
+    const uint64_t out_rows = VIEW ? out_n / ROW : rows_full;
     // Samples of the offsets: every `stride`-th entry, at most 1024.
     const uint32_t nseg = SEG ? sg.num_segments : 0u;
     const uint32_t stride = SEG ? (nseg + 1 + 1023) / 1024 : 1u;
@@ -468,6 +496,11 @@ __global__ void __launch_bounds__(SegShape<Op, RW, SEG>::kThreads, 1)
 #pragma unroll
                 for (int e = 0; e < EPC; ++e) v[c * EPC + e] = qv.v[e];
             }
+            if (VIEW && row == 0) {
+#pragma unroll
+                for (int e = 0; e < EPC - 1; ++e)
+                    if (static_cast<uint32_t>(e) < a.view_lead) v[e] = T{};
+            }
         } else {
             const T* gp = static_cast<const T*>(a.in) + row * ROW + sub * ITEMS;
 #pragma unroll
@@ -493,6 +526,38 @@ __global__ void __launch_bounds__(SegShape<Op, RW, SEG>::kThreads, 1)
 #pragma unroll
             for (int e = 0; e < ITEMS; ++e)
                 if (sub * ITEMS + static_cast<uint32_t>(e) < tail) gp[e] = v[e];
+        }
+    };
+    // The same by output rows: into the stage, or to memory in tile 0 and in the
+    // last, partial row.
+    auto store_view_row = [&](T* stage, uint32_t t, uint32_t thr, const T (&v)[ITEMS]) {
+        const uint64_t row = static_cast<uint64_t>(t) * ROWS + thr;
+        if (row > out_rows) return;
+        const bool staged = t != 0 && row < out_rows;
+        if (staged) {
+#pragma unroll
+            for (int c = 0; c < CHUNKS; ++c) {
+                Chunk<T> qv;
+#pragma unroll
+                for (int e = 0; e < EPC; ++e) qv.v[e] = v[c * EPC + e];
+                *reinterpret_cast<Chunk<T>*>(stage + thr * ROW + (c ^ static_cast<int>(thr & 7u)) * EPC) = qv;
+            }
+            return;
+        }
+        T* gp = static_cast<T*>(a.out) + row * ROW;
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) {
+            Chunk<T> qv;
+#pragma unroll
+            for (int e = 0; e < EPC; ++e) qv.v[e] = v[c * EPC + e];
+            const uint64_t p = row * ROW + c * EPC;
+            if (p >= out_first && p + EPC <= out_n) {
+                *reinterpret_cast<Chunk<T>*>(gp + c * EPC) = qv;
+            } else {
+#pragma unroll
+                for (int e = 0; e < EPC; ++e)
+                    if (p + e >= out_first && p + e < out_n) gp[c * EPC + e] = qv.v[e];
+            }
         }
     };
     auto wait1 = [&](uint64_t* bar, uint32_t ph, uint64_t b) -> bool {
@@ -651,7 +716,7 @@ __global__ void __launch_bounds__(SegShape<Op, RW, SEG>::kThreads, 1)
                 const uint32_t t = ctrl->s_tile[s];
                 if (t == kTileEnd) break;
                 // Rows past the tensor are clipped by the TMA unit.
-                if (tma_bytes_of(t))
+                if (VIEW ? t != 0 && static_cast<uint64_t>(t) * ROWS < out_rows : tma_bytes_of(t) != 0)
                     ptx::tma_store_2d(&tout, 0, static_cast<int32_t>(t * ROWS), sbuf + static_cast<size_t>(s) * TILE,
                                       pol);
                 ptx::bulk_commit();
@@ -781,6 +846,19 @@ __global__ void __launch_bounds__(SegShape<Op, RW, SEG>::kThreads, 1)
             // 118.4 us for 2^26 elements; the other types lose up to 1% that way).
             constexpr bool kLate = SEG && sizeof(S) > sizeof(T);
             C pre = Op::chain_zero();
+            if constexpr (VIEW) {
+                // (An in-place scan has no shift, and may already have written there.)
+                if (lane == 0 && a.view_shift != 0) {
+                    Chunk<T> x{};
+                    const uint64_t end = static_cast<uint64_t>(u) * G * TILE;
+#pragma unroll
+                    for (int e = 1; e < EPC; ++e) {
+                        const uint64_t j = end - EPC + e;
+                        if (u != 0 && j < a.n) x.v[e] = static_cast<const T*>(a.in)[j];
+                    }
+                    ctrl->uedge[q] = x;
+                }
+            }
             if (!kLate && u != 0) pre = seg_lookback<Op, SEG, det_group_units(G, Op::kLongGroups)>(a, u, epoch, lane);
             uint32_t state = 0;
             if (lane == 0) {
@@ -925,6 +1003,14 @@ __global__ void __launch_bounds__(SegShape<Op, RW, SEG>::kThreads, 1)
             const uint32_t hb = SEG ? head_bits(heads_of(q, k), r) : 0u;
             const S agg = (SEG && __any_sync(kFullMask, hb != 0u)) ? thread_aggregate<Op, ITEMS, true>(v, hb)
                                                                    : thread_aggregate<Op, ITEMS, false>(v, 0u);
+            if constexpr (VIEW) {
+                if (lane == 31) {
+                    Chunk<T> x;
+#pragma unroll
+                    for (int e = 0; e < EPC; ++e) x.v[e] = v[ITEMS - EPC + e];
+                    ctrl->edge[q][k][rw] = x;
+                }
+            }
             // Every value of the warp's rows is in registers now.
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&ctrl->rfree[s]);
@@ -1028,6 +1114,36 @@ __global__ void __launch_bounds__(SegShape<Op, RW, SEG>::kThreads, 1)
                         go[e] = INCL ? Op::out(st) : Op::out(before);
                     }
                 }
+            } else if constexpr (VIEW) {
+                // before[m]: the element m + 1 before the row.
+                T before[EPC - 1], last[EPC];
+                const uint32_t fw = f >> 5;
+                const Chunk<T>* edge = fw != 0 ? &ctrl->edge[q][k][fw - 1]
+                                               : k != 0 ? &ctrl->edge[q][k - 1][RW - 1] : &ctrl->uedge[q];
+#pragma unroll
+                for (int m = 0; m < EPC - 1; ++m) {
+                    before[m] = Op::shfl_up(v[ITEMS - 1 - m], 1);
+                    if (lane == 0) before[m] = edge->v[EPC - 1 - m];
+                }
+                // last[EPC - 1 - m]: that element's result.
+                last[0] = T{};
+                T o = INCL ? base : base - before[0];
+                last[EPC - 1] = o;
+#pragma unroll
+                for (int m = 1; m < EPC - 1; ++m) {
+                    o -= before[INCL ? m - 1 : m];
+                    last[EPC - 1 - m] = o;
+                }
+                thread_outputs<Op, ITEMS, false, INCL>(v, base, 0u);
+                auto shift = [&](auto by) {
+                    constexpr int P = decltype(by)::value;
+#pragma unroll
+                    for (int e = ITEMS - 1; e >= 0; --e) v[e] = e >= P ? v[e >= P ? e - P : 0] : last[e < P ? EPC - P + e : 0];
+                };
+                if (a.view_shift == 1) shift(std::integral_constant<int, 1>{});
+                if (EPC > 2 && a.view_shift == 2) shift(std::integral_constant<int, (EPC > 2 ? 2 : 1)>{});
+                if (EPC > 2 && a.view_shift == 3) shift(std::integral_constant<int, (EPC > 2 ? 3 : 1)>{});
+                store_view_row(sb, t, f, v);
             } else {
                 if (SEG && __any_sync(kFullMask, hb != 0u))
                     thread_outputs<Op, ITEMS, true, INCL>(v, base, hb);

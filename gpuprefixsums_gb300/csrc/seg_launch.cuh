@@ -32,33 +32,34 @@ constexpr int kSegQueue = SEG ? (sizeof(typename Op::S) > sizeof(typename Op::T)
 constexpr uint64_t kSegDeepBytes = 512ull << 20;
 constexpr size_t kMaxSmem = 232448;
 
-template <class Op, int G, bool SEG, int SPLIT>
+template <class Op, int G, bool SEG, int SPLIT, bool VIEW = false>
 struct SegStages {
     static constexpr int RW = kSegWarps * SPLIT;  // warps per role
-    static constexpr bool k13 = seg_smem_bytes<Op, RW, 4, 9, kSegQueue<Op, SEG>, G, SEG>() <= kMaxSmem;
-    static constexpr bool k12 = seg_smem_bytes<Op, RW, 4, 8, kSegQueue<Op, SEG>, G, SEG>() <= kMaxSmem;
-    static constexpr bool k11 = seg_smem_bytes<Op, RW, 3, 8, kSegQueue<Op, SEG>, G, SEG>() <= kMaxSmem;
-    static constexpr bool k10 = seg_smem_bytes<Op, RW, 3, 7, kSegQueue<Op, SEG>, G, SEG>() <= kMaxSmem;
+    static constexpr bool k13 = seg_smem_bytes<Op, RW, 4, 9, kSegQueue<Op, SEG>, G, SEG, VIEW>() <= kMaxSmem;
+    static constexpr bool k12 = seg_smem_bytes<Op, RW, 4, 8, kSegQueue<Op, SEG>, G, SEG, VIEW>() <= kMaxSmem;
+    static constexpr bool k11 = seg_smem_bytes<Op, RW, 3, 8, kSegQueue<Op, SEG>, G, SEG, VIEW>() <= kMaxSmem;
+    static constexpr bool k10 = seg_smem_bytes<Op, RW, 3, 7, kSegQueue<Op, SEG>, G, SEG, VIEW>() <= kMaxSmem;
     static constexpr int RS = (k13 || k12 || k11) ? 4 : 3;
     static constexpr int SS = k13 ? 9 : k12 ? 8 : (k11 || k10) ? 7 : 6;
     // Two threads per row double the per-thread prefixes: some types do not
     // fit 9 stages then, and that shape is not offered for them.
-    static constexpr bool kFits = seg_smem_bytes<Op, RW, RS, SS, kSegQueue<Op, SEG>, G, SEG>() <= kMaxSmem;
+    static constexpr bool kFits = seg_smem_bytes<Op, RW, RS, SS, kSegQueue<Op, SEG>, G, SEG, VIEW>() <= kMaxSmem;
     static_assert(kFits || SPLIT > 1, "227 KB per CTA");
 };
 
-template <class Op, bool INCL, bool SEG, int UNIT, int SPLIT>
+template <class Op, bool INCL, bool SEG, int UNIT, int SPLIT, bool VIEW = false>
 cudaError_t launch_seg_t(const ScanArgs& a, const SegArgs& sg, const GenericConfig& cfg, int num_sms,
                          cudaStream_t stream, LaunchInfo* info) {
-    using St = SegStages<Op, UNIT, SEG, SPLIT>;
+    using St = SegStages<Op, UNIT, SEG, SPLIT, VIEW>;
     if constexpr (!St::kFits) {
         return cudaErrorNotSupported;
     } else {
-    auto kern = scan_seg_kernel<Op, St::RW, St::RS, St::SS, kSegQueue<Op, SEG>, UNIT, INCL, SEG>;
-    constexpr size_t smem = seg_smem_bytes<Op, St::RW, St::RS, St::SS, kSegQueue<Op, SEG>, UNIT, SEG>();
-    constexpr int threads = SegShape<Op, St::RW, SEG>::kThreads;
+    auto kern = scan_seg_kernel<Op, St::RW, St::RS, St::SS, kSegQueue<Op, SEG>, UNIT, INCL, SEG, VIEW>;
+    constexpr size_t smem = seg_smem_bytes<Op, St::RW, St::RS, St::SS, kSegQueue<Op, SEG>, UNIT, SEG, VIEW>();
+    constexpr int threads = SegShape<Op, St::RW, SEG, VIEW>::kThreads;
     RowMaps maps;
-    cudaError_t err = encode_row_maps(a.in, a.out, a.n, static_cast<uint32_t>(sizeof(typename Op::T)), &maps);
+    cudaError_t err = encode_row_maps(a.in, a.out, a.n, a.n + (VIEW ? a.view_shift : 0u),
+                                      static_cast<uint32_t>(sizeof(typename Op::T)), &maps);
     if (err != cudaSuccess) return err;
     int occ = 0;
     err = resident_ctas_per_sm(kern, threads, smem, &occ);

@@ -56,9 +56,9 @@ cudaError_t encode_one(CUtensorMap* map, const void* base, uint64_t n, uint32_t 
 
 }  // namespace
 
-cudaError_t encode_row_maps(const void* in, void* out, uint64_t n, uint32_t elem_size, RowMaps* maps) {
+cudaError_t encode_row_maps(const void* in, void* out, uint64_t n, uint64_t out_n, uint32_t elem_size, RowMaps* maps) {
     cudaError_t err = encode_one(&maps->in, in, n, elem_size);
-    if (err == cudaSuccess) err = encode_one(&maps->out, out, n, elem_size);
+    if (err == cudaSuccess) err = encode_one(&maps->out, out, out_n, elem_size);
     return err;
 }
 

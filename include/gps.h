@@ -258,8 +258,7 @@ gps_status gps_plan_set_small_max(gps_plan plan, uint64_t max_n);
  * the persistent kernels' pipeline, whose latency dominates at these sizes;
  * larger ones run on a persistent L2-buffered kernel. 0 sends them all to
  * the persistent kernels. Forced-stall and fallback modes always use the
- * persistent kernel. Buffers that are not 16-byte aligned take it at every
- * size unless max_n is 0. The kernel takes its tile ids from the block index and
+ * persistent kernel. The kernel takes its tile ids from the block index and
  * relies on the hardware starting lower-numbered blocks first, as CUB's
  * decoupled lookback does; its waits are bounded all the same. */
 gps_status gps_plan_set_mid_max(gps_plan plan, uint64_t max_n);
