@@ -118,6 +118,17 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* gmem_src, uint32_t 
                  : "memory");
 }
 
+// Hint: bring the 128-byte line at p into L2. It reads nothing, so a dependent
+// launch may give it before grid_dep_wait(): L2 is where the kernels ahead write.
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory");
+}
+// By at least 128 threads: tile t (16 KB) of a buffer of `bytes` bytes.
+__device__ __forceinline__ void prefetch_tile_l2(const void* buf, uint32_t t, uint64_t bytes, uint32_t tid) {
+    const uint64_t at = t * 16384ull + tid * 128u;
+    if (tid < 128u && at < bytes) prefetch_l2(static_cast<const char*>(buf) + at);
+}
+
 // Tiled tensor copies (TMA) of a 2-D tensor map passed as a __grid_constant__
 // kernel parameter. x is the innermost coordinate (always 0 here: whole
 // 128-byte rows), y the row.

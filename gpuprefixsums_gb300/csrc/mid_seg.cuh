@@ -229,6 +229,8 @@ __global__ void __launch_bounds__(kMidSegThreads, CTAS)
     const uint32_t lane = tid & 31u;
     const uint32_t warp = tid >> 5;
     const uint32_t t = blockIdx.x;
+    // As in mid.cu: FP32 2^20 5.6 -> 5.1 us, 2^22 10.5 -> 9.1; 500 compensated scans 9.8 -> 8.8.
+    ptx::prefetch_tile_l2(a.in, t, a.n * sizeof(T), tid);
     ptx::grid_dep_launch();
     ptx::grid_dep_wait();
     const uint64_t tag = threadIdx.x < 32 ? ptx::ld_relaxed_u64(a.mid_launch) : 0;

@@ -454,6 +454,20 @@ __global__ void __launch_bounds__(SegShape<Op, RW, SEG, VIEW>::kThreads, 1)
         ctrl->end_seq = 0xFFFFFFFFu;
         ptx::fence_mbar_init();
     }
+    // While the kernel ahead drains, a unit comes into L2: number blockIdx.x, which most
+    // likely is the first one this CTA takes, and some CTA's in any case. Measured on
+    // GB300: FP32 2^23 16.9 -> 16.2 us, batched u32 17.7 -> 17.3, nothing from 2^24 on (nor
+    // for two units a CTA).
+    if (tid == 32) {
+#pragma unroll
+        for (int k = 0; k < G; ++k) {
+            const uint64_t r0 = static_cast<uint64_t>(blockIdx.x * G + k) * ROWS;
+            const uint64_t r1 = r0 + ROWS < rows_full ? r0 + ROWS : rows_full;
+            if (r0 < r1)
+                ptx::bulk_prefetch_l2(static_cast<const T*>(a.in) + r0 * ROW, static_cast<uint32_t>((r1 - r0) * 128),
+                                      ptx::policy_evict_last());
+        }
+    }
     ptx::grid_dep_launch();
     ptx::grid_dep_wait();
     __syncthreads();

@@ -44,6 +44,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     constexpr int ITEMS = kSmallItems<T>;
     constexpr int CHUNK = kSmallThreads * ITEMS;
     __shared__ gps_device::BlockScanStorage<kSmallThreads, T> st;
+    for (uint32_t i = threadIdx.x; i * 128u < n * sizeof(T); i += kSmallThreads)
+        ptx::prefetch_l2(reinterpret_cast<const char*>(in) + i * 128u);
     ptx::grid_dep_launch();
     ptx::grid_dep_wait();
     T carry = carry_in != nullptr ? *carry_in : T(0);
