@@ -126,7 +126,7 @@ gps::GenericConfig generic_config(const gps_plan_s* p, bool segmented, uint64_t 
     const int c = p->tuned[segmented ? 1 : 0][size_class(n)];
     if (c >= 0 && c < gps::kNumGenericCandidates) return gps::kGenericCandidates[c];
     const uint64_t tiles = (n + p->tile_elems - 1) / p->tile_elems;
-    if (tiles <= (c == kTunedMid ? gps::kMidSegMaxTiles : gps::mid_seg_default_tiles(p->dtype)))
+    if (tiles <= (c == kTunedMid ? gps::kMidSegMaxTiles : gps::mid_seg_default_tiles(p->dtype, segmented)))
         return gps::kMidSegConfig;
     return gps::default_generic_config(n, p->tile_elems, p->num_sms);
 }

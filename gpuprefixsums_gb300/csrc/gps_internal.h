@@ -233,9 +233,9 @@ bool seg_u32x4_x2_fits(uint32_t unit);
 // element size, and the launch. a.carry_out receives the count (uint64).
 uint32_t select_tile_elems(size_t elem_size);
 // Selects of up to this many tiles run one tile per CTA, on the plan's
-// mid-size descriptors (2048 tiles of u32 16.9 us against 17.5 on the persistent
-// kernel, 2560 19.3 / 19.3, 3072 22.9 / 21.3).
-constexpr uint32_t kMidSelectMaxTiles = 2560;
+// mid-size descriptors (u32 2450 tiles 17.2 us against 18.9 on the persistent kernel, 2500
+// 18.6 / 18.6, 2600 20.6 / 19.0; u64 2600 19.6 / 18.2).
+constexpr uint32_t kMidSelectMaxTiles = 2500;
 cudaError_t launch_select(size_t elem_size, const ScanArgs& a, const uint8_t* flags, int num_sms, cudaStream_t stream,
                           LaunchInfo* info);
 
@@ -247,8 +247,8 @@ cudaError_t launch_small(gps_dtype dtype, bool inclusive, const ScanArgs& a, cud
 // Integer chained scans up to mid size, one 16 KB tile per CTA (mid.cu); the
 // default upper size of a plan, in bytes of input. Measured on GB300 (graph
 // replay) against the persistent kernel that takes over (the generic one):
-// u32 2^22 9.7 against 13.7 us, 2^23 16.7 / 17.9, 2300 tiles 17.9 / 19.0, 2560 20.5 /
-// 19.5, 2^24 31.4 / 26; u64 1800 tiles 16.1 / 15.9, 2048 17.6 / 16.6.
+// u32 2^22 8.4 against 13.7 us, 2^23 15.3 / 17.7, 2320 tiles 17.0 / 19.1, 2560 19.8 /
+// 19.0, 2^24 30.9 / 26; u64 1700 tiles 14.3 / 15.9, 2048 16.2 / 15.9.
 constexpr size_t mid_max_bytes(gps_dtype dtype) { return dtype == GPS_DTYPE_U64 ? 28ull << 20 : 38ull << 20; }
 // Tile descriptors of the one-tile-per-CTA kernels sit one per 128-byte line
 // (a stride of 8 words) when a launch has more than one group of 32 tiles
@@ -274,17 +274,17 @@ constexpr GenericConfig kMidSegConfig = {0, 1, 1};
 // Untuned scans of up to this many tiles take it; larger ones the kernel with
 // units, whose pipeline then pays. The wider the running state, the fewer CTAs
 // an SM holds and the longer each takes. Measured on GB300 (graph replay, us, one
-// tile per CTA against units of 4 tiles): FP32 1536 tiles 14.5 / 16.0, 2048 18.7 /
-// 16.9; batched u32 15.2 / 15.6 and 18.7 / 17.8; compensated 1024 tiles 13.8 / 14.4,
-// 1280 16.0 / 15.2; batched u64 13.1 / 13.5 and 14.5 / 14.3; batched compensated 15.2 /
-// 15.4 and 17.0 / 16.4; structs 640 tiles 10.8 / 11.8, 768 12.9 / 11.9, batched 11.6 /
-// 12.0 and 12.8 / 12.5.
-constexpr uint64_t mid_seg_default_tiles(gps_dtype dtype) {
+// tile per CTA against units of 4 tiles): FP32 1700 tiles 14.3 / 15.3, 1900 15.4 / 15.7,
+// 2100 16.6 / 16.5; batched u32 14.7 / 16.6, 16.1 / 16.9, 17.5 / 17.8; compensated 1250 tiles
+// 13.3 / 14.0, 1400 15.5 / 15.0, batched 15.3 / 15.9 and 16.4 / 16.7, 1700 18.9 / 19.3; batched u64
+// 1250 tiles 12.9 / 13.6, 1700 15.9 / 16.4; structs 640 tiles 10.8 / 11.8, 720 11.4 / 11.0, batched
+// 11.6 / 12.0 and 11.7 / 11.8.
+constexpr uint64_t mid_seg_default_tiles(gps_dtype dtype, bool segmented) {
     switch (dtype) {
         case GPS_DTYPE_U32:
-        case GPS_DTYPE_F32: return 1664;
-        case GPS_DTYPE_U64:
-        case GPS_DTYPE_F32_COMPENSATED: return 1216;
+        case GPS_DTYPE_F32: return 2048;
+        case GPS_DTYPE_U64: return 1728;
+        case GPS_DTYPE_F32_COMPENSATED: return segmented ? 1728 : 1280;
         case GPS_DTYPE_U32X4: break;
     }
     return 704;

@@ -170,8 +170,8 @@ gps_status gps_select_flagged(gps_plan plan, const void* d_in, const uint8_t* d_
  * GPS_ERR_CUDA after tuning with the others. A shape that does not fit one
  * CTA's shared memory for the element type is skipped. Up to 4096 tiles the
  * one-tile-per-CTA form of the kernel is a candidate too. Without tuning, scans
- * of up to 1664 tiles (u32, f32), 1216 (u64, compensated f32) or 704 (structs)
- * take that form; larger ones use one thread per row and units of 4 tiles once
+ * of up to 2048 tiles (u32, f32), 1728 (u64), 1280 (compensated f32, 1728 batched)
+ * or 704 (structs) take that form; larger ones use one thread per row and units of 4 tiles once
  * there is one such unit per SM, else 1 tile. d_out is left holding a correct
  * result. Synchronizes `stream`; not allowed while the stream is being
  * captured. The chosen configuration is returned in out_unit /

@@ -36,7 +36,7 @@ def _lengths(rng, n, style):
 def test_batched_integers(cuda, dtype, style):
     tile = 16384 // np.dtype(NP[dtype]).itemsize
     sizes = [1, 3, tile - 1, tile, tile + 1, 31 * tile + 7, 32 * tile, 32 * tile + 1, 33 * tile + 5, 64 * tile,
-             65 * tile, 100 * tile + 9, 1216 * tile, 1217 * tile - 3, 1665 * tile - 1]
+             65 * tile, 100 * tile + 9, 1216 * tile, 1217 * tile - 3, 1728 * tile, 2049 * tile - 1]
     with Plan("csdl", dtype, max_n=max(sizes)) as plan:
         for n in sizes:
             rng = np.random.default_rng(n)
@@ -56,7 +56,8 @@ def test_batched_integers(cuda, dtype, style):
 @pytest.mark.parametrize("inclusive", [False, True])
 @pytest.mark.parametrize("dt", ["f32", "f32c"])
 def test_floating_point(cuda, dt, inclusive):
-    sizes = [1, 4095, 4097, 32 * 4096 + 1, 65 * 4096 - 2, 129 * 4096, 1216 * 4096 - 1, 1217 * 4096, 1665 * 4096 - 7]
+    sizes = [1, 4095, 4097, 32 * 4096 + 1, 65 * 4096 - 2, 129 * 4096, 1216 * 4096 - 1, 1217 * 4096, 1281 * 4096 - 7,
+             2049 * 4096 - 7]
     with Plan("csdl", dt, max_n=max(sizes)) as plan:
         for n in sizes:
             x = fp_input("mixed", n, seed=n)
