@@ -344,17 +344,18 @@ constexpr size_t seg_smem_bytes() {
            sizeof(SegCtrl<Op, RW, RS, SS, Q, G, SEG, VIEW>);
 }
 
-template <class Op, int RW, bool SEG, bool VIEW = false>
+template <class Op, int RW>
 struct SegShape {
     static constexpr int kLookbackWarps = 3;
-    // Groups of RW finalize warps, each with stages of its own: two for segmented
-    // scans and for states of 8 bytes, one for the rest. A single group is one warp
-    // per scheduler, each waiting on its own chain. Measured on GB300, one group
+    // Groups of RW finalize warps, each with stages of its own: two (one where two
+    // threads share a row). A single group is one warp per scheduler, each waiting on
+    // its own chain. Measured on GB300, one group
     // against two: compensated FP32 2^26 91.7 / 85.9 us, in 500 segments 117 / 108, in
     // 20,000 151 / 131; batched 2^28 u32 317 / 310, 2^26 u64 174 / 162, 2^24 structs
-    // 103 / 99; plain 2^24 u64 48.7 / 46.3, u32 off a boundary 2^27 176 / 160, but aligned
-    // 2^28 u32 318.1 / 319.5 (three groups: compensated batches 117 / 143).
-    static constexpr int kFinalGroups = RW == 4 && (SEG || VIEW || sizeof(typename Op::S) == 8) ? 2 : 1;
+    // 103 / 99; plain 2^24 u64 48.7 / 46.3, u32 2^24 26.1 / 25.6, 2^26 86.5 / 84.9, 2^28 315.7 /
+    // 316.1, off a boundary 2^27 176 / 160, FP32 2^25 47.6 / 46.7 (three groups: compensated
+    // batches 117 / 143).
+    static constexpr int kFinalGroups = RW == 4 ? 2 : 1;
     // R-loader, S-loader, storer, head warp, lookback warps, aggregator,
     // reduce warps, finalize warps.
     static constexpr int kThreads = 32 * (5 + kLookbackWarps + (1 + kFinalGroups) * RW);
@@ -374,7 +375,7 @@ struct SegShape {
 // CTA (mid.cu) against this: u32 2^24 33 / 27-30 us, 2^25 70.6 / 47, 2^27 258 / 160 (aligned
 // 26, 46, 162); u64 2^24 73 / 48. With one finalize group, u32 2^25 53, 2^27 176.
 template <class Op, int RW, int RS, int SS, int Q, int G, bool INCL, bool SEG, bool VIEW = false>
-__global__ void __launch_bounds__(SegShape<Op, RW, SEG, VIEW>::kThreads, 1)
+__global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
     scan_seg_kernel(const ScanArgs a, const SegArgs sg, const __grid_constant__ CUtensorMap tin,
                     const __grid_constant__ CUtensorMap tout) {
     using T = typename Op::T;
@@ -390,9 +391,9 @@ __global__ void __launch_bounds__(SegShape<Op, RW, SEG, VIEW>::kThreads, 1)
     constexpr int CHUNKS = ITEMS / EPC;
     constexpr uint32_t NROLE = RW * 32;
     constexpr uint32_t ROWS = 128;  // rows per tile
-    constexpr uint32_t LW = SegShape<Op, RW, SEG, VIEW>::kLookbackWarps;
+    constexpr uint32_t LW = SegShape<Op, RW>::kLookbackWarps;
     constexpr uint32_t kWarpLookback = 4, kWarpAgg = 4 + LW, kWarpReduce = 5 + LW, kWarpFinal = 5 + LW + RW;
-    constexpr uint32_t FG = SegShape<Op, RW, SEG, VIEW>::kFinalGroups;
+    constexpr uint32_t FG = SegShape<Op, RW>::kFinalGroups;
     constexpr uint32_t kLaneEntries = G * RW;  // aggregator entries per lane
     auto entry_at = [](uint32_t j) -> uint32_t { return j + j / kLaneEntries; };
     constexpr int kHeadWords = TILE / 32;

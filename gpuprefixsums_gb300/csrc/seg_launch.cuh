@@ -20,15 +20,16 @@ namespace gps {
 constexpr int kSegWarps = 4;
 // Units in flight per CTA: each waits in L2 (64 KB, or 16 KB in single-tile
 // units) between the two passes, 152 x 6 x 64 KB at most. A smaller queue also
-// leaves shared memory for stages. Measured on GB300: batched scans take 5 (2^27
+// leaves shared memory for stages. Measured on GB300: integers take 5 (2^26 u32 with 5 / 6:
+// 83.4 / 84.9 us, 3 x 2^25 122.4 / 125.5, 3 x 2^24 u64 121.8 / 125.0), batched scans too (2^27
 // u64 with 4 / 5 / 6: 321 / 313 / 316 us, 4096 u32 segments 355 / 352 / 352), compensated
 // and struct batches 4 (2^24 compensated 35.5 / 36.4 / 37.4, structs 92.8 / 99.4 / 99.9),
-// plain structs 5 (2^24 98 / 107 for 5 / 6), the rest 6 -- of which plain scans of
-// 512 MB and more use 5 (2^28 u32 317 / 322, 2^27 163 / 165; 2^26 FP32 88.0 / 87.3); 4 or 3
-// are slower there (2^28 u32 333 and 385).
+// plain structs 5 (2^24 98 / 107 for 5 / 6), plain FP32 and compensated FP32 6 (2^25
+// compensated 47.4 / 46.9), but 5 from 512 MB on (2^27 FP32 162.1 / 161.2, 2^28 312.8 / 313.1). 4 or 3
+// are slower (2^28 u32 333 and 385).
 template <class Op, bool SEG>
 constexpr int kSegQueue = SEG ? (sizeof(typename Op::S) > sizeof(typename Op::T) || sizeof(typename Op::S) == 16 ? 4 : 5)
-                              : (sizeof(typename Op::S) == 16 ? 5 : 6);
+                              : (sizeof(typename Op::S) == 16 || std::is_integral<typename Op::S>::value ? 5 : 6);
 constexpr uint64_t kSegDeepBytes = 512ull << 20;
 constexpr size_t kMaxSmem = 232448;
 
@@ -56,7 +57,7 @@ cudaError_t launch_seg_t(const ScanArgs& a, const SegArgs& sg, const GenericConf
     } else {
     auto kern = scan_seg_kernel<Op, St::RW, St::RS, St::SS, kSegQueue<Op, SEG>, UNIT, INCL, SEG, VIEW>;
     constexpr size_t smem = seg_smem_bytes<Op, St::RW, St::RS, St::SS, kSegQueue<Op, SEG>, UNIT, SEG, VIEW>();
-    constexpr int threads = SegShape<Op, St::RW, SEG, VIEW>::kThreads;
+    constexpr int threads = SegShape<Op, St::RW>::kThreads;
     RowMaps maps;
     cudaError_t err = encode_row_maps(a.in, a.out, a.n, a.n + (VIEW ? a.view_shift : 0u),
                                       static_cast<uint32_t>(sizeof(typename Op::T)), &maps);
