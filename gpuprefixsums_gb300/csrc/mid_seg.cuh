@@ -10,7 +10,8 @@
 //      Chunk c sits at c ^ ((c >> 3) & 3), so that both the coalesced stores
 //      and each thread's own reads touch every bank once;
 //   2. segmented: while the loads are in flight, find the first offset of the
-//      tile with 256 probes a round and mark the heads in a bitmap;
+//      tile, with 256 probes a round until 1024 are left, and mark the heads in
+//      a bitmap;
 //   3. aggregate each thread's items, scan over the block, publish the tile's
 //      aggregate;
 //   4. lookback in a fixed order (below);
@@ -255,9 +256,14 @@ __global__ void __launch_bounds__(kMidSegThreads, CTAS)
     if constexpr (SEG) {
         for (uint32_t w = tid; w < kHeadWords; w += kMidSegThreads) s_head[w] = 0u;
         const uint32_t nseg = sg.num_segments;
+        // Offsets a thread reads at a time. An interval that one such reading covers is
+        // not narrowed further: up to 1024 segments no probe is left, and one latency
+        // less ahead of the scan (500 compensated scans 8.8 -> 8.5 us, 1000 segments of
+        // 2^20 u32 5.66 -> 5.44; from 5000 segments on no change).
+        constexpr uint32_t kBatch = 4;
         // Entries before lo are below t0; entry hi (if any) is not.
         uint32_t lo = 0, hi = nseg;
-        while (hi - lo > kMidSegThreads) {
+        while (hi - lo > kBatch * kMidSegThreads) {
             const uint32_t step = (hi - lo + kMidSegThreads - 1) / kMidSegThreads;
             const uint64_t idx = lo + static_cast<uint64_t>(tid) * step;
             const bool below = idx < hi && sg.offsets[idx] < t0;
@@ -270,16 +276,15 @@ __global__ void __launch_bounds__(kMidSegThreads, CTAS)
             lo = lo + (c - 1) * step + 1;
         }
         __syncthreads();
-        constexpr int kBatch = 4;  // offset loads in flight per thread
         for (uint64_t cur = lo;; cur += kBatch * kMidSegThreads) {
             uint64_t o[kBatch];
 #pragma unroll
-            for (int j = 0; j < kBatch; ++j) {
+            for (uint32_t j = 0; j < kBatch; ++j) {
                 const uint64_t idx = cur + j * kMidSegThreads + tid;
                 o[j] = idx < nseg ? sg.offsets[idx] : ~0ull;
             }
 #pragma unroll
-            for (int j = 0; j < kBatch; ++j) {
+            for (uint32_t j = 0; j < kBatch; ++j) {
                 if (o[j] >= t0 && o[j] < t0 + cnt) {
                     const uint32_t pos = static_cast<uint32_t>(o[j] - t0);
                     atomicOr(&s_head[pos >> 5], 1u << (pos & 31u));

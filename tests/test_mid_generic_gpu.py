@@ -151,3 +151,18 @@ def test_captured_batches_replay(cuda):
             torch.cuda.synchronize()
             assert np.array_equal(out.cpu().numpy().view(np.uint32), oracle.segscan(y, offs, False)), k
         plan.check()
+
+
+@pytest.mark.parametrize("count", [255, 1023, 1024, 1025, 2049, 70_000])
+def test_segment_counts_around_one_reading(cuda, count):
+    """A CTA reads up to 1024 offsets at once and narrows longer lists first."""
+    n = 130 * 4096 + 11
+    rng = np.random.default_rng(count)
+    offs = np.concatenate([[0], np.sort(rng.integers(0, n + 1, size=count - 1)), [n]])
+    x = rng.integers(0, 1 << 32, size=n, dtype=np.uint64).astype(np.uint32)
+    d_off = torch.from_numpy(offs.astype(np.uint32).view(np.int32)).cuda()
+    with Plan("csdl", "u32", max_n=n) as plan:
+        for inclusive in (False, True):
+            got = plan.scan_segmented(dev(x), d_off, inclusive=inclusive)
+            assert np.array_equal(got.cpu().numpy().view(np.uint32), oracle.segscan(x, offs, inclusive))
+        plan.check()
