@@ -63,10 +63,11 @@ struct gps_plan_s {
     // covers them).
     void* group_desc16;
     // Chained-scan plans: the 16-byte, launch-tagged descriptors of the
-    // one-tile-per-CTA kernels (mid.cu; mid_seg.cuh), and one per group of 32
-    // tiles; else null.
+    // one-tile-per-CTA kernels (mid.cu; mid_seg.cuh), and group descriptors of the
+    // latter; else null.
     void* desc_mid;
     void* group_desc_mid;
+    void* group_sums;  // integer chained-scan plans: the group sums of mid.cu
     // Integer scans of at most this many elements run in one CTA (small.cu).
     uint64_t small_max;
     uint64_t mid_max;  // chained-scan plans: largest scan run as one tile per CTA
@@ -103,6 +104,7 @@ gps_status cuda_fail(cudaError_t err, const char* what) {
 }
 
 constexpr size_t kHeaderBytes = sizeof(gps::WsHeader);
+constexpr size_t kSumsBytes = 2 * 128 * static_cast<size_t>(gps::kMidSums) + 32;
 constexpr size_t kCarryBytes = 128;  // two carry slots, padded to a line
 constexpr uint64_t kDefaultBudgetNs = 1000000000ull;
 
@@ -209,7 +211,7 @@ gps_status launch_scan(gps_plan_s* p, bool inclusive, const void* in, void* out,
     } else if (p->algo == GPS_ALGO_CSDL && (n <= p->mid_max || (unaligned && p->mid_max != 0)) &&
                p->stall.mode == 0 && p->stall.fallback_polls == 0) {
         a.desc = p->desc_mid;
-        a.group_desc = p->group_desc_mid;
+        a.group_desc = p->group_sums;
         err = gps::launch_mid(p->dtype, inclusive, a, p->num_sms, stream, &p->last_launch);
     } else if (p->algo == GPS_ALGO_CSDL) {
         err = gps::launch_csdl(p->dtype, inclusive, p->stall.mode != 0 || p->stall.fallback_polls != 0, a, p->num_sms,
@@ -341,10 +343,9 @@ gps_status gps_plan_create(gps_plan* out_plan, gps_algo algo, gps_dtype dtype, u
     // own so that the two formats never meet in one slot.
     const uint64_t slots16 = (algo == GPS_ALGO_CSDL && dtype == GPS_DTYPE_U32) ? seg_units + seg_groups : 0;
     // One-tile-per-CTA kernels of chained-scan plans: 16-byte descriptors
-    // tagged with the launch, in a region no other kernel uses (for types
-    // without an integer kernel, only as many as the generic one takes).
-    const uint64_t tiles_mid =
-        generic_only(dtype) ? std::min<uint64_t>(tiles, gps::kMidSegMaxTiles) : tiles;
+    // tagged with the launch, in a region no other kernel uses, for as many tiles
+    // as a launch of theirs takes.
+    const uint64_t tiles_mid = std::min<uint64_t>(tiles, gps::kMidMaxTiles);
     const uint64_t slots_mid = algo == GPS_ALGO_CSDL ? tiles_mid + gps::kDescPad : 0;
     const uint64_t groups_mid = slots_mid ? (tiles_mid + 31) / 32 + gps::kDescPad : 0;
     // [header][carries][descriptors or range sums]; for u32 chained-scan
@@ -355,7 +356,10 @@ gps_status gps_plan_create(gps_plan* out_plan, gps_algo algo, gps_dtype dtype, u
     const size_t end16 = slots16 ? region16 + kHeaderBytes + slots16 * 16 : main_bytes;
     const size_t region_mid = (end16 + 255) & ~static_cast<size_t>(255);
     const uint64_t words_mid = slots_mid ? gps::mid_desc_words(tiles_mid) : 0;
-    p->scratch_bytes = slots_mid ? region_mid + (words_mid + groups_mid * gps::kMidDescStride) * 16 : end16;
+    const size_t end_mid = slots_mid ? region_mid + (words_mid + groups_mid * gps::kMidDescStride) * 16 : end16;
+    const size_t region_sums = (end_mid + 255) & ~static_cast<size_t>(255);
+    const bool sums = algo == GPS_ALGO_CSDL && !generic_only(dtype);
+    p->scratch_bytes = sums ? region_sums + kSumsBytes : end_mid;
     err = cudaMalloc(&p->scratch, p->scratch_bytes);
     if (err != cudaSuccess) {
         const size_t bytes = p->scratch_bytes;
@@ -371,6 +375,7 @@ gps_status gps_plan_create(gps_plan* out_plan, gps_algo algo, gps_dtype dtype, u
     if (algo == GPS_ALGO_CSDL) p->group_desc16 = static_cast<char*>(p->desc16) + seg_units * 16;
     p->desc_mid = slots_mid ? static_cast<char*>(p->scratch) + region_mid : nullptr;
     p->group_desc_mid = slots_mid ? static_cast<char*>(p->scratch) + region_mid + words_mid * 16 : nullptr;
+    p->group_sums = sums ? static_cast<char*>(p->scratch) + region_sums : nullptr;
     gps::WsHeader h{};
     h.epoch = 1;
     h.capacity_tiles = slots;
@@ -748,6 +753,10 @@ gps_status gps_plan_check(gps_plan p, gps_stream_t stream) {
         err = cudaMemcpy(&number, &p->hdr->mid_launch, sizeof(number), cudaMemcpyDeviceToHost);
         number += 2;
         if (err == cudaSuccess) err = cudaMemcpy(&p->hdr->mid_launch, &number, sizeof(number), cudaMemcpyHostToDevice);
+        if (err == cudaSuccess && p->group_sums != nullptr) {
+            err = cudaMemset(p->group_sums, 0, kSumsBytes);
+            if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
+        }
         if (err != cudaSuccess) return cuda_fail(err, "advancing the launch number");
     }
     if (all != 0) return fail(GPS_ERR_TIMEOUT, "a device-side wait exceeded its budget (flags 0x%x)", all);

@@ -48,6 +48,7 @@ struct alignas(128) WsHeader {
     unsigned long long stat_inserts;    // fallback aggregates that won the CAS
     unsigned long long stat_stalls;     // tiles that were made to stall
     uint64_t mid_launch;                // launch number of the one-tile-per-CTA kernels
+    uint64_t sums_launch;               // how many of them used the group sums (mid.cu)
 };
 static_assert(sizeof(WsHeader) == 128, "header is one 128-byte line");
 
@@ -106,8 +107,9 @@ struct ScanArgs {
     uint32_t desc_stride;
     WsHeader* hdr;       // plan state (counters, epoch, error flags)
     void* desc;          // tile descriptors (lookback)
-    // Descriptors of groups: of 32 tiles for the one-tile-per-CTA kernels, of
-    // det_group_units() lookback units for the generic kernel.
+    // Descriptors of groups: of kMidSegGroup tiles for the one-tile-per-CTA form
+    // of the generic kernel, of det_group_units() lookback units for the other. For
+    // mid.cu: two sets of kMidSums 128-byte lines, and two 16-byte carries.
     void* group_desc;
     const void* carry_in;  // optional: one element added to every output
     void* carry_out;       // optional: receives carry_in + sum of all n inputs
@@ -251,25 +253,26 @@ cudaError_t launch_small(gps_dtype dtype, bool inclusive, const ScanArgs& a, cud
 // 19.0, 2^24 30.9 / 26; u64 1700 tiles 14.3 / 15.9, 2048 16.2 / 15.9.
 constexpr size_t mid_max_bytes(gps_dtype dtype) { return dtype == GPS_DTYPE_U64 ? 28ull << 20 : 38ull << 20; }
 // Tile descriptors of the one-tile-per-CTA kernels sit one per 128-byte line
-// (a stride of 8 words) when a launch has more than one group of 32 tiles
-// and at most kMidStrideMaxTiles tiles, else packed. Sharing lines between
+// (a stride of 8 words) when a launch has more than one group of 32 tiles, else
+// packed. Sharing lines between
 // tiles that publish and read at the same moment cost up to 3 us per read
 // (2^20 u32: 6.04 us packed, 4.95 us one per line, 5.23 us one per 32-byte
 // sector); with one group, packed reads are faster (2^17: 2.83 against
-// 3.36 us). Group descriptors always take a line each (2^22 u32: 7.56
-// against 8.84 us packed). Tile-descriptor words a plan keeps for `tiles`
-// tiles:
+// 3.36 us). Group sums and group descriptors always take a line each. A launch
+// takes at most kMidMaxTiles tiles. Tile-descriptor words a plan keeps for
+// `tiles` tiles:
 constexpr uint32_t kMidDescStride = 8;
-constexpr uint64_t kMidStrideMaxTiles = 4096;
+constexpr uint64_t kMidMaxTiles = 4096;
 constexpr uint64_t mid_desc_words(uint64_t tiles) {
-    const uint64_t strided = ((tiles < kMidStrideMaxTiles ? tiles : kMidStrideMaxTiles) + kDescPad) * kMidDescStride;
-    return tiles + kDescPad > strided ? tiles + kDescPad : strided;
+    return ((tiles < kMidMaxTiles ? tiles : kMidMaxTiles) + kDescPad) * kMidDescStride;
 }
+// Group sums of the integer kernel: two sets, 128 bytes a group.
+constexpr uint32_t kMidSums = 128;
 // One-tile-per-CTA form of the generic kernel (mid_seg.cuh): tiles per group
 // of its lookback, and the most tiles it takes.
 constexpr uint32_t kMidSegGroup = 64;
 constexpr uint32_t kMidSegMaxTiles = 4096;
-static_assert(kMidSegGroup >= 32 && kMidSegMaxTiles <= kMidStrideMaxTiles, "within the plan's mid-size descriptors");
+static_assert(kMidSegGroup >= 32 && kMidSegMaxTiles <= kMidMaxTiles, "within the plan's mid-size descriptors");
 constexpr GenericConfig kMidSegConfig = {0, 1, 1};
 // Untuned scans of up to this many tiles take it; larger ones the kernel with
 // units, whose pipeline then pays. The wider the running state, the fewer CTAs

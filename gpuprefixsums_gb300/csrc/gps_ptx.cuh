@@ -199,6 +199,9 @@ __device__ __forceinline__ void st_relaxed_u64(uint64_t* p, uint64_t v) {
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
+__device__ __forceinline__ void red_add_u64(uint64_t* p, uint64_t v) {
+    asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 __device__ __forceinline__ uint64_t atom_cas_u64(uint64_t* p, uint64_t cmp, uint64_t val) {
     uint64_t old;
     asm volatile("atom.relaxed.gpu.global.cas.b64 %0, [%1], %2, %3;"

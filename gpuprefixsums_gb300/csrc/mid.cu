@@ -10,18 +10,17 @@
 //      lookback relies on the same order); every wait is bounded, so a
 //      violation would surface as GPS_ERR_TIMEOUT, never as a hang;
 //   2. load the tile and block-scan it;
-//   3. publish the tile aggregate and look back (warp 0): over the tiles of
-//      its group of 32, then, if needed, over the descriptors of earlier
-//      groups;
-//   4. publish the inclusive prefix, add the prefix, store.
+//   3. publish the tile's sum and look back: over the tiles of its group of 32
+//      and over the sums of the earlier groups, at the same time;
+//   4. add the prefix, store.
 // The kernels keep their descriptors in a region of the plan of their own,
 // tagged with the launch's number, which every CTA reads from the plan's
 // header beside its data loads. A descriptor counts only when its tag is the
 // current launch's, so a launch needs no clearing memset. The last tile's CTA
-// advances the number once its own prefix is known: that prefix rests on a
-// descriptor of every tile before it, each written by a CTA that had read the
-// number, so no CTA of this launch can still be about to read it. No atomic
-// and no fence is on any CTA's path. (A number from the driver will not do:
+// advances the number once its own prefix is known: that prefix rests on
+// what every tile before it has published, each by a CTA that had read the
+// number, so no CTA of this launch can still be about to read it. No fence is
+// on any CTA's path. (A number from the driver will not do:
 // %gridid is fixed when a graph is instantiated, the same for all its
 // replays.)
 #include "gps_device.cuh"
@@ -43,7 +42,6 @@ constexpr int kMidCtasPerSm = 8;
 // word is word t * a.desc_stride of the region: launches of more than one
 // group of tiles give each tile a 128-byte line of its own, since tiles that
 // publish while others read the same line waited up to 3 us for a read.
-// Group descriptors always have a line each (word g * kMidDescStride).
 constexpr uint64_t kTagMask = (1ull << 62) - 1;
 
 struct MidDesc {
@@ -58,59 +56,49 @@ struct MidDesc {
     }
 };
 
-// ------------------------------------------------------- two-level lookback
-// Tiles form groups of 32. Besides its tile descriptor, the last tile of each
-// group publishes a group descriptor: the group's aggregate as soon as its
-// in-group lookback is done, and the inclusive prefix through the group once
-// its prefix is known. Warp 0 of a tile sums its in-group predecessors back to
-// the nearest inclusive one (one descriptor per lane) and, when none of them
-// is inclusive, adds the prefix of its group: a decoupled lookback over the
-// group descriptors, 32 per poll. Each tile reads at most 31 tile descriptors
-// and the group descriptors back to the nearest inclusive one. A flat
-// lookback, in which every tile reads its predecessors' descriptors directly
-// (one warp, or all warps of the CTA, 128 to 1024 per poll), measured slower
-// from 2^19 elements on: all CTAs of a launch look back at once, and their
-// reads, quadratic in the tile count, queue on the few L2 lines that hold the
-// descriptors.
+// ---------------------------------------------------------------- lookback
+// Tiles form groups of 32. A tile publishes its sum twice, at once: in its
+// descriptor, and by an atomic addition to its group's sum, a 64-bit word with
+// the number of tiles added so far above bit 40 (two such words for u64, one
+// for each half of the values). The prefix of a tile is then the sums of the
+// groups before, complete at a count of 32, and the descriptors of the tiles
+// before in its own group: warp 0 polls these and the first 32 groups together, the
+// next three warps 32 groups each, so every tile waits for one L2 round trip
+// after the last tile before it has published.
+//
+// The group sums have two sets, which the launches that use them take in turn,
+// counted in the plan's header; tile 0's CTA clears the other set for the next.
+// Warp 0 hands that count to the CTA through shared memory, so that it has been
+// read before the CTA publishes anything, and the last tile's CTA, which has
+// then seen every tile, advances it.
+//
+// Measured on GB300, graph replay, inputs from HBM, u32, against two levels in turn
+// (the last tile of a group reads the group's descriptors and publishes their sum, which
+// the tiles of later groups read): 2^17 3.3 -> 2.9 us, 2^18 3.6 -> 3.2, 2^20 5.0 -> 4.3, 2^22
+// 8.4 -> 7.9, 2^23 15.3 -> 14.1; u64 2^19 5.4 -> 4.75, 3.5 M 14.3 -> 13.6. With the in-group read
+// in a warp of its own beside those of the groups: 2^20 4.3, but 2^22 8.4, 2^23 15.0.
+// A flat lookback, in which every tile reads its predecessors' descriptors directly, was
+// slower from 2^19 elements on: the reads, quadratic in the tile count, queue on the L2
+// lines that hold the descriptors.
 constexpr uint32_t kGroupTiles = 32;
+constexpr uint32_t kGroupWarps = kMidSums / 32;
+constexpr uint64_t kOneTile = 1ull << 40;
+static_assert(kGroupTiles * kMidSums == kMidMaxTiles, "one sum per group");
 
+template <typename T>
 struct LookbackSmem {
-    uint32_t found;    // an inclusive tile was found in the group
-    uint32_t timeout;  // a wait ran past its budget
+    T part[kGroupWarps];  // what each polling warp has found
+    uint32_t set;             // which set of group sums this launch uses
+    uint32_t timeout;         // a wait ran past its budget
 };
 
-// Warp-level lookback over the 32 descriptors at and below `top` (lane l reads
-// slot top - l when it is at least `floor`). Polls until every slot from top
-// down to the nearest inclusive one (or down to `floor`) is ready; returns
-// whether an inclusive one was found and, in `sum`, the sum of those slots.
-// Gives up after the wait budget, setting timed_out (then `sum` is 0).
-template <typename T, uint32_t SPIN = 64>
-__device__ bool warp_window(const ScanArgs& a, const ptx::u64x2* d, uint32_t stride, int64_t top, int64_t floor,
-                            uint64_t tag, uint32_t lane, T& sum, bool& timed_out) {
-    const int64_t idx = top - static_cast<int64_t>(lane);
-    bool ready = idx < floor, incl = false;
-    T v = 0;
+// Polls until `done` holds for every lane of the warp, calling look() each
+// time; false once the wait budget has run out.
+template <class Look>
+__device__ __forceinline__ bool mid_poll(const ScanArgs& a, uint32_t lane, Look look) {
     uint32_t polls = 0, backoff = 32;
     uint64_t deadline = 0;
-    timed_out = false;
-    while (true) {
-        if (!ready) {
-            const ptx::u64x2 w = ptx::ld_relaxed_b128(d + idx * stride);
-            const uint32_t st = MidDesc::status(w, tag);
-            if (st != kNotReady) {
-                ready = true;
-                v = static_cast<T>(w.lo);
-                incl = st == kInclusive;
-            }
-        }
-        const uint32_t inc_mask = __ballot_sync(kFullMask, incl);
-        const uint32_t wait_mask = __ballot_sync(kFullMask, !ready);
-        const uint32_t pinc = inc_mask ? static_cast<uint32_t>(__ffs(inc_mask) - 1) : 32u;
-        const uint32_t need = pinc >= 31u ? kFullMask : (2u << pinc) - 1u;  // lanes 0 .. pinc
-        if ((wait_mask & need) == 0) {
-            sum = warp_sum(lane <= pinc ? v : T(0));
-            return pinc != 32u;
-        }
+    while (!__all_sync(kFullMask, look())) {
         ++polls;
         if ((polls & 15u) == 1u) {
             bool expired = false;
@@ -119,87 +107,91 @@ __device__ bool warp_window(const ScanArgs& a, const ptx::u64x2* d, uint32_t str
                 if (deadline == 0) deadline = now + a.wait_budget_ns;
                 expired = now > deadline || ld_volatile_u32(&a.hdr->error_flags) != 0;
             }
-            if (__shfl_sync(kFullMask, expired, 0)) {
-                timed_out = true;
-                sum = 0;
-                return false;
-            }
+            if (__shfl_sync(kFullMask, expired, 0)) return false;
         }
-        if (polls > SPIN) {
+        if (polls > 64) {
             __nanosleep(backoff);
             backoff = backoff < 1024 ? backoff * 2 : 1024;
         }
     }
+    return true;
 }
 
-// Publishes tile t's aggregate, resolves its exclusive prefix (carry_in for
-// tile 0) and publishes its inclusive prefix; returns the prefix to every
-// thread. `total` is the tile's sum, known to every thread. Warp 0 looks
-// back; a barrier hands its result to the CTA.
-template <typename T>
-__device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint64_t tag, T total, LookbackSmem& sm,
-                                             T* s_pre) {
-    ptx::u64x2* d1 = static_cast<ptx::u64x2*>(a.desc);
-    ptx::u64x2* d2 = static_cast<ptx::u64x2*>(a.group_desc);
-    const uint32_t s1 = a.desc_stride;
-    const T carry = a.carry_in != nullptr ? *static_cast<const T*>(a.carry_in) : T(0);
-    const uint32_t tid = threadIdx.x;
-    const uint32_t g = t / kGroupTiles;
-    const bool group_last = (t % kGroupTiles) == kGroupTiles - 1;
-    if (t == 0) {
-        if (tid == 0) {
-            if (a.num_tiles > 1)
-                ptx::st_relaxed_b128(d1, MidDesc::pack(kInclusive, tag, static_cast<uint64_t>(carry + total)));
-            else if (a.carry_out != nullptr)
-                *static_cast<T*>(a.carry_out) = carry + total;
-        }
+// Publishes tile t's sum `total`, known to every thread, and returns the
+// prefix before it (with carry_in) to every thread. sm.set and a cleared
+// sm.timeout are there already; `tag` is known to warp 0, `used` (the launches
+// that have used the group sums) to thread 0. GROUPS = false: one group.
+template <typename T, bool GROUPS>
+__device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint64_t tag, uint64_t used, T total,
+                                             LookbackSmem<T>& sm) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t g = t / kGroupTiles, i = t % kGroupTiles;
+    const bool last = t == a.num_tiles - 1;
+    T carry = 0;
+    if (a.carry_in != nullptr && t == 0) carry = *static_cast<const T*>(a.carry_in);
+    if (a.num_tiles == 1) {
+        if (tid == 0 && a.carry_out != nullptr) *static_cast<T*>(a.carry_out) = carry + total;
         return carry;
     }
-    if (tid < 32) {
-        const uint32_t lane = tid;
-        if (lane == 0)
-            ptx::st_relaxed_b128(d1 + t * s1, MidDesc::pack(kAggregate, tag, static_cast<uint64_t>(total)));
-        // The tiles of this group before t; tile 0 is inclusive, so group 0
-        // always finds one.
-        T in_sum;
-        bool timed_out;
-        const bool found = warp_window<T>(a, d1, s1, static_cast<int64_t>(t) - 1,
-                                          static_cast<int64_t>(g) * kGroupTiles, tag, lane, in_sum, timed_out);
-        if (lane == 0 && group_last && !timed_out)
-            ptx::st_relaxed_b128(d2 + g * kMidDescStride, MidDesc::pack(found ? kInclusive : kAggregate, tag,
-                                                       static_cast<uint64_t>(in_sum + total)));
-        // No inclusive tile in the group before t: the prefix of the group, a
-        // decoupled lookback over the group descriptors, 32 per poll.
-        T gsum = 0;
-        if (!found && !timed_out) {
-            int64_t top = static_cast<int64_t>(g) - 1;
-            while (true) {
-                T part;
-                const bool gf = warp_window<T>(a, d2, kMidDescStride, top, 0, tag, lane, part, timed_out);
-                if (timed_out) break;
-                gsum += part;
-                if (gf || top < 32) break;  // group 0's descriptor is inclusive
-                top -= 32;
+    char* sums = GROUPS ? static_cast<char*>(a.group_desc) + sm.set * (kMidSums * 128u) : nullptr;
+    if (warp == 0 || (GROUPS && warp * 32 < g)) {
+        ptx::u64x2* desc = static_cast<ptx::u64x2*>(a.desc);
+        if (tid == 0 && !last) {
+            const uint64_t own = static_cast<uint64_t>(static_cast<T>(carry + total));
+            if (i != kGroupTiles - 1)
+                ptx::st_relaxed_b128(desc + t * a.desc_stride, MidDesc::pack(kAggregate, tag, own));
+            if (GROUPS && (g + 1) * kGroupTiles < a.num_tiles) {
+                uint64_t* s = reinterpret_cast<uint64_t*>(sums + g * 128u);
+                ptx::red_add_u64(s, kOneTile + static_cast<uint32_t>(own));
+                if (sizeof(T) == 8) ptx::red_add_u64(s + 1, kOneTile + (own >> 32));
             }
         }
+        T x = 0;
+        bool tile_in = warp != 0 || lane >= i, group_in = !GROUPS || tid >= g;
+        const bool ok = mid_poll(a, lane, [&]() {
+            // Both loads are issued before the first is looked at.
+            ptx::u64x2 w{0, 0}, v{0, 0};
+            if (!tile_in) w = ptx::ld_relaxed_b128(desc + (t - i + lane) * a.desc_stride);
+            if (!group_in) {
+                if (sizeof(T) == 8)
+                    v = ptx::ld_relaxed_b128(reinterpret_cast<const ptx::u64x2*>(sums + tid * 128u));
+                else
+                    v.lo = ptx::ld_relaxed_u64(reinterpret_cast<const uint64_t*>(sums + tid * 128u));
+            }
+            if (!tile_in && MidDesc::status(w, tag) != kNotReady) {
+                tile_in = true;
+                x += static_cast<T>(w.lo);
+            }
+            if (!group_in && v.lo >= kGroupTiles * kOneTile && (sizeof(T) == 4 || v.hi >= kGroupTiles * kOneTile)) {
+                group_in = true;
+                x += static_cast<T>(v.lo & (kOneTile - 1)) + (sizeof(T) == 8 ? static_cast<T>(v.hi << 32) : T(0));
+            }
+            return tile_in && group_in;
+        });
+        x = warp_sum(x);
         if (lane == 0) {
-            if (t == a.num_tiles - 1 && !timed_out) ptx::st_relaxed_u64(a.mid_launch, tag + 1);
-            s_pre[0] = in_sum + gsum;
-            sm.timeout = timed_out ? 1u : 0u;
-            sm.found = found ? 1u : 0u;
+            sm.part[warp] = x;
+            if (!ok) sm.timeout = 1u;
         }
+    }
+    // The other set is used next: by the launch after this one.
+    if (GROUPS && t == 0 && tid >= kMidThreads - kMidSums) {
+        char* other = static_cast<char*>(a.group_desc) + (1u - sm.set) * (kMidSums * 128u);
+        *reinterpret_cast<ptx::u64x2*>(other + (tid - (kMidThreads - kMidSums)) * 128u) = ptx::u64x2{0, 0};
     }
     __syncthreads();
     if (sm.timeout != 0) {
         if (tid == 0) raise_error(a.hdr, kErrLookbackTimeout);
         return T(0);
     }
-    const T pre = s_pre[0];
-    if (tid == 0) {
-        ptx::st_relaxed_b128(d1 + t * s1, MidDesc::pack(kInclusive, tag, static_cast<uint64_t>(pre + total)));
-        if (group_last && sm.found == 0)
-            ptx::st_relaxed_b128(d2 + g * kMidDescStride, MidDesc::pack(kInclusive, tag, static_cast<uint64_t>(pre + total)));
-        if (a.carry_out != nullptr && t == a.num_tiles - 1) *static_cast<T*>(a.carry_out) = pre + total;
+    T pre = carry + sm.part[0];
+#pragma unroll
+    for (uint32_t w = 1; w < kGroupWarps; ++w)
+        if (GROUPS && w * 32 < g) pre += sm.part[w];
+    if (last && tid == 0) {
+        ptx::st_relaxed_u64(a.mid_launch, tag + 1);
+        if (GROUPS) ptx::st_relaxed_u64(&a.hdr->sums_launch, used + 1);
+        if (a.carry_out != nullptr) *static_cast<T*>(a.carry_out) = pre + total;
     }
     return pre;
 }
@@ -231,7 +223,11 @@ __device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint
 // output: 21.3 us a call, where per-thread element loads and stores (64
 // bytes apart across a warp) took 70.9; the generic kernel, which is ahead from
 // about there on, 20.2.
-template <typename T, bool INCL, bool ALIGNED, int HELD>
+//
+// GROUPS = false is for launches of one group of tiles, where the code for the
+// group sums costs fetches though it is not run (32 captured scans of 2^16 with it
+// 84-92 us, without 72-84, by where the plan's memory lies).
+template <typename T, bool INCL, bool ALIGNED, int HELD, bool GROUPS>
 __global__ void __launch_bounds__(kMidThreads, HELD ? HELD : kMidCtasPerSm) mid_vec_kernel(const ScanArgs a) {
     using Rows = TileRows<T, ALIGNED>;
     constexpr int EPC = Rows::kEpc;
@@ -240,8 +236,7 @@ __global__ void __launch_bounds__(kMidThreads, HELD ? HELD : kMidCtasPerSm) mid_
     static_assert(ROWS * WARPS == 32, "one warp scans all (row, warp) totals");
     __shared__ T s_tot[ROWS * WARPS];
     __shared__ T s_off[ROWS][kMidThreads];  // chunk offsets, kept here across the lookback
-    __shared__ LookbackSmem lsm;
-    __shared__ T s_pre[1];
+    __shared__ LookbackSmem<T> lsm;
 
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31u;
@@ -255,6 +250,7 @@ __global__ void __launch_bounds__(kMidThreads, HELD ? HELD : kMidCtasPerSm) mid_
     ptx::grid_dep_wait();
     // Only warp 0 uses the launch number; its load overlaps the tile's.
     const uint64_t tag = threadIdx.x < 32 ? ptx::ld_relaxed_u64(a.mid_launch) : 0;
+    const uint64_t used = GROUPS && threadIdx.x == 0 ? ptx::ld_relaxed_u64(&a.hdr->sums_launch) : 0;
     const Rows rows(a.in, a.out, a.n, t, tid);
     constexpr PlainAccess access;
 
@@ -284,6 +280,10 @@ __global__ void __launch_bounds__(kMidThreads, HELD ? HELD : kMidCtasPerSm) mid_
         cs[r] = gps_device::warp_exclusive_scan<gps_device::WarpAlgo::KoggeStone>(cs[r], gps_device::Plus(), &wt);
         if (lane == 0) s_tot[r * WARPS + warp] = wt;
     }
+    if (tid == 0) {
+        if (GROUPS) lsm.set = static_cast<uint32_t>(used & 1u);
+        lsm.timeout = 0u;
+    }
     __syncthreads();
     T total;
     {
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(kMidThreads, HELD ? HELD : kMidCtasPerSm) mid_
         for (int r = 0; r < ROWS; ++r) s_off[r][tid] = cs[r] + __shfl_sync(kFullMask, xe, r * WARPS + warp);
     }
 
-    const T base = mid_tile_prefix<T>(a, t, tag, total, lsm, s_pre);
+    const T base = mid_tile_prefix<T, GROUPS>(a, t, tag, used, total, lsm);
 
     auto scan_chunk = [&](int r, Chunk<T>& q) {
         T acc = base + s_off[r][tid];
@@ -338,23 +338,38 @@ __global__ void __launch_bounds__(kMidThreads, HELD ? HELD : kMidCtasPerSm) mid_
 
 template <typename T, bool INCL, bool ALIGNED>
 cudaError_t launch_mid_v(const ScanArgs& a0, int num_sms, cudaStream_t stream, LaunchInfo* info) {
+    using Rows = TileRows<T, ALIGNED>;
     ScanArgs a = a0;
-    // At most one more than the plan's (its descriptor regions have kDescPad
-    // to spare).
-    a.num_tiles = TileRows<T, ALIGNED>::tiles(a.in, a.n);
-    a.desc_stride = a.num_tiles > kGroupTiles && a.num_tiles <= kMidStrideMaxTiles ? kMidDescStride : 1u;
-    const int grid = static_cast<int>(a.num_tiles);
-    if (info) *info = LaunchInfo{grid, kMidThreads, 0};
-    // A dependent launch sets its CTAs up while the kernel ahead finishes: a
-    // program that scans one small array after another waits for one launch
-    // less each time (2^20 u32: 6.3 -> 5.5 us a call, 32 captured scans of 2^16:
-    // 102 -> 89 us).
-    // The forms that hold their tile, while the launch is one wave of them.
-    if (a.num_tiles <= static_cast<uint32_t>(4 * num_sms))
-        return launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, 4>, grid, kMidThreads, 0, stream, a);
-    if (a.num_tiles <= static_cast<uint32_t>(6 * num_sms))
-        return launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, 6>, grid, kMidThreads, 0, stream, a);
-    return launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, 0>, grid, kMidThreads, 0, stream, a);
+    // Scans of more tiles than there are group sums for run in pieces, each with
+    // the sum through the piece before as its carry.
+    char* carries = static_cast<char*>(a0.group_desc) + 2 * 128 * kMidSums;
+    if (info) *info = LaunchInfo{static_cast<int>(Rows::tiles(a0.in, a0.n)), kMidThreads, 0};
+    for (uint64_t done = 0, piece = 0; done < a0.n; done += a.n, ++piece) {
+        a.in = static_cast<const T*>(a0.in) + done;
+        a.out = static_cast<T*>(a0.out) + done;
+        const uint64_t most = static_cast<uint64_t>(kMidMaxTiles) * Rows::kTile - Rows::lead_of(a.in);
+        a.n = a0.n - done < most ? a0.n - done : most;
+        a.carry_in = piece == 0 ? a0.carry_in : carries + (piece & 1) * 16;
+        a.carry_out = done + a.n == a0.n ? a0.carry_out : carries + ((piece + 1) & 1) * 16;
+        a.num_tiles = Rows::tiles(a.in, a.n);
+        a.desc_stride = a.num_tiles > kGroupTiles ? kMidDescStride : 1u;
+        const int grid = static_cast<int>(a.num_tiles);
+        // A dependent launch sets its CTAs up while the kernel ahead finishes: a
+        // program that scans one small array after another waits for one launch
+        // less each time (2^20 u32: 6.3 -> 5.5 us a call, 32 captured scans of 2^16:
+        // 102 -> 89 us).
+        // The forms that hold their tile, while the launch is one wave of them.
+        const cudaError_t err =
+            a.num_tiles <= kGroupTiles
+                ? launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, 4, false>, grid, kMidThreads, 0, stream, a)
+            : a.num_tiles <= static_cast<uint32_t>(4 * num_sms)
+                ? launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, 4, true>, grid, kMidThreads, 0, stream, a)
+            : a.num_tiles <= static_cast<uint32_t>(6 * num_sms)
+                ? launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, 6, true>, grid, kMidThreads, 0, stream, a)
+                : launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, 0, true>, grid, kMidThreads, 0, stream, a);
+        if (err != cudaSuccess) return err;
+    }
+    return cudaSuccess;
 }
 
 template <typename T, bool INCL>
