@@ -451,8 +451,8 @@ def run_sweep(stream, d_in, d_out):
     second power of two) on the benchmark's buffers, beside CUB DeviceScan on
     the same buffers, and u64 at n = 2^27. GPU time per scan from CUDA-graph
     replay. Inputs below about 2^24 elements stay in L2 between launches.
-    The plan's defaults pick the kernel: one tile per CTA up to 38 MB (28 MB
-    of u64), the persistent generic kernel above."""
+    The plan's defaults pick the kernel: one tile per CTA up to 38 MB, the
+    persistent generic kernel above."""
     import torch
 
     from gpuprefixsums_gb300 import Plan

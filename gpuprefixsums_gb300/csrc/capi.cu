@@ -196,8 +196,7 @@ gps_status launch_scan(gps_plan_s* p, bool inclusive, const void* in, void* out,
     // Buffers off a 16-byte boundary take the same kernels as others, but where the
     // generic one does not apply: csdl.cu's for them moves single elements, so one tile per
     // CTA takes every size that is left (2^27 u32 elements: 258 against 2017 us;
-    // generic kernel 160). One limit serves both: at 9.5 M u32 off a boundary one tile
-    // per CTA takes 19.5 us and the generic kernel 19.1, at 2.5 M u64 13.4 and 14.0.
+    // generic kernel 160). One limit serves both (mid_max_bytes()).
     const bool unaligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) != 0;
     cudaError_t err;
     if (generic_only(p->dtype)) {
@@ -320,7 +319,7 @@ gps_status gps_plan_create(gps_plan* out_plan, gps_algo algo, gps_dtype dtype, u
     // 2.7 against 4.5 us at 16384 u32). Reduce-then-scan plans keep the
     // one-CTA kernel for small inputs.
     p->small_max = algo == GPS_ALGO_CSDL ? 0 : gps::small_scan_max_elems(dtype);
-    p->mid_max = algo == GPS_ALGO_CSDL && !generic_only(dtype) ? gps::mid_max_bytes(dtype) / gps::dtype_size(dtype) : 0;
+    p->mid_max = algo == GPS_ALGO_CSDL && !generic_only(dtype) ? gps::mid_max_bytes() / gps::dtype_size(dtype) : 0;
     cudaError_t err = cudaGetDevice(&p->device);
     if (err == cudaSuccess) err = cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device);
     if (err != cudaSuccess) {

@@ -247,11 +247,12 @@ uint64_t small_scan_max_elems(gps_dtype dtype);
 cudaError_t launch_small(gps_dtype dtype, bool inclusive, const ScanArgs& a, cudaStream_t stream, LaunchInfo* info);
 
 // Integer chained scans up to mid size, one 16 KB tile per CTA (mid.cu); the
-// default upper size of a plan, in bytes of input. Measured on GB300 (graph
-// replay) against the persistent kernel that takes over (the generic one):
-// u32 2^22 8.4 against 13.7 us, 2^23 15.3 / 17.7, 2320 tiles 17.0 / 19.1, 2560 19.8 /
-// 19.0, 2^24 30.9 / 26; u64 1700 tiles 14.3 / 15.9, 2048 16.2 / 15.9.
-constexpr size_t mid_max_bytes(gps_dtype dtype) { return dtype == GPS_DTYPE_U64 ? 28ull << 20 : 38ull << 20; }
+// default upper size of a plan: two waves of 8 CTAs per SM (2432 tiles) and a few
+// more. Measured on GB300 (graph replay, us) against the persistent kernel that takes
+// over (the generic one): u32 9.96 M elements 16.7 / 18.3, 10.1 M 17.8 / 18.3, 10.2 M 18.2 /
+// 18.2, 10.4 M 19.0 / 18.4, 2^24 29.2 / 25.6; off a 16-byte boundary 9.96 M 18.9 / 19.7, 10.1 M
+// 20.3 / 19.7; u64 4.9 M 17.5 / 18.0, 5.02 M 17.6 / 18.1, 5.06 M 18.4 / 18.1.
+constexpr size_t mid_max_bytes() { return 153ull << 18; }
 // Tile descriptors of the one-tile-per-CTA kernels sit one per 128-byte line
 // (a stride of 8 words) when a launch has more than one group of 32 tiles, else
 // packed. Sharing lines between

@@ -253,7 +253,7 @@ gps_status gps_plan_set_fallback(gps_plan plan, uint32_t fallback_polls);
 gps_status gps_plan_set_small_max(gps_plan plan, uint64_t max_n);
 
 /* Integer scans on a GPS_ALGO_CSDL plan above the one-CTA size and of at
- * most max_n elements (default: 38 MB of u32 or 28 MB of u64) run
+ * most max_n elements (default: 38.25 MB) run
  * as one 16 KB tile per CTA -- a single-pass chained scan without
  * the persistent kernels' pipeline, whose latency dominates at these sizes;
  * larger ones run on a persistent L2-buffered kernel. 0 sends them all to

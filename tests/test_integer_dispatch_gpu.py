@@ -32,7 +32,7 @@ def _check(plan, dtype, n, inclusive):
 def test_sizes_where_the_kernel_changes(cuda, dtype, inclusive):
     es = np.dtype(NP[dtype]).itemsize
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    mid = ((38 if dtype == "u32" else 28) << 20) // es
+    mid = (153 << 18) // es
     units = 8 * sms * 16384 // es  # with mid_max 0: fewest tiles the generic kernel takes
     with Plan("csdl", dtype, max_n=mid + 4096) as plan:
         for n in (mid - 1, mid, mid + 1, mid + 4096):
