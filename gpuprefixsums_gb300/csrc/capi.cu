@@ -67,7 +67,7 @@ struct gps_plan_s {
     // latter; else null.
     void* desc_mid;
     void* group_desc_mid;
-    void* group_sums;  // integer chained-scan plans: the group sums of mid.cu
+    void* group_sums;  // chained-scan plans: the group sums of mid_lookback.cuh
     // Integer scans of at most this many elements run in one CTA (small.cu).
     uint64_t small_max;
     uint64_t mid_max;  // chained-scan plans: largest scan run as one tile per CTA
@@ -357,7 +357,7 @@ gps_status gps_plan_create(gps_plan* out_plan, gps_algo algo, gps_dtype dtype, u
     const uint64_t words_mid = slots_mid ? gps::mid_desc_words(tiles_mid) : 0;
     const size_t end_mid = slots_mid ? region_mid + (words_mid + groups_mid * gps::kMidDescStride) * 16 : end16;
     const size_t region_sums = (end_mid + 255) & ~static_cast<size_t>(255);
-    const bool sums = algo == GPS_ALGO_CSDL && !generic_only(dtype);
+    const bool sums = algo == GPS_ALGO_CSDL;
     p->scratch_bytes = sums ? region_sums + kSumsBytes : end_mid;
     err = cudaMalloc(&p->scratch, p->scratch_bytes);
     if (err != cudaSuccess) {
@@ -654,7 +654,7 @@ gps_status gps_select_flagged(gps_plan p, const void* d_in, const uint8_t* d_fla
     a.hdr = p->hdr16;
     const bool mid = a.num_tiles <= gps::kMidSelectMaxTiles;
     a.desc = mid ? p->desc_mid : p->desc16;
-    a.group_desc = p->group_desc_mid;
+    a.group_desc = p->group_sums;
     a.mid_launch = &p->hdr->mid_launch;
     a.carry_out = d_num_selected;
     a.wait_budget_ns = p->wait_budget_ns;

@@ -48,7 +48,7 @@ struct alignas(128) WsHeader {
     unsigned long long stat_inserts;    // fallback aggregates that won the CAS
     unsigned long long stat_stalls;     // tiles that were made to stall
     uint64_t mid_launch;                // launch number of the one-tile-per-CTA kernels
-    uint64_t sums_launch;               // how many of them used the group sums (mid.cu)
+    uint64_t sums_launch;               // how many of them used the group sums: at mid_launch + 1
 };
 static_assert(sizeof(WsHeader) == 128, "header is one 128-byte line");
 

@@ -31,6 +31,7 @@
 // instead of 256: 260 us (6.4 TB/s, 0.96 of the copy rate), 80% selected 330, 2^24
 // 25.5 against 27.1.
 #include "launch_util.h"
+#include "mid_lookback.cuh"
 #include "mid_seg.cuh"
 
 namespace gps {
@@ -536,16 +537,18 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
 // persistent kernel's pipeline takes 9 us whatever the size, and its units of
 // 4 tiles leave most SMs idle below 600 tiles. Flags and values are loaded
 // together; each thread turns the flags of its 64 bytes of values into a mask,
-// the block scans the counts, and while warp 0 publishes the tile's count and
-// folds the counts before it (mid_seg.cuh's fixed-order lookback), the values
-// are compacted in shared memory. Then the run goes out, coalesced.
-// Latency bounds it: one HBM read, two L2 round trips, a store. Measured on
+// the block scans the counts, the tile's count is published, and while others
+// publish theirs the values are compacted in shared memory; then come the counts before
+// (mid_lookback.cuh, in 32 bits), and the run goes out, coalesced.
+// Latency bounds it: one HBM read, one L2 round trip, a store (with mid_seg.cuh's
+// lookback, two: 2^20 u32 4.8 against 4.0 us, 2^22 8.8 / 8.2, 2^23 15.6 / 14.5; 2^20 u64 5.45 / 4.8).
+// Measured with that on
 // GB300, graph replay, u32, 30% selected, against the persistent kernel:
 // 2^16 elements 2.7 against 7.1 us, 2^20 5.6 / 8.8, 2^22 11.4 / 14.2, 2^23 17.9 /
 // 19.0 (90% selected: 21.0 / 24.0), 2^24 32.3 / 28.4.
 constexpr int kMidSelThreads = kMidSegThreads;
 
-template <typename V, int CTAS>
+template <typename V, int CTAS, bool GROUPS>
 __global__ void __launch_bounds__(kMidSelThreads, CTAS) mid_select_kernel(const ScanArgs a, const SelArgs sa) {
     constexpr int TILE = 16384 / static_cast<int>(sizeof(V));
     constexpr int EPC = 16 / static_cast<int>(sizeof(V));
@@ -554,9 +557,10 @@ __global__ void __launch_bounds__(kMidSelThreads, CTAS) mid_select_kernel(const 
     constexpr int WARPS = kMidSelThreads / 32;
     constexpr int FW = ITEMS / 4;  // flag words per thread
     static_assert(ITEMS == CHUNKS * EPC, "four chunks a thread");
+    static_assert(kMidSelectMaxTiles <= kMidMaxTiles && kMidSelectMaxTiles * 4096ull < (1ull << 32), "32-bit counts");
     __shared__ __align__(16) Chunk<V> s_tile[CHUNKS * kMidSelThreads];
     __shared__ uint32_t s_wtot[WARPS];
-    __shared__ uint64_t s_pre;
+    __shared__ LookbackSmem<uint32_t> lsm;
 
     const uint32_t tid = threadIdx.x;
     const uint32_t lane = tid & 31u;
@@ -571,6 +575,7 @@ __global__ void __launch_bounds__(kMidSelThreads, CTAS) mid_select_kernel(const 
     ptx::grid_dep_launch();
     ptx::grid_dep_wait();
     const uint64_t tag = threadIdx.x < 32 ? ptx::ld_relaxed_u64(a.mid_launch) : 0;
+    const uint64_t used = GROUPS && threadIdx.x == 0 ? ptx::ld_relaxed_u64(a.mid_launch + 1) : 0;
     const uint64_t t0 = static_cast<uint64_t>(t) * TILE;
     const uint32_t cnt = static_cast<uint32_t>(min(static_cast<uint64_t>(TILE), a.n - t0));
     auto slot = [](uint32_t c) -> uint32_t { return c ^ ((c >> 3) & 3u); };
@@ -611,6 +616,10 @@ __global__ void __launch_bounds__(kMidSelThreads, CTAS) mid_select_kernel(const 
     const uint32_t mine = static_cast<uint32_t>(__popc(mask));
     const uint32_t inc = warp_inclusive_scan(mine, lane);
     if (lane == 31) s_wtot[warp] = inc;
+    if (tid == 0) {
+        lsm.set = static_cast<uint32_t>(used & 1u);
+        lsm.timeout = 0u;
+    }
 #pragma unroll
     for (int r = 0; r < CHUNKS; ++r) s_tile[slot(r * kMidSelThreads + tid)] = q[r];
     __syncthreads();
@@ -621,6 +630,7 @@ __global__ void __launch_bounds__(kMidSelThreads, CTAS) mid_select_kernel(const 
         before += static_cast<uint32_t>(k) < warp ? x : 0u;
         total += x;
     }
+    if (tid == 0 && a.num_tiles > 1) mid_publish<uint32_t, GROUPS>(a, t, tag, total, lsm);
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) q[c] = s_tile[slot(tid * CHUNKS + c)];
     __syncthreads();
@@ -634,19 +644,14 @@ __global__ void __launch_bounds__(kMidSelThreads, CTAS) mid_select_kernel(const 
         for (int e = 0; e < EPC; ++e)
             if ((mask >> (c * EPC + e)) & 1u) run[pos++] = q[c].v[e];
 
-    if (warp == 0) {
-        uint64_t pre = 0;
-        const bool last = t == a.num_tiles - 1;
-        const bool ok = a.num_tiles == 1 || mid_seg_prefix<OpU64>(a, t, tag, total, false, lane, pre);
-        if (lane == 0) {
-            if (!ok) raise_error(a.hdr, kErrLookbackTimeout);
-            if (last) *static_cast<uint64_t*>(a.carry_out) = pre + total;
-            s_pre = ok ? pre : ~0ull;
-        }
-    }
-    __syncthreads();
-    if (s_pre == ~0ull) return;
-    V* out = static_cast<V*>(a.out) + s_pre;
+    uint32_t pre = 0;
+    if (a.num_tiles > 1)
+        pre = mid_tile_prefix<uint32_t, GROUPS>(a, t, tag, used, lsm);
+    else
+        __syncthreads();
+    if (lsm.timeout != 0) return;
+    if (tid == 0 && t == a.num_tiles - 1) *static_cast<uint64_t*>(a.carry_out) = static_cast<uint64_t>(pre) + total;
+    V* out = static_cast<V*>(a.out) + pre;
     for (uint32_t i = tid; i < total; i += kMidSelThreads) out[i] = run[i];
 }
 
@@ -657,11 +662,13 @@ cudaError_t launch_mid_select(const ScanArgs& a0, const SelArgs& sa, int num_sms
     a.desc_stride = a.num_tiles > 32 ? kMidDescStride : 1u;
     const int grid = static_cast<int>(a.num_tiles);
     if (info) *info = LaunchInfo{grid, kMidSelThreads, 0};
+    if (a.num_tiles <= kGroupTiles)
+        return launch_dependent(mid_select_kernel<V, 4, false>, grid, kMidSelThreads, 0, stream, a, sa);
     switch (mid_seg_ctas(a.num_tiles, num_sms, 8)) {
-        case 4: return launch_dependent(mid_select_kernel<V, 4>, grid, kMidSelThreads, 0, stream, a, sa);
-        case 6: return launch_dependent(mid_select_kernel<V, 6>, grid, kMidSelThreads, 0, stream, a, sa);
+        case 4: return launch_dependent(mid_select_kernel<V, 4, true>, grid, kMidSelThreads, 0, stream, a, sa);
+        case 6: return launch_dependent(mid_select_kernel<V, 6, true>, grid, kMidSelThreads, 0, stream, a, sa);
     }
-    return launch_dependent(mid_select_kernel<V, 8>, grid, kMidSelThreads, 0, stream, a, sa);
+    return launch_dependent(mid_select_kernel<V, 8, true>, grid, kMidSelThreads, 0, stream, a, sa);
 }
 
 template <typename V>
