@@ -42,15 +42,23 @@ struct alignas(128) WsHeader {
     uint32_t exit_counter;
     uint32_t epoch;
     uint32_t error_flags;
+    // One-tile-per-CTA kernels: their launch number and how many of the launches
+    // used the group sums, read by one 16-byte load. A CTA publishes only what rests
+    // on that load, so none can still be about to read either word once the last
+    // tile, which has seen every other, advances them.
+    alignas(16) uint64_t mid_launch;
+    uint32_t sums_launch;  // mod 2^32: only its lowest bit counts
+    uint32_t pad_;
     unsigned long long capacity_tiles;  // descriptor slots that follow
     unsigned long long stat_polls;      // lookback windows re-polled (stats mode)
     unsigned long long stat_fallbacks;  // predecessor tiles re-reduced
     unsigned long long stat_inserts;    // fallback aggregates that won the CAS
     unsigned long long stat_stalls;     // tiles that were made to stall
-    uint64_t mid_launch;                // launch number of the one-tile-per-CTA kernels
-    uint64_t sums_launch;               // how many of them used the group sums: at mid_launch + 1
 };
 static_assert(sizeof(WsHeader) == 128, "header is one 128-byte line");
+static_assert(offsetof(WsHeader, mid_launch) % 16 == 0 &&
+                  offsetof(WsHeader, sums_launch) == offsetof(WsHeader, mid_launch) + 8,
+              "launch number and set count are one 16-byte word");
 
 // Forced-stall test mode (EmulatedDeadlocking-style).
 //  mode 0: off.
@@ -115,7 +123,7 @@ struct ScanArgs {
     void* carry_out;       // optional: receives carry_in + sum of all n inputs
     uint64_t wait_budget_ns;
     StallConfig stall;
-    uint64_t* mid_launch;  // one-tile-per-CTA kernels: WsHeader::mid_launch
+    uint64_t* mid_launch;  // one-tile-per-CTA kernels: WsHeader::mid_launch, sums_launch after it
     uint32_t units_in_flight;  // generic kernel: per CTA, set by its launcher
     // Generic kernel on buffers off a 16-byte boundary (its launcher sets them):
     // elements before the input in its first 16 bytes, and how many elements

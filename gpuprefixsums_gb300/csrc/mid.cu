@@ -89,8 +89,8 @@ __global__ void __launch_bounds__(kMidThreads, HELD ? HELD : kMidCtasPerSm) mid_
     ptx::grid_dep_launch();
     ptx::grid_dep_wait();
     // Only warp 0 uses the launch number; its load overlaps the tile's.
-    const uint64_t tag = threadIdx.x < 32 ? ptx::ld_relaxed_u64(a.mid_launch) : 0;
-    const uint64_t used = GROUPS && threadIdx.x == 0 ? ptx::ld_relaxed_u64(a.mid_launch + 1) : 0;
+    const ptx::u64x2 launch = mid_launch_state(a);
+    const uint64_t tag = launch.lo;
     const Rows rows(a.in, a.out, a.n, t, tid);
     constexpr PlainAccess access;
 
@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kMidThreads, HELD ? HELD : kMidCtasPerSm) mid_
         if (lane == 0) s_tot[r * WARPS + warp] = wt;
     }
     if (tid == 0) {
-        if (GROUPS) lsm.set = static_cast<uint32_t>(used & 1u);
+        if (GROUPS) lsm.used = static_cast<uint32_t>(launch.hi);
         lsm.timeout = 0u;
     }
     __syncthreads();
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(kMidThreads, HELD ? HELD : kMidCtasPerSm) mid_
     T base = carry;
     if (a.num_tiles > 1) {
         if (tid == 0) mid_publish<T, GROUPS>(a, t, tag, carry + total, lsm);
-        base += mid_tile_prefix<T, GROUPS>(a, t, tag, used, lsm);
+        base += mid_tile_prefix<T, GROUPS>(a, t, tag, lsm);
     }
     if (a.carry_out != nullptr && tid == 0 && t == a.num_tiles - 1) *static_cast<T*>(a.carry_out) = base + total;
 

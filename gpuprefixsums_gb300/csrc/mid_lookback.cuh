@@ -37,9 +37,10 @@ struct MidDesc {
 //
 // The group sums have two sets, which the launches that use them take in turn,
 // counted in the plan's header; tile 0's CTA clears the other set for the next.
-// Warp 0 hands that count to the CTA through shared memory, so that it has been
-// read before the CTA publishes anything, and the last tile's CTA, which has
-// then seen every tile, advances it.
+// Warp 0 reads the launch number and that count in one load and hands the count
+// to the CTA through shared memory. Everything a tile publishes depends on that
+// load (a descriptor on the number, a group sum on the count, by its address), so
+// the last tile's CTA, which has then seen every tile, can advance both.
 //
 // Measured on GB300, graph replay, inputs from HBM, u32, against two levels in turn
 // (the last tile of a group reads the group's descriptors and publishes their sum, which
@@ -57,9 +58,15 @@ static_assert(kGroupTiles * kMidSums == kMidMaxTiles, "one sum per group");
 template <typename T>
 struct LookbackSmem {
     T part[kGroupWarps];  // what each polling warp has found
-    uint32_t set;             // which set of group sums this launch uses
-    uint32_t timeout;         // a wait ran past its budget
+    uint32_t used;        // launches that have used the group sums: even ones use one set, odd ones the other
+    uint32_t timeout;     // a wait ran past its budget
 };
+
+// By all threads; warp 0's get {launch number, launches that have used the group sums}.
+__device__ __forceinline__ ptx::u64x2 mid_launch_state(const ScanArgs& a) {
+    return threadIdx.x < 32 ? ptx::ld_relaxed_b128(reinterpret_cast<const ptx::u64x2*>(a.mid_launch))
+                            : ptx::u64x2{0, 0};
+}
 
 // Polls until `done` holds for every lane of the warp, calling look() each
 // time; false once the wait budget has run out.
@@ -88,7 +95,7 @@ __device__ __forceinline__ bool mid_poll(const ScanArgs& a, uint32_t lane, Look 
 
 template <typename T, bool GROUPS>
 __device__ __forceinline__ char* mid_sums(const ScanArgs& a, const LookbackSmem<T>& sm) {
-    return GROUPS ? static_cast<char*>(a.group_desc) + sm.set * (kMidSums * 128u) : nullptr;
+    return GROUPS ? static_cast<char*>(a.group_desc) + (sm.used & 1u) * (kMidSums * 128u) : nullptr;
 }
 
 // By thread 0: publishes tile t's sum `own` (tile 0's with the carry).
@@ -110,11 +117,9 @@ __device__ __forceinline__ void mid_publish(const ScanArgs& a, uint32_t t, uint6
 
 // Returns the sum of the tiles before t, of a launch of more than one, to every
 // thread, after its own has been published; sm.timeout is set if a wait ran out.
-// `tag` is known to warp 0, `used` (the launches that have used the group
-// sums) to thread 0; sm.set and a cleared sm.timeout are there already.
+// `tag` is known to warp 0; sm.used and a cleared sm.timeout are there already.
 template <typename T, bool GROUPS>
-__device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint64_t tag, uint64_t used,
-                                             LookbackSmem<T>& sm) {
+__device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint64_t tag, LookbackSmem<T>& sm) {
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t g = t / kGroupTiles, i = t % kGroupTiles;
     const bool last = t == a.num_tiles - 1;
@@ -151,7 +156,7 @@ __device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint
     }
     // The other set is used next: by the launch after this one.
     if (GROUPS && t == 0 && tid >= kRowThreads - kMidSums) {
-        char* other = static_cast<char*>(a.group_desc) + (1u - sm.set) * (kMidSums * 128u);
+        char* other = static_cast<char*>(a.group_desc) + ((sm.used & 1u) ^ 1u) * (kMidSums * 128u);
         *reinterpret_cast<ptx::u64x2*>(other + (tid - (kRowThreads - kMidSums)) * 128u) = ptx::u64x2{0, 0};
     }
     __syncthreads();
@@ -165,7 +170,7 @@ __device__ __forceinline__ T mid_tile_prefix(const ScanArgs& a, uint32_t t, uint
         if (GROUPS && w * 32 < g) pre += sm.part[w];
     if (last && tid == 0) {
         ptx::st_relaxed_u64(a.mid_launch, tag + 1);
-        if (GROUPS) ptx::st_relaxed_u64(a.mid_launch + 1, used + 1);
+        if (GROUPS) ptx::st_relaxed_u32(reinterpret_cast<uint32_t*>(a.mid_launch + 1), sm.used + 1);
     }
     return pre;
 }

@@ -574,8 +574,8 @@ __global__ void __launch_bounds__(kMidSelThreads, CTAS) mid_select_kernel(const 
     }
     ptx::grid_dep_launch();
     ptx::grid_dep_wait();
-    const uint64_t tag = threadIdx.x < 32 ? ptx::ld_relaxed_u64(a.mid_launch) : 0;
-    const uint64_t used = GROUPS && threadIdx.x == 0 ? ptx::ld_relaxed_u64(a.mid_launch + 1) : 0;
+    const ptx::u64x2 launch = mid_launch_state(a);
+    const uint64_t tag = launch.lo;
     const uint64_t t0 = static_cast<uint64_t>(t) * TILE;
     const uint32_t cnt = static_cast<uint32_t>(min(static_cast<uint64_t>(TILE), a.n - t0));
     auto slot = [](uint32_t c) -> uint32_t { return c ^ ((c >> 3) & 3u); };
@@ -617,7 +617,7 @@ __global__ void __launch_bounds__(kMidSelThreads, CTAS) mid_select_kernel(const 
     const uint32_t inc = warp_inclusive_scan(mine, lane);
     if (lane == 31) s_wtot[warp] = inc;
     if (tid == 0) {
-        lsm.set = static_cast<uint32_t>(used & 1u);
+        lsm.used = static_cast<uint32_t>(launch.hi);
         lsm.timeout = 0u;
     }
 #pragma unroll
@@ -646,7 +646,7 @@ __global__ void __launch_bounds__(kMidSelThreads, CTAS) mid_select_kernel(const 
 
     uint32_t pre = 0;
     if (a.num_tiles > 1)
-        pre = mid_tile_prefix<uint32_t, GROUPS>(a, t, tag, used, lsm);
+        pre = mid_tile_prefix<uint32_t, GROUPS>(a, t, tag, lsm);
     else
         __syncthreads();
     if (lsm.timeout != 0) return;
