@@ -733,8 +733,9 @@ gps_status gps_plan_check(gps_plan p, gps_stream_t stream) {
     cudaError_t err = cudaStreamSynchronize(reinterpret_cast<cudaStream_t>(stream));
     if (err != cudaSuccess) return cuda_fail(err, "cudaStreamSynchronize");
     uint32_t all = 0;
-    for (gps::WsHeader* h : {p->hdr, p->hdr16}) {
-        if (h == p->hdr16 && h == p->hdr) break;
+    // The generic kernel has a header of its own on u32 chained-scan plans only.
+    for (gps::WsHeader* h : {p->hdr, p->hdr16 != p->hdr ? p->hdr16 : nullptr}) {
+        if (h == nullptr) break;
         uint32_t flags = 0;
         err = cudaMemcpy(&flags, &h->error_flags, sizeof(flags), cudaMemcpyDeviceToHost);
         if (err != cudaSuccess) return cuda_fail(err, "reading device error flags");
