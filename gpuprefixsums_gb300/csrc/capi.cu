@@ -52,7 +52,7 @@ struct gps_plan_s {
     gps::WsHeader* hdr;
     void* carries;        // two elements (host-array scans)
     void* area;
-    // Generic kernel (batched and floating-point scans): its workspace header
+    // Generic kernel with units (batched and floating-point scans): its workspace header
     // and 16-byte descriptors. On u32 chained-scan plans they are a region of
     // their own, with their own epoch, next to the 8-byte descriptors of the
     // u32 kernel; on other plans they are hdr and area.
@@ -63,8 +63,8 @@ struct gps_plan_s {
     // covers them).
     void* group_desc16;
     // Chained-scan plans: the 16-byte, launch-tagged descriptors of the
-    // one-tile-per-CTA kernels (mid.cu; mid_seg.cuh), and group descriptors of the
-    // latter; else null.
+    // one-tile-per-CTA kernels (mid.cu, mid_seg.cuh, small selects), and group descriptors
+    // of mid_seg.cuh; else null. Their header is hdr.
     void* desc_mid;
     void* group_desc_mid;
     void* group_sums;  // chained-scan plans: the group sums of mid_lookback.cuh
@@ -139,7 +139,7 @@ cudaError_t launch_generic(const gps_plan_s* p, bool inclusive, gps::ScanArgs a,
                            const gps::GenericConfig& cfg, cudaStream_t stream, gps::LaunchInfo* info,
                            bool unaligned = false) {
     const int num_sms = p->num_sms;
-    a.hdr = p->hdr16;
+    a.hdr = cfg.unit == 0 ? p->hdr : p->hdr16;
     a.mid_launch = &p->hdr->mid_launch;
     a.desc = cfg.unit == 0 ? p->desc_mid : p->desc16;
     a.group_desc = cfg.unit == 0 ? p->group_desc_mid : p->group_desc16;
@@ -651,8 +651,8 @@ gps_status gps_select_flagged(gps_plan p, const void* d_in, const uint8_t* d_fla
     a.out = d_out;
     a.n = n;
     a.num_tiles = static_cast<uint32_t>((n + gps::select_tile_elems(es) - 1) / gps::select_tile_elems(es));
-    a.hdr = p->hdr16;
     const bool mid = a.num_tiles <= gps::kMidSelectMaxTiles;
+    a.hdr = mid ? p->hdr : p->hdr16;
     a.desc = mid ? p->desc_mid : p->desc16;
     a.group_desc = p->group_sums;
     a.mid_launch = &p->hdr->mid_launch;
@@ -746,8 +746,8 @@ gps_status gps_plan_check(gps_plan p, gps_stream_t stream) {
         }
         all |= flags;
     }
-    // A wait that ran out may have left the launch number behind, or CTAs
-    // that read it late: skip past both.
+    // A wait that ran out may have left the launch number behind, with descriptors
+    // and half-filled group sums under it: go past it and clear the sums.
     if (all != 0 && p->algo == GPS_ALGO_CSDL) {
         uint64_t number = 0;
         err = cudaMemcpy(&number, &p->hdr->mid_launch, sizeof(number), cudaMemcpyDeviceToHost);

@@ -113,7 +113,11 @@ struct ScanArgs {
     // One-tile-per-CTA and generic kernels: 16-byte words from one descriptor
     // to the next (0: packed), set by their launchers.
     uint32_t desc_stride;
-    WsHeader* hdr;       // plan state (counters, epoch, error flags)
+    // Plan state (counters, epoch, error flags). Kernels that share descriptors share a
+    // header, the one-tile-per-CTA kernels the one with their launch number: after a wait
+    // that ran out the number may stay, and what one of them has published under it is not
+    // to be taken for another's.
+    WsHeader* hdr;
     void* desc;          // tile descriptors (lookback)
     // Descriptors of groups: of kMidSegGroup tiles for the one-tile-per-CTA form
     // of the generic kernel, of det_group_units() lookback units for the other. For

@@ -645,10 +645,15 @@ __global__ void __launch_bounds__(kMidSelThreads, CTAS) mid_select_kernel(const 
             if ((mask >> (c * EPC + e)) & 1u) run[pos++] = q[c].v[e];
 
     uint32_t pre = 0;
-    if (a.num_tiles > 1)
+    if (a.num_tiles > 1) {
+        // After a wait that ran out in a launch before (and has not been reported yet) the
+        // descriptors and sums under this launch's number may be other values than counts:
+        // nothing is written. (By a warp that does not poll, while others do.)
+        if (tid == kMidSelThreads - 32 && ld_volatile_u32(&a.hdr->error_flags) != 0) lsm.timeout = 1u;
         pre = mid_tile_prefix<uint32_t, GROUPS>(a, t, tag, lsm);
-    else
+    } else {
         __syncthreads();
+    }
     if (lsm.timeout != 0) return;
     if (tid == 0 && t == a.num_tiles - 1) *static_cast<uint64_t*>(a.carry_out) = static_cast<uint64_t>(pre) + total;
     V* out = static_cast<V*>(a.out) + pre;

@@ -210,7 +210,8 @@ gps_status gps_scan_host(gps_plan plan, gps_scan_kind kind, const void* h_in, vo
 
 /* Synchronizes `stream`, then reads and clears the plan's device error
  * flags: GPS_ERR_TIMEOUT if a bounded device-side wait expired since the last
- * check (the affected output is then undefined), else GPS_OK. */
+ * check (the output of that call, and of the plan's later calls up to this one,
+ * is then undefined; nothing outside their outputs is written), else GPS_OK. */
 gps_status gps_plan_check(gps_plan plan, gps_stream_t stream);
 
 /* Budget for each device-side wait of this plan's kernels, in nanoseconds
