@@ -38,6 +38,7 @@
 // 15.1.
 #pragma once
 #include "scan_seg.cuh"
+#include "segment_search.h"
 
 namespace gps {
 
@@ -261,22 +262,14 @@ __global__ void __launch_bounds__(kMidSegThreads, CTAS)
         // less ahead of the scan (500 compensated scans 8.8 -> 8.5 us, 1000 segments of
         // 2^20 u32 5.66 -> 5.44; from 5000 segments on no change).
         constexpr uint32_t kBatch = 4;
-        // Entries before lo are below t0; entry hi (if any) is not.
-        uint32_t lo = 0, hi = nseg;
-        while (hi - lo > kBatch * kMidSegThreads) {
-            const uint32_t step = (hi - lo + kMidSegThreads - 1) / kMidSegThreads;
-            const uint64_t idx = lo + static_cast<uint64_t>(tid) * step;
-            const bool below = idx < hi && sg.offsets[idx] < t0;
-            const uint32_t c = static_cast<uint32_t>(__syncthreads_count(below));
-            if (c == 0) {
-                hi = lo;
-                break;
-            }
-            hi = min(lo + c * step, hi);
-            lo = lo + (c - 1) * step + 1;
+        OffsetInterval at{0, nseg};
+        while (at.size() > kBatch * kMidSegThreads) {
+            const uint32_t probe = at.probe(tid, kMidSegThreads);
+            const bool below = probe < at.size() && sg.offsets[at.lo + probe] < t0;
+            at.narrow(static_cast<uint32_t>(__syncthreads_count(below)), kMidSegThreads);
         }
         __syncthreads();
-        for (uint64_t cur = lo;; cur += kBatch * kMidSegThreads) {
+        for (uint64_t cur = at.lo;; cur += kBatch * kMidSegThreads) {
             uint64_t o[kBatch];
 #pragma unroll
             for (uint32_t j = 0; j < kBatch; ++j) {

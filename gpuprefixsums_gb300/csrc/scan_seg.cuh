@@ -29,6 +29,7 @@
 
 #include "scan_ops.cuh"
 #include "scan_pipeline.cuh"
+#include "segment_search.h"
 
 namespace gps {
 
@@ -430,8 +431,7 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
     const uint64_t out_rows = VIEW ? out_n / ROW : rows_full;
     // Samples of the offsets: every `stride`-th entry, at most 1024.
     const uint32_t nseg = SEG ? sg.num_segments : 0u;
-    const uint32_t stride = SEG ? (nseg + 1 + 1023) / 1024 : 1u;
-    const uint32_t nsample = SEG ? (nseg + stride) / stride : 0u;  // samples cover entries 0..nseg
+    const OffsetSamples samples(nseg);  // cover entries 0..nseg
 
     if (tid == 0) {
         for (int s = 0; s < RS; ++s) {
@@ -479,8 +479,8 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
     constexpr uint32_t kSampleThreads = 2 * NROLE;
     if constexpr (SEG) {
         if (warp >= kWarpReduce && warp < kWarpFinal + RW) {
-            for (uint32_t j = tid - kWarpReduce * 32; j < nsample; j += kSampleThreads)
-                ctrl->sample[j] = sg.offsets[min(j * stride, nseg)];
+            for (uint32_t j = tid - kWarpReduce * 32; j < samples.count; j += kSampleThreads)
+                ctrl->sample[j] = sg.offsets[j * samples.stride];
             ptx::named_bar_arrive(1, kSampleThreads + 32);
         }
     }
@@ -792,7 +792,7 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
                     const uint64_t ustart = static_cast<uint64_t>(u) * G * TILE;
                     const uint64_t uend = min(ustart + static_cast<uint64_t>(G) * TILE, a.n);
                     // First sample greater than ustart (binary search in smem).
-                    uint32_t lo_s = 0, hi_s = nsample;  // invariant: sample[lo_s-1] <= ustart < sample[hi_s]
+                    uint32_t lo_s = 0, hi_s = samples.count;  // invariant: sample[lo_s-1] <= ustart < sample[hi_s]
                     while (lo_s < hi_s) {
                         const uint32_t mid = (lo_s + hi_s) >> 1;
                         if (ctrl->sample[mid] <= ustart)
@@ -800,28 +800,24 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
                         else
                             hi_s = mid;
                     }
-                    // The first offset >= ustart has an index in [lo_i, hi_i].
-                    uint32_t lo_i = lo_s == 0 ? 0u : (lo_s - 1) * stride;
-                    uint32_t hi_i = lo_s < nsample ? min(lo_s * stride, nseg) : nseg;
+                    OffsetInterval at = samples.interval(lo_s, nseg);
                     // Narrow a wide interval (many short segments) 32-fold per
-                    // round: one offset per lane, the last lane below ustart wins.
-                    while (hi_i - lo_i > kHeadBatch * 32u) {
-                        const uint32_t step = (hi_i - lo_i + 31u) / 32u;
-                        const uint32_t idx = min(lo_i + lane * step, nseg - 1u);
-                        const uint32_t below = __ballot_sync(kFullMask, sg.offsets[idx] < ustart);
-                        if (below == 0u) break;  // offsets[lo_i] >= ustart already
-                        const uint32_t last = 31u - static_cast<uint32_t>(__clz(below));
-                        hi_i = min(lo_i + (last + 1u) * step, hi_i);
-                        lo_i = lo_i + last * step;
+                    // round: one offset per lane.
+                    while (at.size() > kHeadBatch * 32u) {
+                        const uint32_t probe = at.probe(lane, 32u);
+                        const uint32_t below =
+                            __ballot_sync(kFullMask, probe < at.size() && sg.offsets[at.lo + probe] < ustart);
+                        at.narrow(static_cast<uint32_t>(__popc(below)), 32u);
                     }
-                    // Walk forward from lo_i, kHeadBatch loads of 32 offsets in
+                    // Walk forward from there, kHeadBatch loads of 32 offsets in
                     // flight per round, until an offset at or past uend.
-                    for (uint32_t cur = lo_i; cur < nseg; cur += kHeadBatch * 32u) {
+                    const uint32_t* head = sg.offsets + at.lo;
+                    for (uint32_t left = nseg - at.lo; left != 0;) {
                         uint32_t o[kHeadBatch];
     #pragma unroll
                         for (int j = 0; j < kHeadBatch; ++j) {
-                            const uint32_t idx = cur + static_cast<uint32_t>(j) * 32u + lane;
-                            o[j] = idx < nseg ? sg.offsets[idx] : 0xFFFFFFFFu;
+                            const uint32_t d = static_cast<uint32_t>(j) * 32u + lane;
+                            o[j] = d < left ? head[d] : 0xFFFFFFFFu;
                         }
                         bool past = false;
     #pragma unroll
@@ -833,6 +829,8 @@ __global__ void __launch_bounds__(SegShape<Op, RW>::kThreads, 1)
                             past = past || o[j] >= uend;
                         }
                         if (__any_sync(kFullMask, past)) break;
+                        head += kHeadBatch * 32u;
+                        left -= kHeadBatch * 32u;  // (fewer were left: then some lane was past)
                     }
                 }
                 __syncwarp();
