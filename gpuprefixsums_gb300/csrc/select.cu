@@ -468,7 +468,10 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
             if (k == static_cast<int>(group)) {
                 bool pok = wait1(&ctrl->uprefix[q], (i / Q) & 1u, long_budget);
                 pok = __all_sync(kFullMask, pok);
-                if (!pok && lane == 0) raise_error(a.hdr, kErrPipelineTimeout);
+                if (!pok) {  // without the unit's position nothing may be written
+                    if (lane == 0) raise_error(a.hdr, kErrPipelineTimeout);
+                    break;
+                }
                 run = ctrl->upre[q];
             }
             const uint32_t mask = ctrl->tmask[q][k][f];  // bit e: logical item e
