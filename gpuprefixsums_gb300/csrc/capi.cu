@@ -588,6 +588,14 @@ gps_status gps_plan_autotune(gps_plan p, gps_scan_kind kind, const void* d_in, v
 gps_status gps_plan_set_generic_config(gps_plan p, int segmented, uint64_t n, uint32_t unit, uint32_t ctas_div,
                                        uint32_t threads_per_row) {
     if (p == nullptr) return fail(GPS_ERR_INVALID_ARGUMENT, "plan is NULL");
+    if (unit == gps::kMidSegConfig.unit && ctas_div == gps::kMidSegConfig.ctas_div &&
+        threads_per_row == gps::kMidSegConfig.split) {
+        if (n > static_cast<uint64_t>(gps::kMidSegMaxTiles) * p->tile_elems)
+            return fail(GPS_ERR_UNSUPPORTED, "one tile per CTA takes at most %u tiles of %u elements",
+                        gps::kMidSegMaxTiles, p->tile_elems);
+        p->tuned[segmented ? 1 : 0][size_class(n)] = static_cast<int8_t>(kTunedMid);
+        return GPS_OK;
+    }
     for (int c = 0; c < gps::kNumGenericCandidates; ++c) {
         const gps::GenericConfig& g = gps::kGenericCandidates[c];
         if (g.unit == unit && g.ctas_div == ctas_div && g.split == threads_per_row) {
@@ -606,10 +614,7 @@ gps_status gps_plan_set_generic_config(gps_plan p, int segmented, uint64_t n, ui
 gps_status gps_plan_generic_config(gps_plan p, int segmented, uint64_t n, uint32_t* out_unit, uint32_t* out_ctas_div,
                                    uint32_t* out_threads_per_row, int* out_tuned) {
     if (p == nullptr) return fail(GPS_ERR_INVALID_ARGUMENT, "plan is NULL");
-    gps::GenericConfig cfg = generic_config(p, segmented != 0, n);
-    // One tile per CTA has no units: report the default of the kernel with
-    // units, a configuration gps_plan_set_generic_config() takes.
-    if (cfg.unit == 0) cfg = gps::default_generic_config(n, p->tile_elems, p->num_sms);
+    const gps::GenericConfig cfg = generic_config(p, segmented != 0, n);
     if (out_unit) *out_unit = cfg.unit;
     if (out_ctas_div) *out_ctas_div = cfg.ctas_div;
     if (out_threads_per_row) *out_threads_per_row = cfg.split;

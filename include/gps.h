@@ -169,7 +169,8 @@ gps_status gps_select_flagged(gps_plan plan, const void* d_in, const uint8_t* d_
  * a configuration whose result differs is not taken and the call returns
  * GPS_ERR_CUDA after tuning with the others. A shape that does not fit one
  * CTA's shared memory for the element type is skipped. Up to 4096 tiles the
- * one-tile-per-CTA form of the kernel is a candidate too. Without tuning, scans
+ * one-tile-per-CTA form of the kernel is a candidate too: unit 0, ctas_div 1,
+ * one thread per row. Without tuning, scans
  * of up to 2048 tiles (u32, f32), 1728 (u64), 1280 (compensated f32, 1728 batched)
  * or 704 (structs) take that form; larger ones use one thread per row and units of 4 tiles once
  * there is one such unit per SM, else 1 tile. d_out is left holding a correct
@@ -183,18 +184,19 @@ gps_status gps_plan_autotune(gps_plan plan, gps_scan_kind kind, const void* d_in
                              uint32_t* out_unit, uint32_t* out_ctas_div, uint32_t* out_threads_per_row);
 
 /* Launch configuration a batched (segmented != 0) or plain generic-kernel
- * scan of n elements would use now: tiles per unit, CTA divisor (1: one CTA
- * per SM, 2: half), threads per row (1 or 2), and whether it comes from
- * gps_plan_autotune() or gps_plan_set_generic_config(). Where the
- * one-tile-per-CTA form would run (untuned at small sizes, or the autotuner's
- * choice), which has no such units, this is the untuned configuration of the
- * kernel with units. */
+ * scan of n elements would use now: tiles per unit (0: the one-tile-per-CTA
+ * form, which has no units), CTA divisor (1: one CTA per SM, 2: half), threads
+ * per row (1 or 2), and whether it comes from gps_plan_autotune() or
+ * gps_plan_set_generic_config(). Setting on another plan what this reports
+ * makes the same launch there. */
 gps_status gps_plan_generic_config(gps_plan plan, int segmented, uint64_t n, uint32_t* out_unit,
                                    uint32_t* out_ctas_div, uint32_t* out_threads_per_row, int* out_tuned);
 
 /* Sets the launch configuration of a size class by hand (to restore a saved
  * tuning, or to test one configuration): unit 1 or 4, ctas_div 1 or 2,
- * threads_per_row 1 or 2. */
+ * threads_per_row 1 or 2; or unit 0, ctas_div 1, threads_per_row 1 for one tile
+ * per CTA, where n has at most 4096 tiles (scans of more in the same size
+ * class then run untuned). */
 gps_status gps_plan_set_generic_config(gps_plan plan, int segmented, uint64_t n, uint32_t unit, uint32_t ctas_div,
                                        uint32_t threads_per_row);
 
