@@ -78,6 +78,10 @@ struct gps_plan_s {
     uint64_t wait_budget_ns;
     gps::StallConfig stall;
     gps::LaunchInfo last_launch;
+    // Elements and launches of the last scan (0: none since a setting changed), for
+    // gps_plan_geometry().
+    uint64_t scanned_n;
+    uint32_t scanned_launches;
     // Staging for gps_scan_host, created on first use.
     void* stage[kHostStages];
     uint64_t stage_elems;
@@ -178,6 +182,24 @@ gps_status check_device(const gps_plan_s* p) {
     return GPS_OK;
 }
 
+// Which kernel a scan of n elements (n >= 1) runs on; `carries`: it takes or gives one.
+enum class ScanPath { Generic, Small, GenericUnits, Mid, Csdl, Rts };
+ScanPath scan_path(const gps_plan_s* p, uint64_t n, bool unaligned, bool carries) {
+    if (generic_only(p->dtype)) return ScanPath::Generic;
+    const bool plain = p->stall.mode == 0 && p->stall.fallback_polls == 0;
+    if (plain && n <= p->small_max) return ScanPath::Small;
+    if (p->algo != GPS_ALGO_CSDL) return ScanPath::Rts;
+    const uint32_t tiles = static_cast<uint32_t>((n + p->tile_elems - 1) / p->tile_elems);
+    if (plain && n > p->mid_max && !carries && gps::integer_scan_takes_generic(n, tiles, p->num_sms))
+        return ScanPath::GenericUnits;
+    // Buffers off a 16-byte boundary take the same kernels as others, but where the
+    // generic one does not apply: csdl.cu's for them moves single elements, so one tile per
+    // CTA takes every size that is left (2^27 u32 elements: 258 against 2017 us;
+    // generic kernel 160). One limit serves both (mid_max_bytes()).
+    if (plain && (n <= p->mid_max || (unaligned && p->mid_max != 0))) return ScanPath::Mid;
+    return ScanPath::Csdl;
+}
+
 // Device-side launch of one scan of n elements (n >= 1, already validated).
 gps_status launch_scan(gps_plan_s* p, bool inclusive, const void* in, void* out, uint64_t n, const void* carry_in,
                        void* carry_out, cudaStream_t stream) {
@@ -193,31 +215,31 @@ gps_status launch_scan(gps_plan_s* p, bool inclusive, const void* in, void* out,
     a.wait_budget_ns = p->wait_budget_ns;
     a.stall = p->stall;
     a.mid_launch = &p->hdr->mid_launch;
-    // Buffers off a 16-byte boundary take the same kernels as others, but where the
-    // generic one does not apply: csdl.cu's for them moves single elements, so one tile per
-    // CTA takes every size that is left (2^27 u32 elements: 258 against 2017 us;
-    // generic kernel 160). One limit serves both (mid_max_bytes()).
     const bool unaligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) != 0;
-    cudaError_t err;
-    if (generic_only(p->dtype)) {
-        err = launch_generic(p, inclusive, a, nullptr, generic_config(p, false, n), stream, &p->last_launch);
-    } else if (n <= p->small_max && p->stall.mode == 0 && p->stall.fallback_polls == 0) {
-        err = gps::launch_small(p->dtype, inclusive, a, stream, &p->last_launch);
-    } else if (p->algo == GPS_ALGO_CSDL && p->stall.mode == 0 && p->stall.fallback_polls == 0 && n > p->mid_max &&
-               carry_in == nullptr && carry_out == nullptr &&
-               gps::integer_scan_takes_generic(n, a.num_tiles, p->num_sms)) {
-        err = launch_generic(p, inclusive, a, nullptr, gps::kGenericCandidates[0], stream, &p->last_launch, unaligned);
-    } else if (p->algo == GPS_ALGO_CSDL && (n <= p->mid_max || (unaligned && p->mid_max != 0)) &&
-               p->stall.mode == 0 && p->stall.fallback_polls == 0) {
-        a.desc = p->desc_mid;
-        a.group_desc = p->group_sums;
-        err = gps::launch_mid(p->dtype, inclusive, a, p->num_sms, stream, &p->last_launch);
-    } else if (p->algo == GPS_ALGO_CSDL) {
-        err = gps::launch_csdl(p->dtype, inclusive, p->stall.mode != 0 || p->stall.fallback_polls != 0, a, p->num_sms,
-                               stream, &p->last_launch);
-    } else {
-        err = gps::launch_rts(p->dtype, inclusive, a, p->area, p->num_sms, stream, &p->last_launch);
+    cudaError_t err = cudaErrorInvalidValue;
+    switch (scan_path(p, n, unaligned, carry_in != nullptr || carry_out != nullptr)) {
+        case ScanPath::Generic:
+            err = launch_generic(p, inclusive, a, nullptr, generic_config(p, false, n), stream, &p->last_launch);
+            break;
+        case ScanPath::Small: err = gps::launch_small(p->dtype, inclusive, a, stream, &p->last_launch); break;
+        case ScanPath::GenericUnits:
+            err = launch_generic(p, inclusive, a, nullptr, gps::kGenericCandidates[0], stream, &p->last_launch, unaligned);
+            break;
+        case ScanPath::Mid:
+            a.desc = p->desc_mid;
+            a.group_desc = p->group_sums;
+            err = gps::launch_mid(p->dtype, inclusive, a, p->num_sms, stream, &p->last_launch);
+            break;
+        case ScanPath::Csdl:
+            err = gps::launch_csdl(p->dtype, inclusive, p->stall.mode != 0 || p->stall.fallback_polls != 0, a,
+                                   p->num_sms, stream, &p->last_launch);
+            break;
+        case ScanPath::Rts:
+            err = gps::launch_rts(p->dtype, inclusive, a, p->area, p->num_sms, stream, &p->last_launch);
+            break;
     }
+    p->scanned_n = err == cudaSuccess ? n : 0;
+    p->scanned_launches = p->last_launch.launches;
     if (err != cudaSuccess) return cuda_fail(err, "scan launch");
     return GPS_OK;
 }
@@ -784,6 +806,7 @@ gps_status gps_plan_set_stall(gps_plan p, uint32_t mode, uint32_t period, uint32
     if (mode != 0 && period == 0) return fail(GPS_ERR_INVALID_ARGUMENT, "period must be positive");
     if (delay_ns > 1000000000u) return fail(GPS_ERR_INVALID_ARGUMENT, "delay %u ns exceeds one second", delay_ns);
     p->stall = gps::StallConfig{mode, period, seed, delay_ns, fallback_polls, 0};
+    p->scanned_n = 0;
     return GPS_OK;
 }
 
@@ -792,6 +815,7 @@ gps_status gps_plan_set_fallback(gps_plan p, uint32_t fallback_polls) {
     if (fallback_polls != 0 && p->algo != GPS_ALGO_CSDL)
         return fail(GPS_ERR_UNSUPPORTED, "the decoupled fallback applies to the chained scan only");
     p->stall = gps::StallConfig{0, 1, 0, 0, fallback_polls, 0};
+    p->scanned_n = 0;
     return GPS_OK;
 }
 
@@ -812,8 +836,15 @@ gps_status gps_plan_geometry(gps_plan p, uint64_t n, uint32_t* tile_elems, uint3
     if (p == nullptr) return fail(GPS_ERR_INVALID_ARGUMENT, "plan is NULL");
     if (tile_elems) *tile_elems = p->tile_elems;
     if (grid) *grid = static_cast<uint32_t>(p->last_launch.grid);
-    const bool small = !generic_only(p->dtype) && n <= p->small_max && p->stall.mode == 0 && p->stall.fallback_polls == 0;
-    if (launches) *launches = n == 0 ? 0u : (small || p->algo == GPS_ALGO_CSDL ? 1u : gps::rts_launches(n, p->tile_elems, p->num_sms));
+    if (launches == nullptr) return GPS_OK;
+    *launches = n == 0 ? 0u : 1u;
+    if (n != 0 && n == p->scanned_n) {
+        *launches = p->scanned_launches;
+    } else if (n != 0) {
+        const ScanPath path = scan_path(p, n, false, false);
+        if (path == ScanPath::Rts) *launches = gps::rts_launches(n, p->tile_elems, p->num_sms);
+        if (path == ScanPath::Mid) *launches = gps::mid_launches(n, p->tile_elems);
+    }
     return GPS_OK;
 }
 
@@ -822,6 +853,7 @@ gps_status gps_plan_set_mid_max(gps_plan p, uint64_t max_n) {
     if (max_n != 0 && (p->algo != GPS_ALGO_CSDL || generic_only(p->dtype)))
         return fail(GPS_ERR_UNSUPPORTED, "the one-tile-per-CTA scan runs integer chained-scan plans only");
     p->mid_max = max_n;
+    p->scanned_n = 0;
     return GPS_OK;
 }
 
@@ -832,6 +864,7 @@ gps_status gps_plan_set_small_max(gps_plan p, uint64_t max_n) {
         return fail(GPS_ERR_INVALID_ARGUMENT, "the one-CTA scan takes at most %llu elements of this type",
                     static_cast<unsigned long long>(cap));
     p->small_max = max_n;
+    p->scanned_n = 0;
     return GPS_OK;
 }
 

@@ -160,6 +160,7 @@ struct LaunchInfo {
     int grid;
     int block;
     size_t smem;
+    uint32_t launches = 1;
 };
 
 cudaError_t launch_csdl(gps_dtype dtype, bool inclusive, bool stall_mode, const ScanArgs& a,
@@ -170,7 +171,7 @@ cudaError_t prepare_csdl(gps_dtype dtype);
 cudaError_t launch_rts(gps_dtype dtype, bool inclusive, const ScanArgs& a, void* scratch,
                        int num_sms, cudaStream_t stream, LaunchInfo* info);
 // Elements of scratch a reduce-then-scan plan keeps, and the kernel launches
-// of a scan of n elements.
+// of a scan of n elements of an aligned buffer.
 uint64_t rts_scratch_elems(int num_sms);
 uint32_t rts_launches(uint64_t n, uint32_t tile_elems, int num_sms);
 // Tensor maps of the generic kernel: the buffer seen as rows of 128 bytes
@@ -304,6 +305,10 @@ constexpr uint64_t mid_seg_default_tiles(gps_dtype dtype, bool segmented) {
         case GPS_DTYPE_U32X4: break;
     }
     return 704;
+}
+// Launches of a scan of n elements of an aligned buffer by the integer kernel.
+constexpr uint32_t mid_launches(uint64_t n, uint32_t tile_elems) {
+    return static_cast<uint32_t>((n + kMidMaxTiles * tile_elems - 1) / (kMidMaxTiles * tile_elems));
 }
 cudaError_t launch_mid(gps_dtype dtype, bool inclusive, const ScanArgs& a, int num_sms, cudaStream_t stream,
                        LaunchInfo* info);

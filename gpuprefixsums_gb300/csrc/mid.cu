@@ -190,7 +190,7 @@ cudaError_t launch_mid_v(const ScanArgs& a0, int num_sms, cudaStream_t stream, L
     // Scans of more tiles than there are group sums for run in pieces, each with
     // the sum through the piece before as its carry.
     char* carries = static_cast<char*>(a0.group_desc) + 2 * 128 * kMidSums;
-    if (info) *info = LaunchInfo{static_cast<int>(Rows::tiles(a0.in, a0.n)), kMidThreads, 0};
+    if (info) *info = LaunchInfo{static_cast<int>(Rows::tiles(a0.in, a0.n)), kMidThreads, 0, 0};
     for (uint64_t done = 0, piece = 0; done < a0.n; done += a.n, ++piece) {
         a.in = static_cast<const T*>(a0.in) + done;
         a.out = static_cast<T*>(a0.out) + done;
@@ -215,6 +215,7 @@ cudaError_t launch_mid_v(const ScanArgs& a0, int num_sms, cudaStream_t stream, L
                 ? launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, 6, true>, grid, kMidThreads, 0, stream, a)
                 : launch_dependent(mid_vec_kernel<T, INCL, ALIGNED, 0, true>, grid, kMidThreads, 0, stream, a);
         if (err != cudaSuccess) return err;
+        if (info) ++info->launches;
     }
     return cudaSuccess;
 }

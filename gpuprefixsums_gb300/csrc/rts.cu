@@ -256,7 +256,7 @@ cudaError_t dispatch_rts(bool inclusive, const ScanArgs& s, void* scratch, int n
               sums + 3ull * static_cast<uint64_t>(kRtsCtasPerSm * num_sms), s.carry_in, s.carry_out, s.hdr, s.wait_budget_ns};
     const int grid = static_cast<int>(sh.ranges);
     const size_t smem = sh.chunks > 1 ? 16384 : 0;
-    if (info) *info = LaunchInfo{grid, kRowThreads, smem};
+    if (info) *info = LaunchInfo{grid, kRowThreads, smem, sh.chunks + 1};
     for (; a.chunk <= sh.chunks; ++a.chunk) {
         const cudaError_t err =
             inclusive ? launch_dependent(rts_kernel<T, true, ALIGNED>, grid, kRowThreads, smem, stream, a)

@@ -277,8 +277,10 @@ typedef struct gps_lookback_stats {
 gps_status gps_plan_stats(gps_plan plan, gps_stream_t stream, gps_lookback_stats* out_stats);
 
 /* Kernel geometry of the plan (for tools and tests): elements per tile of the
- * main scan kernel, its grid size for a scan of n elements, and the number of
- * kernel launches one gps_scan of n elements makes. */
+ * main scan kernel, the grid size of the plan's last call, and the number of
+ * kernel launches one gps_scan of n elements makes: of the last one if it had n
+ * elements, else of one on 16-byte aligned buffers (a view off that boundary may
+ * take one more). */
 gps_status gps_plan_geometry(gps_plan plan, uint64_t n, uint32_t* tile_elems, uint32_t* grid,
                              uint32_t* launches);
 
