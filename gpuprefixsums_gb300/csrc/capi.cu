@@ -134,7 +134,7 @@ gps::GenericConfig generic_config(const gps_plan_s* p, bool segmented, uint64_t 
     const uint64_t tiles = (n + p->tile_elems - 1) / p->tile_elems;
     if (tiles <= (c == kTunedMid ? gps::kMidSegMaxTiles : gps::mid_seg_default_tiles(p->dtype, segmented)))
         return gps::kMidSegConfig;
-    return gps::default_generic_config(n, p->tile_elems, p->num_sms);
+    return gps::kGenericCandidates[0];
 }
 
 // Generic kernel (scan_seg.cuh, mid_seg.cuh): floating-point scans and batched
@@ -275,10 +275,6 @@ cudaError_t hash_buffer(const void* d, uint64_t bytes, unsigned long long* d_has
 
 namespace gps {
 size_t dtype_size(gps_dtype dtype) { return dtype == GPS_DTYPE_U64 ? 8 : dtype == GPS_DTYPE_U32X4 ? 16 : 4; }
-GenericConfig default_generic_config(uint64_t n, uint32_t tile_elems, int num_sms) {
-    const uint64_t units4 = (n + 4ull * tile_elems - 1) / (4ull * tile_elems);
-    return units4 >= static_cast<uint64_t>(num_sms) ? GenericConfig{4, 1, 1} : GenericConfig{1, 1, 1};
-}
 // Plain integer scans above the mid size run on the generic kernel too, in units
 // of 4 tiles: its reduce warps need no warp scan and no barrier per tile (the
 // aggregator warp scans a unit's row sums once), and its fixed-order lookback

@@ -197,14 +197,12 @@ struct GenericConfig {
     uint32_t ctas_div;
     uint32_t split;
 };
+// The first is the untuned choice above the sizes of one tile per CTA: every SM has a
+// unit of 4 tiles there. Measured on GB300, units of 4 tiles against single-tile units, batched
+// u32: 640 tiles 11.7 / 13.1 us, 1024 tiles 13.5 / 16.3.
 constexpr GenericConfig kGenericCandidates[] = {{4, 1, 1}, {1, 1, 1}, {4, 2, 1}, {1, 2, 1},
                                                 {4, 1, 2}, {1, 1, 2}, {4, 2, 2}, {1, 2, 2}};
 constexpr int kNumGenericCandidates = 8;
-// Untuned choice: units of 4 tiles once there is one such unit per SM, else
-// single-tile units (more CTAs busy on small inputs). Measured on GB300, 640 tiles
-// (160 units of 4): FP32 11.2 us either way, batched u32 11.7 against 13.1 with
-// single-tile units; 1024 tiles 13.5 / 13.7 and 13.5 / 16.3.
-GenericConfig default_generic_config(uint64_t n, uint32_t tile_elems, int num_sms);
 // Whether a plain u32 or u64 scan above the mid size runs on the generic kernel.
 bool integer_scan_takes_generic(uint64_t n, uint32_t tiles, int num_sms);
 

@@ -44,7 +44,6 @@ struct OpInt {
     static constexpr bool kPackedRowSum = false;
     __device__ static S zero() { return 0; }
     __device__ static S lift(T x) { return x; }
-    __device__ static S add(S a, S b) { return a + b; }
     __device__ static S acc(S a, T x) { return a + x; }
     __device__ static S combine(S a, S b) { return a + b; }
     __device__ static S norm(S a) { return a; }
@@ -76,7 +75,6 @@ struct OpF32 {
     static constexpr bool kPackedRowSum = false;
     __device__ static S zero() { return 0.0f; }
     __device__ static S lift(T x) { return x; }
-    __device__ static S add(S a, S b) { return a + b; }
     __device__ static S acc(S a, T x) { return a + x; }
     __device__ static S combine(S a, S b) { return a + b; }
     __device__ static S norm(S a) { return a; }
@@ -143,15 +141,6 @@ struct OpF32C {
     static constexpr bool kPackedRowSum = true;
     __device__ static S zero() { return F2{0.0f, 0.0f}; }
     __device__ static S lift(T x) { return F2{x, 0.0f}; }
-    __device__ static S add(S a, S b) {
-        const float s = a.hi + b.hi;
-        const float bb = s - a.hi;
-        float e = (a.hi - (s - bb)) + (b.hi - bb);
-        e += a.lo + b.lo;
-        const float hi = s + e;
-        const float lo = e - (hi - s);
-        return F2{hi, lo};
-    }
     __device__ static S acc(S a, T x) {
         const float s = a.hi + x;
         const float bb = s - a.hi;

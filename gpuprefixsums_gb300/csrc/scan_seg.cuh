@@ -52,13 +52,6 @@ __device__ __forceinline__ void seg_combine(typename Op::S& a, bool& fa, typenam
     fa = fa || fb;
 }
 
-template <class Op>
-__device__ __forceinline__ typename Op::C chain_warp_sum(typename Op::C x) {
-#pragma unroll
-    for (int m = 16; m; m >>= 1) x = Op::chain_add(x, Op::chain_shfl_xor(x, m));
-    return x;
-}
-
 // Inclusive warp scan of (state, head flag) in lane order. Without FLAGS the
 // flags are known to be false and only the states move.
 template <class Op, bool FLAGS>

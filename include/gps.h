@@ -172,8 +172,7 @@ gps_status gps_select_flagged(gps_plan plan, const void* d_in, const uint8_t* d_
  * one-tile-per-CTA form of the kernel is a candidate too: unit 0, ctas_div 1,
  * one thread per row. Without tuning, scans
  * of up to 2048 tiles (u32, f32), 1728 (u64), 1280 (compensated f32, 1728 batched)
- * or 704 (structs) take that form; larger ones use one thread per row and units of 4 tiles once
- * there is one such unit per SM, else 1 tile. d_out is left holding a correct
+ * or 704 (structs) take that form; larger ones use one thread per row and units of 4 tiles. d_out is left holding a correct
  * result. Synchronizes `stream`; not allowed while the stream is being
  * captured. The chosen configuration is returned in out_unit /
  * out_ctas_div / out_threads_per_row (any may be NULL).
