@@ -68,12 +68,14 @@ def parse_args():
                    help="only the timed scans (for profiling): no copy/CUB/RTS/e2e/CPU legs")
     p.add_argument("--no-extras", action="store_true", help="skip the batched, fp32 and mixed workloads")
     p.add_argument("--profile-case", choices=["batched", "f32c", "select", "struct", "mid", "f32c_batched",
-                                              "u64_batched"], default=None,
+                                              "u64_batched", "mid_f32", "mid_select", "view", "rts"], default=None,
                    help="launch one small case three times and exit (ncu captures): 1024 of the batched "
                         "workload's segments, 2^26 compensated-f32 elements, a select of 2^26 u32 by "
                         "Bernoulli(0.3) flags, an inclusive scan of 2^24 structs of four u32, an "
-                        "exclusive u32 scan of 2^20 elements (the one-tile-per-CTA kernel), or the first "
-                        "1000 compensated-f32 / u64 segments of the mixed workload")
+                        "exclusive u32 scan of 2^20 elements (the one-tile-per-CTA kernel), the first "
+                        "1000 compensated-f32 / u64 segments of the mixed workload, a plain f32 scan or a "
+                        "select of 2^20 (one tile per CTA too), an exclusive u32 scan of 2^26 elements from "
+                        "a view one element past a 16-byte boundary, or a reduce-then-scan of 2^26 u32")
     p.add_argument("--e2e-steps", type=int, default=8)
     p.add_argument("--clock-soak-s", type=float, default=1.0,
                    help="seconds of untimed steps sampled for clocks right before the timed region")
@@ -829,6 +831,7 @@ def run_profile_case(args):
     import torch
 
     from gpuprefixsums_gb300 import Plan
+    small = args.profile_case.startswith("mid")
     if args.profile_case == "batched":
         lengths = log_uniform_lengths(4096, 2 ** 20, seed=3)[:1024]
         offs = np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint32)
@@ -839,8 +842,8 @@ def run_profile_case(args):
             for _ in range(3):
                 out = plan.scan_segmented(x, d_off)
             plan.check()
-    elif args.profile_case == "select":
-        n = 1 << 26
+    elif args.profile_case in ("select", "mid_select"):
+        n = 1 << 20 if small else 1 << 26
         x = torch.randint(-2 ** 31, 2 ** 31 - 1, (n,), dtype=torch.int32, device="cuda")
         fl = (torch.rand(n, device="cuda") < 0.3).to(torch.uint8)
         with Plan("csdl", "u32", max_n=n) as plan:
@@ -863,12 +866,13 @@ def run_profile_case(args):
                 out = plan.scan_segmented(x, d_off)
             plan.check()
         out = out.float()
-    elif args.profile_case == "mid":
-        n = 1 << 20
-        x = torch.randint(0, 256, (n,), dtype=torch.int32, device="cuda")
-        with Plan("csdl", "u32", max_n=n) as plan:
+    elif args.profile_case in ("mid", "view", "rts"):
+        n, off = 1 << 20 if small else 1 << 26, int(args.profile_case == "view")
+        x = torch.randint(0, 256, (n + off,), dtype=torch.int32, device="cuda")[off:]
+        out = torch.empty(n, dtype=torch.int32, device="cuda")
+        with Plan("rts" if args.profile_case == "rts" else "csdl", "u32", max_n=n) as plan:
             for _ in range(3):
-                out = plan.scan(x)
+                plan.scan(x, out=out)
             plan.check()
     elif args.profile_case == "struct":
         n = 1 << 24  # 256 MiB of structs
@@ -879,9 +883,9 @@ def run_profile_case(args):
             plan.check()
         out = out[:, 0]
     else:
-        n = 1 << 26
+        n = 1 << 20 if small else 1 << 26
         x = torch.randn(n, device="cuda")
-        with Plan("csdl", "f32c", max_n=n) as plan:
+        with Plan("csdl", "f32" if small else "f32c", max_n=n) as plan:
             for _ in range(3):
                 out = plan.scan(x, inclusive=True)
             plan.check()

@@ -278,9 +278,9 @@ size_t dtype_size(gps_dtype dtype) { return dtype == GPS_DTYPE_U64 ? 8 : dtype =
 // Plain integer scans above the mid size run on the generic kernel too, in units
 // of 4 tiles: its reduce warps need no warp scan and no barrier per tile (the
 // aggregator warp scans a unit's row sums once), and its fixed-order lookback
-// reads 128 descriptors a poll, not 512. Measured on GB300 against
-// scan_l2_kernel, graph replay: u32 2^24 26.3 / 33.4 us, 2^25 46.5 / 53.4, 2^26
-// 86.2 / 92.0, 2^28 320 / 330; u64 2^27 322 / 345. Below two units per SM its
+// reads 64 descriptors a poll, not 512. Measured on GB300 against
+// scan_l2_kernel, graph replay: u32 2^24 25.9 / 33.4 us, 2^25 44.5 / 53.6, 2^26
+// 83.9 / 92.1, 2^28 315.8 / 330.2; u64 2^27 319 / 341. Below two units per SM its
 // pipeline does not fill. The tensor maps count rows of 128 bytes in 32 bits.
 bool integer_scan_takes_generic(uint64_t n, uint32_t tiles, int num_sms) {
     return tiles >= 8ull * static_cast<uint64_t>(num_sms) && n <= (1ull << 34);

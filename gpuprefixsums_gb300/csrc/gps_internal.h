@@ -189,8 +189,8 @@ cudaError_t encode_row_maps(const void* in, void* out, uint64_t n, uint64_t out_
 // Launch configuration of the generic kernel: tiles per lookback unit (1 or
 // 4; the unit is what one CTA takes from the work counter), the CTA count as
 // a fraction of the resident maximum (1 = all, 2 = half), and threads per
-// 128-byte row of a tile (1: 4 reduce and 4 finalize warps, each thread
-// scanning 128 bytes; 2: 8 and 8, each thread scanning 64 bytes). A unit of 0
+// 128-byte row of a tile (1: 4 reduce warps and two groups of 4 finalize warps,
+// each thread scanning 128 bytes; 2: 8 and 8, each thread scanning 64 bytes). A unit of 0
 // stands for one tile per CTA (mid_seg.cuh).
 struct GenericConfig {
     uint32_t unit;
@@ -246,8 +246,11 @@ bool seg_u32x4_x2_fits(uint32_t unit);
 // element size, and the launch. a.carry_out receives the count (uint64).
 uint32_t select_tile_elems(size_t elem_size);
 // Selects of up to this many tiles run one tile per CTA, on the plan's
-// mid-size descriptors (u32 2450 tiles 17.2 us against 18.9 on the persistent kernel, 2500
-// 18.6 / 18.6, 2600 20.6 / 19.0; u64 2600 19.6 / 18.2).
+// mid-size descriptors: where that met the persistent kernel before its lookback came
+// down to one round trip. Measured since (152 SMs, graph replay, inputs from HBM, us, against the
+// persistent kernel): u32, 30% selected, 2400 tiles 15.6 / 20.3, 2500 17.5 / 20.6, 3200
+// 20.2 / 23.8, 4095 25.7 / 25.7; u64 2500 17.7 / 19.2, 3200 20.2 / 22.0; 10% and 90% alike. The two
+// meet at about 4095 tiles now; the limit stands where it was.
 constexpr uint32_t kMidSelectMaxTiles = 2500;
 cudaError_t launch_select(size_t elem_size, const ScanArgs& a, const uint8_t* flags, int num_sms, cudaStream_t stream,
                           LaunchInfo* info);
@@ -258,11 +261,12 @@ uint64_t small_scan_max_elems(gps_dtype dtype);
 cudaError_t launch_small(gps_dtype dtype, bool inclusive, const ScanArgs& a, cudaStream_t stream, LaunchInfo* info);
 
 // Integer chained scans up to mid size, one 16 KB tile per CTA (mid.cu); the
-// default upper size of a plan: two waves of 8 CTAs per SM (2432 tiles) and a few
-// more. Measured on GB300 (graph replay, us) against the persistent kernel that takes
-// over (the generic one): u32 9.96 M elements 16.7 / 18.3, 10.1 M 17.8 / 18.3, 10.2 M 18.2 /
-// 18.2, 10.4 M 19.0 / 18.4, 2^24 29.2 / 25.6; off a 16-byte boundary 9.96 M 18.9 / 19.7, 10.1 M
-// 20.3 / 19.7; u64 4.9 M 17.5 / 18.0, 5.02 M 17.6 / 18.1, 5.06 M 18.4 / 18.1.
+// default upper size of a plan: 2448 tiles, one limit for three curves. Measured on GB300
+// (152 SMs: two waves of 8 CTAs per SM are 2432 tiles; graph replay, inputs from HBM, us)
+// against the generic kernel, which takes over: u32 2400 tiles 17.4 / 18.9, 2440 18.0 / 18.7, 2448
+// 19.0 / 18.8, 2500 19.9 / 18.8; off a 16-byte boundary 2400 20.0 / 20.2, 2432 20.4 / 20.3, 2448
+// 21.3 / 20.5; u64 2300 18.3 / 18.1, 2400 19.1 / 18.6, 2448 19.9 / 18.6: u32 meets it at the limit, views
+// 30 tiles below, u64 some 150 below. Earlier measurements had all three within 30 tiles of it.
 constexpr size_t mid_max_bytes() { return 153ull << 18; }
 // Tile descriptors of the one-tile-per-CTA kernels sit one per 128-byte line
 // (a stride of 8 words) when a launch has more than one group of 32 tiles, else
@@ -288,12 +292,12 @@ static_assert(kMidSegGroup >= 32 && kMidSegMaxTiles <= kMidMaxTiles, "within the
 constexpr GenericConfig kMidSegConfig = {0, 1, 1};
 // Untuned scans of up to this many tiles take it; larger ones the kernel with
 // units, whose pipeline then pays. The wider the running state, the fewer CTAs
-// an SM holds and the longer each takes. Measured on GB300 (graph replay, us, one
-// tile per CTA against units of 4 tiles): FP32 1700 tiles 14.3 / 15.3, 1900 15.4 / 15.7,
-// 2100 16.6 / 16.5; batched u32 14.7 / 16.6, 16.1 / 16.9, 17.5 / 17.8; compensated 1250 tiles
-// 13.3 / 14.0, 1400 15.5 / 15.0, batched 15.3 / 15.9 and 16.4 / 16.7, 1700 18.9 / 19.3; batched u64
-// 1250 tiles 12.9 / 13.6, 1700 15.9 / 16.4; structs 640 tiles 10.8 / 11.8, 720 11.4 / 11.0, batched
-// 11.6 / 12.0 and 11.7 / 11.8.
+// an SM holds and the longer each takes. Measured on GB300 (152 SMs, for which these are
+// constants; graph replay, inputs from HBM, us, one tile per CTA against units of 4 tiles): FP32
+// 1728 tiles 14.8 / 15.9, 1900 15.8 / 16.4, 2048 16.9 / 16.6; batched u32 1900 tiles 16.3 / 17.6,
+// 2048 17.3 / 17.9, 2200 18.1 / 18.6; compensated 1250 tiles 13.8 / 14.6, 1400 16.0 / 16.0, batched
+// 1728 tiles 18.7 / 20.2, 2048 21.7 / 22.0; batched u64 1728 tiles 15.9 / 16.9, 1900 17.4 / 17.5, 2048
+// 18.6 / 17.7; structs 640 tiles 10.8 / 11.8, 720 11.4 / 11.0, batched 11.6 / 12.0 and 11.7 / 11.8.
 constexpr uint64_t mid_seg_default_tiles(gps_dtype dtype, bool segmented) {
     switch (dtype) {
         case GPS_DTYPE_U32:

@@ -1,7 +1,7 @@
 // Single-pass chained scan for mid-size inputs: one 16 KB tile per CTA.
 //
-// The persistent L2-buffered kernel (scan_l2.cuh) pays a pipeline latency of
-// about 10 us per launch (unit claim, HBM load, reduce, lookback, reload from
+// The persistent kernel of large scans (scan_seg.cuh) pays a pipeline latency of
+// 8 to 10 us per launch (unit claim, HBM load, reduce, lookback, reload from
 // L2, scan, store), which dominates at small sizes. Here every tile gets its
 // own CTA of 256 threads, as in the reference's single-pass kernel
 // (ChainedScanDecoupledLookback.cuh:79-139):
@@ -49,10 +49,11 @@ constexpr int kMidCtasPerSm = 8;
 // registers) or six (40). With 0 its chunks are
 // read again after it (from L1 or L2): 32 registers, eight CTAs per SM, so that
 // up to 1216 tiles (2^22 u32 elements fit on 152 SMs) run in one wave. Which is
-// faster turns on the number of waves: up to one wave of the HELD form it is
-// ahead (graph replay, u32: 1000 elements 1.43 against 1.62 us, 2^16 2.74 / 2.91,
-// 2^20 5.67 / 5.92, 2^21 7.1 / 7.4), beyond it the other (2^22 11.0 / 9.7, 2^23
-// 17.8 / 16.7; with four CTAs instead of six, 500 tiles 6.7 / 7.1). There is no shared-memory staging and no mbarrier to set up, so
+// fastest turns on the number of waves: the form that holds most while the launch
+// is one wave of it. Measured on GB300 (graph replay, inputs from HBM, us, HELD 4 / 6 /
+// 0): u32 256 tiles 4.36 / 4.49 / 4.66, 608 tiles 5.64 / 6.04 / 6.08, 700 tiles 8.22 / 6.23 / 6.79,
+// 912 tiles 9.32 / 7.14 / 7.73, 1024 tiles 9.84 / 9.31 / 8.27, 1216 tiles 10.9 / 10.5 / 9.6; u64 and views
+// alike. There is no shared-memory staging and no mbarrier to set up, so
 // every CTA issues its loads as soon as it starts.
 //
 // ALIGNED = false takes buffers at any element offset from a 16-byte boundary
@@ -60,13 +61,14 @@ constexpr int kMidCtasPerSm = 8;
 // registers.
 // Bound by the same latency chain as the aligned form. Measured on GB300,
 // 10,000,019 u32 from a view one element past a boundary, into an aligned
-// output: 21.3 us a call, where per-thread element loads and stores (64
-// bytes apart across a warp) took 70.9; the generic kernel, which is ahead from
-// about there on, 20.2.
+// output: 20.0 us a call, where per-thread element loads and stores (64
+// bytes apart across a warp) took 70.9; 1024 tiles 9.5 us against 8.3 aligned. The
+// generic kernel is ahead from 2420 tiles on (mid_max_bytes()).
 //
 // GROUPS = false is for launches of one group of tiles, where the code for the
 // group sums costs fetches though it is not run (32 captured scans of 2^16 with it
-// 84-92 us, without 72-84, by where the plan's memory lies).
+// 84-92 us, without 72-84, by where the plan's memory lies; 78-86 in the latest
+// measurement, over eight plans of one process).
 template <typename T, bool INCL, bool ALIGNED, int HELD, bool GROUPS>
 __global__ void __launch_bounds__(kMidThreads, HELD ? HELD : kMidCtasPerSm) mid_vec_kernel(const ScanArgs a) {
     using Rows = TileRows<T, ALIGNED>;

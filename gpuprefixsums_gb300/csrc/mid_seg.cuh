@@ -30,12 +30,11 @@
 // tiles wait for the same two L2 round trips instead of a chain.
 //
 // Measured on GB300, graph replay, inputs from HBM, against the generic kernel
-// with single-tile units (its untuned choice at these sizes): FP32 2^16 2.7
-// against 7.9 us, 2^20 6.1 against 9.6, 2^22 12.4 against 15.5; compensated
-// FP32 2^20 7.8 against 10.9; batched u32 (500 segments) 2^20 7.3 against
-// 11.7; 300,000 segments in 2^20 elements 8.7 against 22.3. Groups of 64 tiles
-// against 32 / 128: 2^20 6.13 / 6.35 / 6.46 us, compensated 2^22 14.5 / 15.3 /
-// 15.1.
+// in units of 4 tiles: FP32 2^20 5.2 against 8.4 us, 2^22 9.4 / 12.5; compensated
+// FP32 2^20 6.6 / 9.2, 2^22 11.9 / 13.8; batched u32 (500 segments) 2^20 5.3 / 10.3;
+// 300,000 segments in 2^20 elements 6.7 / 17.2; 500 compensated segments of 2.2 M
+// 8.4 / 14.7. Groups of 64 tiles against 32 / 128: FP32 2^20 5.16 / 5.33 / 5.33 us, compensated
+// 2^22 11.9 / 12.5 / 12.5.
 #pragma once
 #include "scan_seg.cuh"
 #include "segment_search.h"
@@ -197,10 +196,11 @@ __device__ __forceinline__ bool mid_seg_prefix(const ScanArgs& a, uint32_t t, ui
 // registers, the faster form while a launch fits one wave of them; larger
 // launches want more tiles in flight: the smallest of 4, 6 and 8 that takes the
 // launch in one wave (segmented scans at most 6, structs always 4). Measured on
-// GB300 (graph replay, us, 4 / 6 / 8 CTAs): FP32 256 tiles 5.64 / 5.80 / 6.43, 1024
-// tiles 12.1 / 11.1 / 10.5; compensated 1024 tiles 15.0 / 13.8 / 12.8; batched compensated
-// 551 tiles 9.9 / 10.9 / 11.3, 1024 tiles 15.5 / 15.2 / 15.1; batched u64 512 tiles 7.9 / 9.1 /
-// 9.4; select 800 tiles 9.1 / 7.8 / 8.7, 2048 tiles 17.3 / 16.9 / 15.8.
+// GB300 (graph replay, inputs from HBM, us, 4 / 6 / 8 CTAs): FP32 256 tiles 5.12 / 5.19 / 5.42, 768
+// tiles 9.47 / 7.53 / 8.39, 1024 tiles 11.3 / 10.4 / 9.5; compensated 1024 tiles 14.1 / 13.2 / 11.8;
+// batched (4 / 6) compensated 500 tiles 8.27 / 9.46, 768 tiles 12.2 / 10.6; batched u64 500 tiles
+// 6.65 / 7.79; select u32 500 tiles 5.11 / 5.07 / 5.78, 608 tiles 5.44 / 5.60 / 5.46, 768 tiles 8.16 / 6.13 /
+// 7.00, 1024 tiles 8.94 / 8.90 / 7.85 (1300 tiles, two waves of every form, 10.1 / 9.9 / 11.0).
 inline int mid_seg_ctas(uint32_t tiles, int num_sms, int most) {
     for (int c = 4; c < most; c += 2)
         if (tiles <= static_cast<uint32_t>(c * num_sms)) return c;

@@ -8,7 +8,8 @@
 
 namespace gps {
 
-// 4 reduce + 4 finalize warps over 16 KB tiles. Stages: as many as fit in 227 KB of shared memory next to the control
+// 4 reduce warps and two groups of 4 finalize warps over 16 KB tiles (8 and 8 where two
+// threads share a row). Stages: as many as fit in 227 KB of shared memory next to the control
 // block (whose per-thread prefixes and head bitmaps grow with the state size
 // and the unit), taken as 4 reduce-pass + 9 scan-pass stages when 13 fit
 // (measured on GB300: 4 + 9 beats 5 + 8 by 3-8% on the batched workloads),

@@ -545,10 +545,9 @@ __global__ void __launch_bounds__(kSelThreads, 1) select_kernel(const ScanArgs a
 // (mid_lookback.cuh, in 32 bits), and the run goes out, coalesced.
 // Latency bounds it: one HBM read, one L2 round trip, a store (with mid_seg.cuh's
 // lookback, two: 2^20 u32 4.8 against 4.0 us, 2^22 8.8 / 8.2, 2^23 15.6 / 14.5; 2^20 u64 5.45 / 4.8).
-// Measured with that on
-// GB300, graph replay, u32, 30% selected, against the persistent kernel:
-// 2^16 elements 2.7 against 7.1 us, 2^20 5.6 / 8.8, 2^22 11.4 / 14.2, 2^23 17.9 /
-// 19.0 (90% selected: 21.0 / 24.0), 2^24 32.3 / 28.4.
+// Measured on GB300, graph replay, inputs from HBM, u32, 30% selected, against the
+// persistent kernel: 2^20 elements 3.9 against 9.1 us, 2^22 7.9 / 12.9, 2^23 13.9 / 17.2 (90%
+// selected 16.9 / 21.4), 2^24 25.7 / 25.7.
 constexpr int kMidSelThreads = kMidSegThreads;
 
 template <typename V, int CTAS, bool GROUPS>
